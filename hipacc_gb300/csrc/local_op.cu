@@ -6,6 +6,7 @@
 // declarations only: the kernels are instantiated in the lop_*.cu units, which
 // compile in parallel
 #include "local_op.cuh"
+#include "local_minmax.h"
 
 namespace hgb {
 
@@ -146,6 +147,16 @@ extern "C" int hgb_local_op(const hgb_view *in, const hgb_window *accw, const hg
     }
     return run_conv(in->dtype, out->dtype, p, kw, kh, in->batch, st);
   }
+  // MIN / MAX over a Domain of centred row runs (squares, discs, crosses,
+  // diamonds, lines) up to 7 x 7: the tiled kernel.  Masks with weights, other
+  // row shapes, larger windows and mixed storage go to the general kernel
+  // (7 x 7 disc, 6 u8 images of 1408 x 3357: 700 us there, 72 us tiled; 3 x 3,
+  // 4 f32 images of 1152 x 2870: 135 us and 39 us; a 300 x 280 image costs its
+  // launch in both).
+  MinMaxDomain dom;
+  if ((reduce == HGB_REDUCE_MIN || reduce == HGB_REDUCE_MAX) && !mask && !mask_dev && in->dtype == out->dtype &&
+      minmax_domain(domain, mask_w, mask_h, &dom))
+    return run_minmax_domain(*in, acc, *out, is, dom, reduce, boundary, const_val, st);
   GenParams g;
   memset(&g, 0, sizeof(g));
   fill_conv_params(*in, acc, *out, is, boundary, const_val, &g.c);

@@ -1,0 +1,107 @@
+// stage_groups.cuh -- staging of a halo tile into shared memory as FP32 for any
+// row alignment and any boundary, four columns at a time.
+//
+// Rows [Y0, Y0 + SH) x columns [X0, X0 + SW) of an accessor window are copied
+// into `tile` (row pitch SW floats).  A group of four columns that lies inside
+// the window is loaded whole: one vector load where its address allows it,
+// else the aligned 32-bit words around it, shifted into place (u8 and 16-bit
+// rows of odd length start at any byte).  Only groups that leave the window
+// evaluate the boundary remap (lib/AST/BorderHandling.cpp:41-120), so a border
+// tile costs little more than an inner one.
+//
+// Why: the per-element staging this replaces spent a remap (two compares and
+// often a branch per axis) and one byte load on every staged cell, ~21 cells
+// per thread and tile, also in tiles far from any border.
+#pragma once
+
+#include "hgb_internal.cuh"
+
+namespace hgb {
+
+// four bytes of a word as floats: a byte in the mantissa of 2^23 is 2^23 + b
+__device__ __forceinline__ float4 bytes_to_f4(uint32_t w) {
+  const f2 k23 = f2_pack(8388608.0f, 8388608.0f);
+  const f2 lo = f2_sub(f2_pack(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440)),
+                               __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7441))), k23);
+  const f2 hi = f2_sub(f2_pack(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7442)),
+                               __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7443))), k23);
+  return make_float4(f2_lo(lo), f2_hi(lo), f2_lo(hi), f2_hi(hi));
+}
+
+// Four consecutive elements at `p`, which have at least four more elements of
+// the same row on either side unless `p` is aligned for a vector load.
+template <typename T> struct Load4;
+template <> struct Load4<uint8_t> {
+  static constexpr int kAlign = 4;
+  static __device__ __forceinline__ float4 whole(const uint8_t *p) {
+    return bytes_to_f4(__ldg(reinterpret_cast<const uint32_t *>(p)));
+  }
+  static __device__ __forceinline__ float4 shifted(const uint8_t *p) {
+    const unsigned s = (unsigned)(reinterpret_cast<uintptr_t>(p) & 3u);
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(p - s);
+    return bytes_to_f4(__funnelshift_r(__ldg(w), __ldg(w + 1), 8 * s));
+  }
+};
+template <> struct Load4<float> {
+  static constexpr int kAlign = 16;
+  static __device__ __forceinline__ float4 whole(const float *p) { return __ldg(reinterpret_cast<const float4 *>(p)); }
+  static __device__ __forceinline__ float4 shifted(const float *p) {
+    return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+  }
+};
+template <typename T> struct Load4Half {
+  static constexpr int kAlign = 8;
+  static __device__ __forceinline__ float4 widen(uint32_t a, uint32_t b) {
+    T h[4];
+    const uint2 v = make_uint2(a, b);
+    __builtin_memcpy(h, &v, 8);
+    return make_float4(Storage<T>::to_f(h[0]), Storage<T>::to_f(h[1]), Storage<T>::to_f(h[2]), Storage<T>::to_f(h[3]));
+  }
+  static __device__ __forceinline__ float4 whole(const T *p) {
+    const uint2 v = __ldg(reinterpret_cast<const uint2 *>(p));
+    return widen(v.x, v.y);
+  }
+  static __device__ __forceinline__ float4 shifted(const T *p) {
+    const unsigned s = (unsigned)(reinterpret_cast<uintptr_t>(p) & 2u);
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(reinterpret_cast<const char *>(p) - s);
+    const uint32_t a = __ldg(w), b = __ldg(w + 1), c = s ? __ldg(w + 2) : 0u;
+    return widen(__funnelshift_r(a, b, 8 * s), __funnelshift_r(b, c, 8 * s));
+  }
+};
+template <> struct Load4<__nv_bfloat16> : Load4Half<__nv_bfloat16> {};
+template <> struct Load4<__half> : Load4Half<__half> {};
+
+// The group of columns [x, x + 4) of row y of the window.
+template <typename TI>
+__device__ __forceinline__ float4 load_group(const char *in, int64_t pitch, int x, int y, int ax_lo, int ax_hi,
+                                             int ay_lo, int ay_hi, int bmode, float cval) {
+  if (y >= ay_lo && y < ay_hi && x >= ax_lo && x + 4 <= ax_hi) {
+    const TI *p = reinterpret_cast<const TI *>(in + (int64_t)y * pitch) + x;
+    if ((reinterpret_cast<uintptr_t>(p) & (Load4<TI>::kAlign - 1)) == 0) return Load4<TI>::whole(p);
+    if (x >= ax_lo + 4 && x + 8 <= ax_hi) return Load4<TI>::shifted(p);
+  }
+  const int ry = remap(bmode, y, ay_lo, ay_hi);
+  const TI *row = reinterpret_cast<const TI *>(in + (int64_t)(ry == (int)0x80000000 ? ay_lo : ry) * pitch);
+  float f[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int rx = remap(bmode, x + q, ax_lo, ax_hi);
+    f[q] = (rx == (int)0x80000000 || ry == (int)0x80000000) ? cval : Storage<TI>::load(row + rx);
+  }
+  return make_float4(f[0], f[1], f[2], f[3]);
+}
+
+template <typename TI, int SW, int SH, int NT>
+__device__ __forceinline__ void stage_groups(float *tile, const char *in, int64_t pitch, int X0, int Y0, int ax_lo,
+                                             int ax_hi, int ay_lo, int ay_hi, int bmode, float cval) {
+  static_assert(SW % 4 == 0, "whole groups");
+  constexpr int G = SW / 4;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < SH * G; c += NT) {
+    const int r = c / G, k = c - r * G;
+    reinterpret_cast<float4 *>(tile)[c] =
+        load_group<TI>(in, pitch, X0 + 4 * k, Y0 + r, ax_lo, ax_hi, ay_lo, ay_hi, bmode, cval);
+  }
+}
+
+}  // namespace hgb
