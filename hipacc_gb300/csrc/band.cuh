@@ -58,4 +58,52 @@ __device__ __forceinline__ int preimages(int mode, int j, int n, int rad, int *o
   return k;
 }
 
+// The same pre-images, besides j itself, as bits: bit t < R stands for the
+// virtual position t - R, bit t >= R for n + t - R (no tap reaches farther).
+template <int R>
+__device__ __forceinline__ unsigned preimage_bits(int mode, int j, int n) {
+  unsigned m = 0;
+  if (mode == HGB_BOUNDARY_CONSTANT || (j >= R && j < n - R)) return 0;
+#pragma unroll
+  for (int t = 0; t < R; ++t) {
+    if (remap(mode, t - R, 0, n) == j) m |= 1u << t;
+    if (remap(mode, n + t, 0, n) == j) m |= 1u << (R + t);
+  }
+  return m;
+}
+template <int R>
+__device__ __forceinline__ int preimage_pos(int t, int n) { return t < R ? t - R : n + t - R; }
+
+// Band pixels (within R of an edge of the image) of a tw x th tile at (i0, j0),
+// for a CTA to take one per thread.
+struct TileBand {
+  int tw, th, top, bottom, left, right, count;
+};
+template <int R>
+__device__ __forceinline__ TileBand tile_band(int i0, int j0, int tw, int th, int W, int H, bool rows, bool cols) {
+  TileBand b;
+  b.tw = min(tw, W - i0);
+  b.th = min(th, H - j0);
+  b.top = rows ? min(b.th, max(0, R - j0)) : 0;
+  b.bottom = rows ? min(b.th - b.top, max(0, j0 + b.th - (H - R))) : 0;
+  b.left = cols ? min(b.tw, max(0, R - i0)) : 0;
+  b.right = cols ? min(b.tw - b.left, max(0, i0 + b.tw - (W - R))) : 0;
+  b.count = (b.top + b.bottom) * b.tw + (b.th - b.top - b.bottom) * (b.left + b.right);
+  return b;
+}
+__device__ __forceinline__ void tile_band_pos(const TileBand &b, int k, int &x, int &y) {  // tile-relative
+  const int full = (b.top + b.bottom) * b.tw;
+  if (k < full) {
+    y = k / b.tw;
+    x = k - y * b.tw;
+    if (y >= b.top) y += b.th - b.top - b.bottom;
+    return;
+  }
+  const int n = b.left + b.right, d = k - full;
+  y = d / n;
+  x = d - y * n;
+  y += b.top;
+  if (x >= b.left) x += b.tw - n;
+}
+
 }  // namespace hgb

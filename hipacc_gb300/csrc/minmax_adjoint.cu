@@ -11,10 +11,12 @@
 // mask weight for convolve.  Nothing flows when the initial value was never
 // replaced, or when the winning tap read the CONSTANT value outside the image.
 //
-// Two kernels, deterministic:
-//   1. minmax_select_kernel: per output, the winning tap (0 .. taps-1) or 0xFF,
+// Two kernels, deterministic, for any window (minmax_select_kernel,
+// minmax_gather_kernel) and on tiles for Domains of up to 7 x 7 cells
+// (minmax_select_tile_kernel, minmax_gather_tile_kernel):
+//   1. select: per output, the winning tap (0 .. taps-1) or 0xFF,
 //      into a byte per output in the library workspace;
-//   2. minmax_gather_kernel: per input pixel, the sum over every (virtual
+//   2. gather: per input pixel, the sum over every (virtual
 //      position that the boundary remap sends to it, tap) of the gradients of
 //      the outputs whose winner is that tap, in a fixed order: rows and
 //      columns of the pre-images ascending, then taps in row-major order.
@@ -22,7 +24,8 @@
 #include <cfloat>
 #include <cstring>
 
-#include "hgb_internal.cuh"
+#include "band.cuh"
+#include "stage_groups.cuh"
 
 namespace hgb {
 namespace {
@@ -118,6 +121,226 @@ __global__ void __launch_bounds__(MM_T) minmax_gather_kernel(const __grid_consta
   p.gin[(int64_t)b * p.gin_b + (int64_t)iy * p.gin_p + ix] = acc;
 }
 
+// ---------------------------------------------------------------- tiles
+// 64 x 32 pixels per CTA, a thread per 4 x 4.  The general kernels above spend
+// a remap and a global load on every tap of every pixel; here the tile and its
+// halo are staged once and a row's taps come from a register window.  Bound by
+// the ALU pipe: a compare and two selects per tap (select), a compare and a
+// predicated add per tap (gather).  Forward and adjoint of the 5 x 5 disc on 8
+// images of 509 x 381: 182 -> 47 us (host calls included); of the 7 x 7 disc on
+// 2309 x 2207: 778 -> 161 us.
+constexpr int MT_BX = 16, MT_NT = 128, MT_PY = 4, MT_TW = 64, MT_TH = 32, MT_SW = MT_TW + 8, MT_G = MT_SW / 4;
+
+struct MinMaxTileParams {
+  const float *in, *gout;
+  float *gin;
+  uint8_t *sel;
+  int64_t in_p, in_b, gout_p, gout_b, gin_p, gin_b;  // bytes
+  int64_t sel_p, sel_b;
+  int w, h, bmode;
+  float cval;
+  uint32_t flip;     // MAX runs as MIN of the negated values: every comparison has the same outcome
+  uint32_t rows[7];  // cells of the K x K window, a bit per column
+};
+
+__device__ __forceinline__ void window12(const float *row, float (&w)[12]) {
+#pragma unroll
+  for (int v = 0; v < 3; ++v) {
+    const float4 t = reinterpret_cast<const float4 *>(row)[v];
+    w[4 * v] = t.x;
+    w[4 * v + 1] = t.y;
+    w[4 * v + 2] = t.z;
+    w[4 * v + 3] = t.w;
+  }
+}
+
+template <int K>
+__global__ void __launch_bounds__(MT_NT) minmax_select_tile_kernel(const __grid_constant__ MinMaxTileParams p) {
+  constexpr int R = K / 2, SH = MT_TH + 2 * R;
+  __shared__ __align__(16) float tile[SH * MT_SW];
+  const int b = blockIdx.z, i0 = blockIdx.x * MT_TW, j0 = blockIdx.y * MT_TH;
+  stage_groups<float, MT_SW, SH, MT_NT>(tile, (const char *)p.in + b * p.in_b, p.in_p, i0 - 4, j0 - R, 0, p.w, 0, p.h,
+                                        p.bmode, p.cval);
+  __syncthreads();
+  const int tx = threadIdx.x % MT_BX, ty = threadIdx.x / MT_BX;
+  const float first = p.flip ? -FLT_MIN : FLT_MAX;
+  float acc[MT_PY][4];
+  int win[MT_PY][4];
+#pragma unroll
+  for (int oy = 0; oy < MT_PY; ++oy)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      acc[oy][q] = first;
+      win[oy][q] = MM_NONE;
+    }
+#pragma unroll
+  for (int r = 0; r < MT_PY + K - 1; ++r) {
+    float w[12];
+    window12(&tile[(ty * MT_PY + r) * MT_SW + tx * 4], w);
+#pragma unroll
+    for (int i = 0; i < 12; ++i) w[i] = __uint_as_float(__float_as_uint(w[i]) ^ p.flip);
+#pragma unroll
+    for (int oy = 0; oy < MT_PY; ++oy) {
+      const int my = r - oy;  // ascending in r: row-major order per output
+      if (my < 0 || my >= K) continue;
+#pragma unroll
+      for (int mx = 0; mx < K; ++mx) {
+        if (!(p.rows[my] >> mx & 1u)) continue;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float v = w[4 - R + mx + q];
+          const bool keep = acc[oy][q] < v;
+          acc[oy][q] = keep ? acc[oy][q] : v;
+          win[oy][q] = keep ? win[oy][q] : my * K + mx;
+        }
+      }
+    }
+  }
+  const int x = i0 + 4 * tx;
+  if (x >= p.w) return;
+#pragma unroll
+  for (int oy = 0; oy < MT_PY; ++oy) {
+    const int y = j0 + ty * MT_PY + oy;
+    if (y >= p.h) break;
+    if (p.bmode == HGB_BOUNDARY_CONSTANT && (x < R || x + 4 > p.w - R || y < R || y >= p.h - R)) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {  // a CONSTANT tap outside carries no gradient
+        const int my = win[oy][q] / K, ay = y + my - R, ax = x + q + (win[oy][q] - my * K) - R;
+        if (ay < 0 || ay >= p.h || ax < 0 || ax >= p.w) win[oy][q] = MM_NONE;
+      }
+    }
+    // rows of the byte plane start on words and are padded to whole words
+    *reinterpret_cast<uint32_t *>(p.sel + b * p.sel_b + y * p.sel_p + x) =
+        (uint32_t)win[oy][0] | (uint32_t)win[oy][1] << 8 | (uint32_t)win[oy][2] << 16 | (uint32_t)win[oy][3] << 24;
+  }
+}
+
+template <int K>
+__global__ void __launch_bounds__(MT_NT, 6) minmax_gather_tile_kernel(const __grid_constant__ MinMaxTileParams p) {
+  constexpr int R = K / 2, SH = MT_TH + 2 * R;
+  __shared__ __align__(16) float g[SH * MT_SW];
+  __shared__ __align__(16) int sel[SH * MT_SW];
+  const int b = blockIdx.z, i0 = blockIdx.x * MT_TW, j0 = blockIdx.y * MT_TH;
+  const char *gout = (const char *)p.gout + b * p.gout_b;
+  const uint8_t *selb = p.sel + b * p.sel_b;
+#pragma unroll 2
+  for (int c = threadIdx.x; c < SH * MT_G; c += MT_NT) {
+    const int r = c / MT_G, k = c - r * MT_G, x = i0 - 4 + 4 * k, y = j0 - R + r;
+    uint32_t s = 0xffffffffu;
+    if (y >= 0 && y < p.h && x >= 0 && x < p.w) s = __ldcg(reinterpret_cast<const uint32_t *>(selb + y * p.sel_p + x));
+    int4 v;
+    v.x = s & 0xffu;
+    v.y = x + 1 < p.w ? (int)(s >> 8 & 0xffu) : MM_NONE;
+    v.z = x + 2 < p.w ? (int)(s >> 16 & 0xffu) : MM_NONE;
+    v.w = x + 3 < p.w ? (int)(s >> 24) : MM_NONE;
+    reinterpret_cast<int4 *>(sel)[c] = v;
+    reinterpret_cast<float4 *>(g)[c] =
+        load_group<float>(gout, p.gout_p, x, y, 0, p.w, 0, p.h, HGB_BOUNDARY_CONSTANT, 0.0f);
+  }
+  __syncthreads();
+  const int tx = threadIdx.x % MT_BX, ty = threadIdx.x / MT_BX;
+  const int x = i0 + 4 * tx;
+  float acc[MT_PY][4];
+#pragma unroll
+  for (int oy = 0; oy < MT_PY; ++oy)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[oy][q] = 0.0f;
+#pragma unroll
+  for (int r = MT_PY + K - 2; r >= 0; --r) {  // tap rows ascending: output rows descending
+    float gw[12];
+    int sw[12];
+    window12(&g[(ty * MT_PY + r) * MT_SW + tx * 4], gw);
+    const int4 *srow = reinterpret_cast<const int4 *>(&sel[(ty * MT_PY + r) * MT_SW + tx * 4]);
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+      const int4 t = srow[v];
+      sw[4 * v] = t.x;
+      sw[4 * v + 1] = t.y;
+      sw[4 * v + 2] = t.z;
+      sw[4 * v + 3] = t.w;
+    }
+#pragma unroll
+    for (int oy = 0; oy < MT_PY; ++oy) {
+      const int my = oy + 2 * R - r;
+      if (my < 0 || my >= K) continue;
+#pragma unroll
+      for (int mx = 0; mx < K; ++mx) {
+        if (!(p.rows[my] >> mx & 1u)) continue;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)  // output column x + q - (mx - R)
+          if (sw[4 + R - mx + q] == my * K + mx) acc[oy][q] = __fadd_rn(acc[oy][q], gw[4 + R - mx + q]);
+      }
+    }
+  }
+#pragma unroll
+  for (int oy = 0; oy < MT_PY; ++oy) {
+    const int y = j0 + ty * MT_PY + oy;
+    if (x >= p.w || y >= p.h) break;
+    float *dst = reinterpret_cast<float *>((char *)p.gin + b * p.gin_b + y * p.gin_p) + x;
+    if (x + 4 <= p.w && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+      *reinterpret_cast<float4 *>(dst) = make_float4(acc[oy][0], acc[oy][1], acc[oy][2], acc[oy][3]);
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (x + q < p.w) dst[q] = acc[oy][q];
+    }
+  }
+  // ---- near a border: the virtual positions that the remap sends to a pixel
+  // add to its own sum, a band pixel per thread and only the taps that reach
+  // back into the image, from the staged tile where it holds the output (REPEAT
+  // reaches the other side).  Walking every tap of every position in the lane
+  // that owns the pixel made the border tiles the slowest: 87 us against
+  // 47 us for 8 images of 509 x 381, forward included.
+  if (p.bmode == HGB_BOUNDARY_CONSTANT) return;
+  const TileBand band = tile_band<R>(i0, j0, MT_TW, MT_TH, p.w, p.h, true, true);
+  if (band.count == 0) return;
+  __syncthreads();  // the pixels' own sums are in grad_in
+#pragma unroll 1
+  for (int k = threadIdx.x; k < band.count; k += MT_NT) {
+    int bx, by;
+    tile_band_pos(band, k, bx, by);
+    const int ix = i0 + bx, iy = j0 + by;
+    const unsigned px = preimage_bits<R>(p.bmode, ix, p.w), py = preimage_bits<R>(p.bmode, iy, p.h);
+    if (!(px | py)) continue;
+    float *dst = reinterpret_cast<float *>((char *)p.gin + b * p.gin_b + iy * p.gin_p) + ix;
+    float s = *dst;
+#pragma unroll 1
+    for (int a = -1; a < 2 * R; ++a) {
+      if (a >= 0 && !(py >> a & 1u)) continue;
+      const int vy = a < 0 ? iy : preimage_pos<R>(a, p.h);
+#pragma unroll 1
+      for (int c = a < 0 ? 0 : -1; c < 2 * R; ++c) {  // (itself, itself) is in the sum already
+        if (c >= 0 && !(px >> c & 1u)) continue;
+        const int vx = c < 0 ? ix : preimage_pos<R>(c, p.w);
+        const int m0 = max(0, vx + R - p.w + 1), m1 = min(K - 1, vx + R);  // columns of taps inside the image
+#pragma unroll 1
+        for (int my = max(0, vy + R - p.h + 1); my <= min(K - 1, vy + R); ++my) {
+          const int jy = vy - (my - R), ry = jy - (j0 - R);
+#pragma unroll 2
+          for (int mx = m0; mx <= m1; ++mx) {
+            const int jx = vx - (mx - R), rx = jx - (i0 - 4);
+            if (ry >= 0 && ry < SH && rx >= 0 && rx < MT_SW) {
+              if (sel[ry * MT_SW + rx] == my * K + mx) s = __fadd_rn(s, g[ry * MT_SW + rx]);
+            } else if (__ldcg(selb + jy * p.sel_p + jx) == my * K + mx) {
+              s = __fadd_rn(s, __ldg(reinterpret_cast<const float *>(gout + jy * p.gout_p) + jx));
+            }
+          }
+        }
+      }
+    }
+    *dst = s;
+  }
+}
+
+// The tiled form of a Domain of at most 7 x 7 cells: its window embedded in an
+// odd K x K one (tap numbers are private to the two kernels).
+template <int K>
+void launch_minmax_tiles(const MinMaxTileParams &p, int batch, cudaStream_t st) {
+  const dim3 grid(cdiv(p.w, MT_TW), cdiv(p.h, MT_TH), batch);
+  minmax_select_tile_kernel<K><<<grid, MT_NT, 0, st>>>(p);
+  minmax_gather_tile_kernel<K><<<grid, MT_NT, 0, st>>>(p);
+}
+
 }  // namespace
 }  // namespace hgb
 
@@ -169,14 +392,51 @@ extern "C" int hgb_local_op_minmax_adjoint(const hgb_view *in, const hgb_view *g
     p.mask[k] = mask ? mask[k] : 1.0f;
     p.dom[k] = domain ? (domain[k] != 0) : 1;
   }
+  cudaStream_t st = (cudaStream_t)stream;
   const int64_t npx = (int64_t)p.w * p.h;
+  const int span = std::max(std::max(mask_w, mask_h), 3), K = span | 1;
+  if (!mask && K <= 7 && cdiv(p.h, MT_TH) <= 65535) {
+    MinMaxTileParams t;
+    memset(&t, 0, sizeof(t));
+    t.in = p.in;
+    t.gout = p.gout;
+    t.gin = p.gin;
+    t.in_p = in->pitch;
+    t.in_b = in->batch_stride;
+    t.gout_p = grad_out->pitch;
+    t.gout_b = grad_out->batch_stride;
+    t.gin_p = grad_in->pitch;
+    t.gin_b = grad_in->batch_stride;
+    t.w = p.w;
+    t.h = p.h;
+    t.bmode = boundary;
+    t.cval = const_val;
+    t.flip = reduce == HGB_REDUCE_MAX ? 0x80000000u : 0u;
+    const int dx = K / 2 - mask_w / 2, dy = K / 2 - mask_h / 2;
+    for (int y = 0; y < mask_h; ++y)
+      for (int x = 0; x < mask_w; ++x)
+        if (p.dom[y * mask_w + x]) t.rows[y + dy] |= 1u << (x + dx);
+    t.sel_p = ((int64_t)p.w + 3) / 4 * 4;
+    t.sel_b = t.sel_p * p.h;
+    Workspace ws;
+    rc = workspace_get((size_t)t.sel_b * p.batch + 64, &ws);
+    if (rc) return rc;
+    t.sel = (uint8_t *)ws.base;
+    cudaEvent_t ev = before_launch(st);
+    if (K == 3)
+      launch_minmax_tiles<3>(t, p.batch, st);
+    else if (K == 5)
+      launch_minmax_tiles<5>(t, p.batch, st);
+    else
+      launch_minmax_tiles<7>(t, p.batch, st);
+    return after_launch("minmax_gather_tile_kernel", st, ev);
+  }
   const int64_t nblk = (npx + MM_T - 1) / MM_T;
   HGB_REQUIRE(nblk < (int64_t)0x7fffffff, "hgb_local_op_minmax_adjoint: image too large");
   Workspace ws;
   rc = workspace_get((size_t)npx * p.batch + 64, &ws);
   if (rc) return rc;
   p.sel = (uint8_t *)ws.base;
-  cudaStream_t st = (cudaStream_t)stream;
   const dim3 grid((unsigned)nblk, (unsigned)p.batch);
   cudaEvent_t ev = before_launch(st);
   minmax_select_kernel<<<grid, MM_T, 0, st>>>(p);

@@ -77,3 +77,21 @@ def test_domain_minmax_windows(gpu, oracle):
     ref = np.zeros((100, 160), np.float32)
     oracle.local_op(img, domain=DISC5, reduce=2, boundary=2, acc=acc, out=ref, iter_space=it)
     assert np.array_equal(_bits(out.cpu().numpy()), _bits(ref))
+
+
+@pytest.mark.parametrize("red", [1, 2])
+@pytest.mark.parametrize("boundary", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("name", ["square3", "disc5", "square7", "row7", "col5", "ring3"])
+def test_domain_minmax_adjoint_tiles(gpu, oracle, name, boundary, red):
+    """The tiled select / gather kernels at the edges of their 64 x 32 tiles and
+    on images smaller than the window (pre-images on both sides of the image);
+    small integers give ties.  At most 49 FP32 additions of a few pre-images
+    per pixel: 2e-6 relative (L2) against the FP64 gather."""
+    rng = np.random.default_rng(31 * boundary + red)
+    for h, w in [(2, 3)] + SIZES:
+        img = rng.integers(0, 9, (h, w)).astype(np.float32) if w % 2 else rng.random((h, w)).astype(np.float32)
+        gout = rng.normal(0, 1, (h, w)).astype(np.float32)
+        got = gpu.minmax_adjoint(torch.from_numpy(img).cuda(), torch.from_numpy(gout).cuda(), red, domain=DOMAINS[name],
+                                 boundary=boundary, const=0.5).cpu().numpy()
+        _, ref = oracle.minmax_adjoint(img, gout, red, domain=DOMAINS[name], boundary=boundary, const=0.5)
+        assert np.linalg.norm(got - ref) <= 2e-6 * max(np.linalg.norm(ref), 1e-30), (name, h, w)
