@@ -62,9 +62,22 @@ __device__ __forceinline__ int preimages(int mode, int j, int n, int rad, int *o
 // virtual position t - R, bit t >= R for n + t - R (no tap reaches farther).
 template <int R>
 __device__ __forceinline__ unsigned preimage_bits(int mode, int j, int n) {
-  unsigned m = 0;
   if (mode == HGB_BOUNDARY_CONSTANT || (j >= R && j < n - R)) return 0;
-#pragma unroll
+  unsigned m = 0;
+  if (n >= R) {  // no position is remapped twice
+    if (mode == HGB_BOUNDARY_MIRROR) {  // -1 - j, 2n - 1 - j
+      if (j < R) m = 1u << (R - 1 - j);
+      if (n - 1 - j < R) m |= 1u << (R + n - 1 - j);
+    } else if (mode == HGB_BOUNDARY_REPEAT) {  // j - n, j + n
+      if (n - j <= R) m = 1u << (R + j - n);
+      if (j < R) m |= 1u << (R + j);
+    } else {
+      if (j == 0) m = (1u << R) - 1u;
+      if (j == n - 1) m |= ((1u << R) - 1u) << R;
+    }
+    return m;
+  }
+#pragma unroll 1
   for (int t = 0; t < R; ++t) {
     if (remap(mode, t - R, 0, n) == j) m |= 1u << t;
     if (remap(mode, n + t, 0, n) == j) m |= 1u << (R + t);

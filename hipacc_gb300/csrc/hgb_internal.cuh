@@ -89,14 +89,22 @@ int check_window(const hgb_window &w, const hgb_view &v, const char *name);
 // Returns INT_MIN for CONSTANT out of range.
 __host__ __device__ __forceinline__ int remap(int mode, int idx, int lo, int hi) {
   if (idx >= lo && idx < hi) return idx;
+  // REPEAT and MIRROR: one step lands inside unless the window is narrower than
+  // the reach; the division and the loop are for that case only
   switch (mode) {
     case HGB_BOUNDARY_REPEAT: {
       const int w = hi - lo;
+      const int near = idx < lo ? idx + w : idx - w;
+      if (near >= lo && near < hi) return near;
       int r = (idx - lo) % w;
       if (r < 0) r += w;
       return lo + r;
     }
     case HGB_BOUNDARY_MIRROR:
+      {
+        const int near = (idx < lo ? lo : hi) * 2 - 1 - idx;
+        if (near >= lo && near < hi) return near;
+      }
       // bounded: each pass moves idx strictly closer to the window
       for (int it = 0; it < 64 && (idx < lo || idx >= hi); ++it) {
         if (idx >= hi) idx = hi - (idx + 1 - hi);

@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(MM_NT) minmax_kernel(const __grid_constant__ M
   for (int c = threadIdx.x; c < SH * G; c += MM_NT) {
     const int r = c / G, k = c - r * G;
     const float4 v = load_group<TI>(in, p.in_pitch, p.ax + i0 - HL + 4 * k, p.ay + j0 - R + r, p.ax, p.ax + p.aw, p.ay,
-                                    p.ay + p.ah, p.bmode, p.cval);
+                                    p.ay + p.ah, p.bmode, p.cval, R);
     const uint32_t u[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
     if constexpr (sizeof(TI) > 1) {
 #pragma unroll
@@ -187,13 +187,15 @@ __global__ void __launch_bounds__(MM_NT) minmax_kernel(const __grid_constant__ M
 
 template <typename TI, int K, uint32_t PROFILE>
 int launch_minmax(const MinMaxKernelParams &p, int batch, cudaStream_t st) {
-  // 64 x 64 tiles; 64 x 32 where the taller ones would not give every SM four CTAs
-  const bool tall = (int64_t)cdiv(p.iw, 64) * cdiv(p.ih, 64) * batch >= 4 * num_sms();
+  // 64 x 64 tiles; lower ones where those would not give every SM four CTAs
+  const int64_t cols = (int64_t)cdiv(p.iw, 64) * batch, want = 4 * num_sms();
   cudaEvent_t ev = before_launch(st);
-  if (tall)
+  if (cols * cdiv(p.ih, 64) >= want)
     minmax_kernel<TI, K, 8, PROFILE><<<dim3(cdiv(p.iw, 64), cdiv(p.ih, 64), batch), MM_NT, 0, st>>>(p);
-  else
+  else if (cols * cdiv(p.ih, 32) >= want)
     minmax_kernel<TI, K, 4, PROFILE><<<dim3(cdiv(p.iw, 64), cdiv(p.ih, 32), batch), MM_NT, 0, st>>>(p);
+  else
+    minmax_kernel<TI, K, 2, PROFILE><<<dim3(cdiv(p.iw, 64), cdiv(p.ih, 16), batch), MM_NT, 0, st>>>(p);
   return after_launch("minmax_kernel", st, ev);
 }
 

@@ -122,14 +122,15 @@ __global__ void __launch_bounds__(MM_T) minmax_gather_kernel(const __grid_consta
 }
 
 // ---------------------------------------------------------------- tiles
-// 64 x 32 pixels per CTA, a thread per 4 x 4.  The general kernels above spend
+// 64 x 8 PY pixels per CTA, a thread per 4 x PY (PY = 4, fewer on small
+// batches).  The general kernels above spend
 // a remap and a global load on every tap of every pixel; here the tile and its
 // halo are staged once and a row's taps come from a register window.  Bound by
 // the ALU pipe: a compare and two selects per tap (select), a compare and a
 // predicated add per tap (gather).  Forward and adjoint of the 5 x 5 disc on 8
-// images of 509 x 381: 182 -> 47 us (host calls included); of the 7 x 7 disc on
-// 2309 x 2207: 778 -> 161 us.
-constexpr int MT_BX = 16, MT_NT = 128, MT_PY = 4, MT_TW = 64, MT_TH = 32, MT_SW = MT_TW + 8, MT_G = MT_SW / 4;
+// images of 509 x 381: 183 -> 51 us (now its host calls); of the 7 x 7 disc on
+// 2309 x 2207: 779 -> 142 us.
+constexpr int MT_BX = 16, MT_NT = 128, MT_PAD = 3, MT_TW = 64, MT_SW = MT_TW + 8, MT_G = MT_SW / 4;
 
 struct MinMaxTileParams {
   const float *in, *gout;
@@ -140,7 +141,10 @@ struct MinMaxTileParams {
   int w, h, bmode;
   float cval;
   uint32_t flip;     // MAX runs as MIN of the negated values: every comparison has the same outcome
-  uint32_t rows[7];  // cells of the K x K window, a bit per column
+  // cells of the K x K window, a bit per column: row my at [my + MT_PAD], with
+  // empty rows on either side, so that a staged row finds its window row for
+  // each of a thread's outputs without a test
+  uint32_t rows[7 + 2 * MT_PAD];
 };
 
 __device__ __forceinline__ void window12(const float *row, float (&w)[12]) {
@@ -154,44 +158,47 @@ __device__ __forceinline__ void window12(const float *row, float (&w)[12]) {
   }
 }
 
-template <int K>
+template <int K, int PY>
 __global__ void __launch_bounds__(MT_NT) minmax_select_tile_kernel(const __grid_constant__ MinMaxTileParams p) {
-  constexpr int R = K / 2, SH = MT_TH + 2 * R;
+  constexpr int R = K / 2, MT_TH = 8 * PY, SH = MT_TH + 2 * R;
   __shared__ __align__(16) float tile[SH * MT_SW];
   const int b = blockIdx.z, i0 = blockIdx.x * MT_TW, j0 = blockIdx.y * MT_TH;
   stage_groups<float, MT_SW, SH, MT_NT>(tile, (const char *)p.in + b * p.in_b, p.in_p, i0 - 4, j0 - R, 0, p.w, 0, p.h,
-                                        p.bmode, p.cval);
+                                        p.bmode, p.cval, R);
   __syncthreads();
   const int tx = threadIdx.x % MT_BX, ty = threadIdx.x / MT_BX;
   const float first = p.flip ? -FLT_MIN : FLT_MAX;
-  float acc[MT_PY][4];
-  int win[MT_PY][4];
+  float acc[PY][4];
+  int win[PY][4];
 #pragma unroll
-  for (int oy = 0; oy < MT_PY; ++oy)
+  for (int oy = 0; oy < PY; ++oy)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       acc[oy][q] = first;
       win[oy][q] = MM_NONE;
     }
-#pragma unroll
-  for (int r = 0; r < MT_PY + K - 1; ++r) {
+  // rolled over the staged rows: the loop unrolled is 20 to 30 KB of code, and a
+  // CTA runs through it once, at the pace of instruction cache misses
+#pragma unroll 1
+  for (int r = 0; r < PY + K - 1; ++r) {
     float w[12];
-    window12(&tile[(ty * MT_PY + r) * MT_SW + tx * 4], w);
+    window12(&tile[(ty * PY + r) * MT_SW + tx * 4], w);
 #pragma unroll
     for (int i = 0; i < 12; ++i) w[i] = __uint_as_float(__float_as_uint(w[i]) ^ p.flip);
 #pragma unroll
-    for (int oy = 0; oy < MT_PY; ++oy) {
-      const int my = r - oy;  // ascending in r: row-major order per output
-      if (my < 0 || my >= K) continue;
+    for (int oy = 0; oy < PY; ++oy) {
+      const uint32_t bits = p.rows[r - oy + MT_PAD];  // window row r - oy, ascending in r: row-major per output
+      if (!bits) continue;
+      const int k0 = (r - oy) * K;
 #pragma unroll
       for (int mx = 0; mx < K; ++mx) {
-        if (!(p.rows[my] >> mx & 1u)) continue;
+        if (!(bits >> mx & 1u)) continue;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const float v = w[4 - R + mx + q];
           const bool keep = acc[oy][q] < v;
           acc[oy][q] = keep ? acc[oy][q] : v;
-          win[oy][q] = keep ? win[oy][q] : my * K + mx;
+          win[oy][q] = keep ? win[oy][q] : k0 + mx;
         }
       }
     }
@@ -199,8 +206,8 @@ __global__ void __launch_bounds__(MT_NT) minmax_select_tile_kernel(const __grid_
   const int x = i0 + 4 * tx;
   if (x >= p.w) return;
 #pragma unroll
-  for (int oy = 0; oy < MT_PY; ++oy) {
-    const int y = j0 + ty * MT_PY + oy;
+  for (int oy = 0; oy < PY; ++oy) {
+    const int y = j0 + ty * PY + oy;
     if (y >= p.h) break;
     if (p.bmode == HGB_BOUNDARY_CONSTANT && (x < R || x + 4 > p.w - R || y < R || y >= p.h - R)) {
 #pragma unroll
@@ -215,9 +222,60 @@ __global__ void __launch_bounds__(MT_NT) minmax_select_tile_kernel(const __grid_
   }
 }
 
-template <int K>
+// The band pixels of a gather tile.  S = float: added to the pixel's own sum in
+// grad_in; S = double: the whole sum, own taps included.
+template <int K, int SH, typename S>
+__device__ __forceinline__ void minmax_band(const MinMaxTileParams &p, const TileBand &band, int b, int i0, int j0,
+                                            const int *sel, const float *g, const uint8_t *selb, const char *gout) {
+  constexpr int R = K / 2;
+  constexpr bool whole = sizeof(S) == 8;
+  const int part = threadIdx.x % 4;  // a quarter of the window's rows each
+#pragma unroll 1
+  for (int k0 = 0; k0 < 4 * band.count; k0 += MT_NT) {
+    const int k = (k0 + (int)threadIdx.x) / 4;
+    int bx = 0, by = 0;
+    unsigned px = 0, py = 0;
+    if (k < band.count) {
+      tile_band_pos(band, k, bx, by);
+      px = preimage_bits<R>(p.bmode, i0 + bx, p.w);
+      py = preimage_bits<R>(p.bmode, j0 + by, p.h);
+    }
+    const int ix = i0 + bx, iy = j0 + by;
+    float *dst = reinterpret_cast<float *>((char *)p.gin + b * p.gin_b + iy * p.gin_p) + ix;
+    S s = S(0);
+    if (px | py) {
+      if (!whole && part == 0) s = (S)*dst;
+      for (unsigned ym = py << 1 | 1u; ym; ym &= ym - 1u) {  // bit 0: the row itself
+        const int vy = ym & 1u ? iy : preimage_pos<R>(__ffs((int)ym) - 2, p.h), lo = max(0, vy + R - p.h + 1);
+        const unsigned xs = (ym & 1u) && !whole ? px << 1 : px << 1 | 1u;
+#pragma unroll 1
+        for (int my = lo + ((part - lo) & 3); my <= min(K - 1, vy + R); my += 4) {
+          const int jy = vy - (my - R), ry = jy - (j0 - R);
+          for (unsigned xm = xs; xm; xm &= xm - 1u) {
+            const int vx = xm & 1u ? ix : preimage_pos<R>(__ffs((int)xm) - 2, p.w);
+            const int m1 = min(K - 1, vx + R);  // columns of taps inside the image
+#pragma unroll 2
+            for (int mx = max(0, vx + R - p.w + 1); mx <= m1; ++mx) {
+              const int jx = vx - (mx - R), rx = jx - (i0 - 4);
+              if (ry >= 0 && ry < SH && rx >= 0 && rx < MT_SW) {
+                if (sel[ry * MT_SW + rx] == my * K + mx) s += (S)g[ry * MT_SW + rx];
+              } else if (__ldcg(selb + jy * p.sel_p + jx) == my * K + mx) {
+                s += (S)__ldg(reinterpret_cast<const float *>(gout + jy * p.gout_p) + jx);
+              }
+            }
+          }
+        }
+      }
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if ((px | py) && part == 0) *dst = (float)s;
+  }
+}
+
+template <int K, int PY>
 __global__ void __launch_bounds__(MT_NT, 6) minmax_gather_tile_kernel(const __grid_constant__ MinMaxTileParams p) {
-  constexpr int R = K / 2, SH = MT_TH + 2 * R;
+  constexpr int R = K / 2, MT_TH = 8 * PY, SH = MT_TH + 2 * R;
   __shared__ __align__(16) float g[SH * MT_SW];
   __shared__ __align__(16) int sel[SH * MT_SW];
   const int b = blockIdx.z, i0 = blockIdx.x * MT_TW, j0 = blockIdx.y * MT_TH;
@@ -235,22 +293,22 @@ __global__ void __launch_bounds__(MT_NT, 6) minmax_gather_tile_kernel(const __gr
     v.w = x + 3 < p.w ? (int)(s >> 24) : MM_NONE;
     reinterpret_cast<int4 *>(sel)[c] = v;
     reinterpret_cast<float4 *>(g)[c] =
-        load_group<float>(gout, p.gout_p, x, y, 0, p.w, 0, p.h, HGB_BOUNDARY_CONSTANT, 0.0f);
+        load_group<float>(gout, p.gout_p, x, y, 0, p.w, 0, p.h, HGB_BOUNDARY_CONSTANT, 0.0f, 0);
   }
   __syncthreads();
   const int tx = threadIdx.x % MT_BX, ty = threadIdx.x / MT_BX;
   const int x = i0 + 4 * tx;
-  float acc[MT_PY][4];
+  float acc[PY][4];
 #pragma unroll
-  for (int oy = 0; oy < MT_PY; ++oy)
+  for (int oy = 0; oy < PY; ++oy)
 #pragma unroll
     for (int q = 0; q < 4; ++q) acc[oy][q] = 0.0f;
-#pragma unroll
-  for (int r = MT_PY + K - 2; r >= 0; --r) {  // tap rows ascending: output rows descending
+#pragma unroll 1
+  for (int r = PY + K - 2; r >= 0; --r) {  // tap rows ascending: output rows descending
     float gw[12];
     int sw[12];
-    window12(&g[(ty * MT_PY + r) * MT_SW + tx * 4], gw);
-    const int4 *srow = reinterpret_cast<const int4 *>(&sel[(ty * MT_PY + r) * MT_SW + tx * 4]);
+    window12(&g[(ty * PY + r) * MT_SW + tx * 4], gw);
+    const int4 *srow = reinterpret_cast<const int4 *>(&sel[(ty * PY + r) * MT_SW + tx * 4]);
 #pragma unroll
     for (int v = 0; v < 3; ++v) {
       const int4 t = srow[v];
@@ -260,21 +318,23 @@ __global__ void __launch_bounds__(MT_NT, 6) minmax_gather_tile_kernel(const __gr
       sw[4 * v + 3] = t.w;
     }
 #pragma unroll
-    for (int oy = 0; oy < MT_PY; ++oy) {
+    for (int oy = 0; oy < PY; ++oy) {
       const int my = oy + 2 * R - r;
-      if (my < 0 || my >= K) continue;
+      const uint32_t bits = p.rows[my + MT_PAD];
+      if (!bits) continue;
+      const int k0 = my * K;
 #pragma unroll
       for (int mx = 0; mx < K; ++mx) {
-        if (!(p.rows[my] >> mx & 1u)) continue;
+        if (!(bits >> mx & 1u)) continue;
 #pragma unroll
         for (int q = 0; q < 4; ++q)  // output column x + q - (mx - R)
-          if (sw[4 + R - mx + q] == my * K + mx) acc[oy][q] = __fadd_rn(acc[oy][q], gw[4 + R - mx + q]);
+          if (sw[4 + R - mx + q] == k0 + mx) acc[oy][q] = __fadd_rn(acc[oy][q], gw[4 + R - mx + q]);
       }
     }
   }
 #pragma unroll
-  for (int oy = 0; oy < MT_PY; ++oy) {
-    const int y = j0 + ty * MT_PY + oy;
+  for (int oy = 0; oy < PY; ++oy) {
+    const int y = j0 + ty * PY + oy;
     if (x >= p.w || y >= p.h) break;
     float *dst = reinterpret_cast<float *>((char *)p.gin + b * p.gin_b + y * p.gin_p) + x;
     if (x + 4 <= p.w && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
@@ -286,59 +346,44 @@ __global__ void __launch_bounds__(MT_NT, 6) minmax_gather_tile_kernel(const __gr
     }
   }
   // ---- near a border: the virtual positions that the remap sends to a pixel
-  // add to its own sum, a band pixel per thread and only the taps that reach
-  // back into the image, from the staged tile where it holds the output (REPEAT
-  // reaches the other side).  Walking every tap of every position in the lane
-  // that owns the pixel made the border tiles the slowest: 87 us against
-  // 47 us for 8 images of 509 x 381, forward included.
+  // add to its own sum, only the taps that reach back into the image, from the
+  // staged tile where it holds the output (REPEAT reaches the other side).
+  // Four lanes share a band pixel.  Walking every tap of every position in the
+  // lane that owns the pixel made the border tiles the slowest: 87 us against
+  // 51 us for 8 images of 509 x 381, forward included.  On images hardly wider
+  // than the window hundreds of terms meet in one pixel and cancel: there the
+  // whole sum is taken again, in FP64.
   if (p.bmode == HGB_BOUNDARY_CONSTANT) return;
   const TileBand band = tile_band<R>(i0, j0, MT_TW, MT_TH, p.w, p.h, true, true);
   if (band.count == 0) return;
-  __syncthreads();  // the pixels' own sums are in grad_in
-#pragma unroll 1
-  for (int k = threadIdx.x; k < band.count; k += MT_NT) {
-    int bx, by;
-    tile_band_pos(band, k, bx, by);
-    const int ix = i0 + bx, iy = j0 + by;
-    const unsigned px = preimage_bits<R>(p.bmode, ix, p.w), py = preimage_bits<R>(p.bmode, iy, p.h);
-    if (!(px | py)) continue;
-    float *dst = reinterpret_cast<float *>((char *)p.gin + b * p.gin_b + iy * p.gin_p) + ix;
-    float s = *dst;
-#pragma unroll 1
-    for (int a = -1; a < 2 * R; ++a) {
-      if (a >= 0 && !(py >> a & 1u)) continue;
-      const int vy = a < 0 ? iy : preimage_pos<R>(a, p.h);
-#pragma unroll 1
-      for (int c = a < 0 ? 0 : -1; c < 2 * R; ++c) {  // (itself, itself) is in the sum already
-        if (c >= 0 && !(px >> c & 1u)) continue;
-        const int vx = c < 0 ? ix : preimage_pos<R>(c, p.w);
-        const int m0 = max(0, vx + R - p.w + 1), m1 = min(K - 1, vx + R);  // columns of taps inside the image
-#pragma unroll 1
-        for (int my = max(0, vy + R - p.h + 1); my <= min(K - 1, vy + R); ++my) {
-          const int jy = vy - (my - R), ry = jy - (j0 - R);
-#pragma unroll 2
-          for (int mx = m0; mx <= m1; ++mx) {
-            const int jx = vx - (mx - R), rx = jx - (i0 - 4);
-            if (ry >= 0 && ry < SH && rx >= 0 && rx < MT_SW) {
-              if (sel[ry * MT_SW + rx] == my * K + mx) s = __fadd_rn(s, g[ry * MT_SW + rx]);
-            } else if (__ldcg(selb + jy * p.sel_p + jx) == my * K + mx) {
-              s = __fadd_rn(s, __ldg(reinterpret_cast<const float *>(gout + jy * p.gout_p) + jx));
-            }
-          }
-        }
-      }
-    }
-    *dst = s;
-  }
+  __syncthreads();  // the sums without the other pre-images are written
+  if (p.w < 2 * K || p.h < 2 * K)
+    minmax_band<K, SH, double>(p, band, b, i0, j0, sel, g, selb, gout);
+  else
+    minmax_band<K, SH, float>(p, band, b, i0, j0, sel, g, selb, gout);
 }
 
 // The tiled form of a Domain of at most 7 x 7 cells: its window embedded in an
-// odd K x K one (tap numbers are private to the two kernels).
+// odd K x K one (tap numbers are private to the two kernels).  Tiles are lower
+// where 32 rows would leave an SM fewer than eight CTAs: a thread runs through
+// a few thousand dependent instructions whatever the image, so a small image is
+// done sooner with fewer pixels per thread (140 x 131, three
+// calls as one graph: 37 -> 18 us).
+template <int K, int PY>
+void launch_minmax_tiles(const MinMaxTileParams &p, int batch, cudaStream_t st) {
+  const dim3 grid(cdiv(p.w, MT_TW), cdiv(p.h, 8 * PY), batch);
+  minmax_select_tile_kernel<K, PY><<<grid, MT_NT, 0, st>>>(p);
+  minmax_gather_tile_kernel<K, PY><<<grid, MT_NT, 0, st>>>(p);
+}
 template <int K>
 void launch_minmax_tiles(const MinMaxTileParams &p, int batch, cudaStream_t st) {
-  const dim3 grid(cdiv(p.w, MT_TW), cdiv(p.h, MT_TH), batch);
-  minmax_select_tile_kernel<K><<<grid, MT_NT, 0, st>>>(p);
-  minmax_gather_tile_kernel<K><<<grid, MT_NT, 0, st>>>(p);
+  const int64_t cols = (int64_t)cdiv(p.w, MT_TW) * batch, want = 8 * num_sms();
+  if (cols * cdiv(p.h, 32) >= want)
+    launch_minmax_tiles<K, 4>(p, batch, st);
+  else if (cols * cdiv(p.h, 16) >= want)
+    launch_minmax_tiles<K, 2>(p, batch, st);
+  else
+    launch_minmax_tiles<K, 1>(p, batch, st);
 }
 
 }  // namespace
@@ -395,7 +440,7 @@ extern "C" int hgb_local_op_minmax_adjoint(const hgb_view *in, const hgb_view *g
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t npx = (int64_t)p.w * p.h;
   const int span = std::max(std::max(mask_w, mask_h), 3), K = span | 1;
-  if (!mask && K <= 7 && cdiv(p.h, MT_TH) <= 65535) {
+  if (!mask && K <= 7 && cdiv(p.h, 8) <= 65535) {
     MinMaxTileParams t;
     memset(&t, 0, sizeof(t));
     t.in = p.in;
@@ -415,7 +460,7 @@ extern "C" int hgb_local_op_minmax_adjoint(const hgb_view *in, const hgb_view *g
     const int dx = K / 2 - mask_w / 2, dy = K / 2 - mask_h / 2;
     for (int y = 0; y < mask_h; ++y)
       for (int x = 0; x < mask_w; ++x)
-        if (p.dom[y * mask_w + x]) t.rows[y + dy] |= 1u << (x + dx);
+        if (p.dom[y * mask_w + x]) t.rows[y + dy + MT_PAD] |= 1u << (x + dx);
     t.sel_p = ((int64_t)p.w + 3) / 4 * 4;
     t.sel_b = t.sel_p * p.h;
     Workspace ws;

@@ -71,21 +71,25 @@ template <typename T> struct Load4Half {
 template <> struct Load4<__nv_bfloat16> : Load4Half<__nv_bfloat16> {};
 template <> struct Load4<__half> : Load4Half<__half> {};
 
-// The group of columns [x, x + 4) of row y of the window.
+// The group of columns [x, x + 4) of row y of the window.  Cells farther than
+// `reach` outside the window serve no output and read the constant (a tile that
+// overhangs a small image would spend most of its staging on them).
 template <typename TI>
 __device__ __forceinline__ float4 load_group(const char *in, int64_t pitch, int x, int y, int ax_lo, int ax_hi,
-                                             int ay_lo, int ay_hi, int bmode, float cval) {
+                                             int ay_lo, int ay_hi, int bmode, float cval, int reach) {
   if (y >= ay_lo && y < ay_hi && x >= ax_lo && x + 4 <= ax_hi) {
     const TI *p = reinterpret_cast<const TI *>(in + (int64_t)y * pitch) + x;
     if ((reinterpret_cast<uintptr_t>(p) & (Load4<TI>::kAlign - 1)) == 0) return Load4<TI>::whole(p);
     if (x >= ax_lo + 4 && x + 8 <= ax_hi) return Load4<TI>::shifted(p);
   }
+  if (x + 3 < ax_lo - reach || x >= ax_hi + reach || y < ay_lo - reach || y >= ay_hi + reach)
+    return make_float4(cval, cval, cval, cval);
   const int ry = remap(bmode, y, ay_lo, ay_hi);
   const TI *row = reinterpret_cast<const TI *>(in + (int64_t)(ry == (int)0x80000000 ? ay_lo : ry) * pitch);
   float f[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    const int rx = remap(bmode, x + q, ax_lo, ax_hi);
+    const int rx = x + q >= ax_hi + reach ? (int)0x80000000 : remap(bmode, x + q, ax_lo, ax_hi);
     f[q] = (rx == (int)0x80000000 || ry == (int)0x80000000) ? cval : Storage<TI>::load(row + rx);
   }
   return make_float4(f[0], f[1], f[2], f[3]);
@@ -93,14 +97,15 @@ __device__ __forceinline__ float4 load_group(const char *in, int64_t pitch, int 
 
 template <typename TI, int SW, int SH, int NT>
 __device__ __forceinline__ void stage_groups(float *tile, const char *in, int64_t pitch, int X0, int Y0, int ax_lo,
-                                             int ax_hi, int ay_lo, int ay_hi, int bmode, float cval) {
+                                             int ax_hi, int ay_lo, int ay_hi, int bmode, float cval,
+                                             int reach) {
   static_assert(SW % 4 == 0, "whole groups");
   constexpr int G = SW / 4;
 #pragma unroll 4
   for (int c = threadIdx.x; c < SH * G; c += NT) {
     const int r = c / G, k = c - r * G;
     reinterpret_cast<float4 *>(tile)[c] =
-        load_group<TI>(in, pitch, X0 + 4 * k, Y0 + r, ax_lo, ax_hi, ay_lo, ay_hi, bmode, cval);
+        load_group<TI>(in, pitch, X0 + 4 * k, Y0 + r, ax_lo, ax_hi, ay_lo, ay_hi, bmode, cval, reach);
   }
 }
 
