@@ -23,6 +23,7 @@
 #include <cstring>
 
 #include "band.cuh"
+#include "line_adjoint.h"
 #include "reduce_common.cuh"
 #include "tma.cuh"
 
@@ -547,6 +548,48 @@ extern "C" int hgb_local_op_adjoint(const hgb_view *in, const hgb_view *grad_out
   p.grad_mask_dev = grad_mask_dev;
   cudaStream_t st = (cudaStream_t)stream;
   const int K = mask_w;
+  if ((mask_h == 1 && line_adjoint_size(mask_w)) || (mask_w == 1 && line_adjoint_size(mask_h))) {
+    // line masks: the tiled kernels of line_adjoint_kernels.cuh
+    const LineForm form = mask_h == 1 ? kLineRow : kLineCol;
+    const int n = mask_h == 1 ? mask_w : mask_h;
+    LineAdjParams l;
+    memset(&l, 0, sizeof(l));
+    l.in = grad_mask_dev ? p.in : nullptr;
+    l.in_p = in ? in->pitch : 0;
+    l.in_b = in ? in->batch_stride : 0;
+    l.gout = p.gout;
+    l.gout_p = grad_out->pitch;
+    l.gout_b = grad_out->batch_stride;
+    if (grad_in) {
+      l.gin = p.gin;
+      l.gin_p = grad_in->pitch;
+      l.gin_b = grad_in->batch_stride;
+    }
+    l.w = p.w;
+    l.h = p.h;
+    l.batch = p.batch;
+    l.bmode = boundary;
+    l.mask_dev = mask_dev;
+    memcpy(l.mask, p.mask, n * sizeof(float));
+    const int grid = line_adjoint_grid(form, n, mask_dev != nullptr, p.w, p.h, p.batch);
+    LineCombine c;
+    memset(&c, 0, sizeof(c));
+    if (grad_mask_dev) {
+      Workspace ws;
+      rc = workspace_get((size_t)n * grid * sizeof(float) + 64, &ws);
+      if (rc) return rc;
+      l.part = (float *)ws.base;
+      c.part[0] = l.part;
+      c.out[0] = grad_mask_dev;
+      c.taps[0] = n;
+      c.nparts[0] = grid;
+    }
+    cudaEvent_t ev = before_launch(st);
+    rc = run_line_adjoint(form, n, &l, grid, st);
+    if (rc) return rc;
+    if (grad_mask_dev) run_line_combine(c, st);
+    return after_launch("line_adjoint", st, ev);
+  }
   if (grad_in && grad_mask_dev && mask_w == mask_h && (K == 3 || K == 5 || K == 7) && p.w >= 8 && p.h >= 8 &&
       tma_legal(p.gout, grad_out->pitch, grad_out->batch_stride, p.batch) &&
       tma_legal(p.in, in->pitch, in->batch_stride, p.batch)) {
