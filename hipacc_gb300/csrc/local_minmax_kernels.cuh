@@ -52,25 +52,23 @@ __host__ __device__ constexpr uint32_t disc_profile(int k) {  // x^2 + y^2 <= (k
 
 template <typename TI, int K, int PY, uint32_t PROFILE>
 __global__ void __launch_bounds__(MM_NT) minmax_kernel(const __grid_constant__ MinMaxKernelParams p) {
-  constexpr int R = K / 2, HL = 4, TW = MM_BX * MM_PX, TH = MM_BY * PY, SW = TW + 2 * HL, SH = TH + 2 * R, G = SW / 4;
+  constexpr int R = K / 2, HL = 4, TW = MM_BX * MM_PX, TH = MM_BY * PY, SW = TW + 2 * HL, SH = TH + 2 * R;
   __shared__ __align__(16) float tile[SH * SW];
   const int b = blockIdx.z, i0 = blockIdx.x * TW, j0 = blockIdx.y * TH;
   const char *in = p.in + (int64_t)b * p.in_bstride;
   const uint32_t flip = p.flip;
   // ---- stage, with the sign of MAX; note NaNs and negative zeros
   int odd = 0;
-#pragma unroll 4
-  for (int c = threadIdx.x; c < SH * G; c += MM_NT) {
-    const int r = c / G, k = c - r * G;
-    const float4 v = load_group<TI>(in, p.in_pitch, p.ax + i0 - HL + 4 * k, p.ay + j0 - R + r, p.ax, p.ax + p.aw, p.ay,
-                                    p.ay + p.ah, p.bmode, p.cval, R);
+  auto put = [&](int c, float4 v) {
     const uint32_t u[4] = {__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w)};
     if constexpr (sizeof(TI) > 1) {
 #pragma unroll
       for (int q = 0; q < 4; ++q) odd |= (u[q] == 0x80000000u) | ((u[q] & 0x7fffffffu) > 0x7f800000u);
     }
     reinterpret_cast<uint4 *>(tile)[c] = make_uint4(u[0] ^ flip, u[1] ^ flip, u[2] ^ flip, u[3] ^ flip);
-  }
+  };
+  stage_groups_each<TI, SW, SH, MM_NT>(in, p.in_pitch, p.ax + i0 - HL, p.ay + j0 - R, p.ax, p.ax + p.aw, p.ay,
+                                       p.ay + p.ah, p.bmode, p.cval, R, put);
   if constexpr (sizeof(TI) == 1) {  // bytes are neither; the constant may be
     const uint32_t u = __float_as_uint(p.cval);
     odd = u == 0x80000000u || (u & 0x7fffffffu) > 0x7f800000u;

@@ -95,18 +95,56 @@ __device__ __forceinline__ float4 load_group(const char *in, int64_t pitch, int 
   return make_float4(f[0], f[1], f[2], f[3]);
 }
 
+// Every group of the tile to put(c, values), c = row * (SW / 4) + group, NT
+// threads.  A tile that lies inside the window with four columns to spare takes
+// its addresses by adding to one pointer and tests nothing per group: the tests,
+// the division and the 64-bit products of the general loop are about 30
+// instructions a group, several per pixel.
+template <typename TI, int SW, int SH, int NT, typename F>
+__device__ __forceinline__ void stage_groups_each(const char *in, int64_t pitch, int X0, int Y0, int ax_lo, int ax_hi,
+                                                  int ay_lo, int ay_hi, int bmode, float cval, int reach, F put) {
+  static_assert(SW % 4 == 0, "whole groups");
+  constexpr int G = SW / 4, ES = (int)sizeof(TI);
+  int r = threadIdx.x / G, k = threadIdx.x - r * G;
+  if (X0 - 4 >= ax_lo && X0 + SW + 4 <= ax_hi && Y0 >= ay_lo && Y0 + SH <= ay_hi) {
+    const char *p = in + (int64_t)(Y0 + r) * pitch + (int64_t)(X0 + 4 * k) * ES;
+    const int64_t step = (int64_t)(NT / G) * pitch + (NT % G) * 4 * ES, wrap = pitch - G * 4 * ES;
+    const uint64_t bits = reinterpret_cast<uint64_t>(in) | (uint64_t)pitch | (uint64_t)((int64_t)X0 * ES);
+    auto run = [&](auto load) {
+#pragma unroll 4
+      for (int c = threadIdx.x; c < SH * G; c += NT) {
+        put(c, load(reinterpret_cast<const TI *>(p)));
+        k += NT % G;
+        p += step;
+        if (k >= G) {
+          k -= G;
+          p += wrap;
+        }
+      }
+    };
+    if ((bits & (uint64_t)(Load4<TI>::kAlign - 1)) == 0)
+      run([](const TI *q) { return Load4<TI>::whole(q); });
+    else
+      run([](const TI *q) { return Load4<TI>::shifted(q); });
+    return;
+  }
+#pragma unroll 2
+  for (int c = threadIdx.x; c < SH * G; c += NT) {
+    put(c, load_group<TI>(in, pitch, X0 + 4 * k, Y0 + r, ax_lo, ax_hi, ay_lo, ay_hi, bmode, cval, reach));
+    k += NT % G;
+    r += NT / G;
+    if (k >= G) {
+      k -= G;
+      ++r;
+    }
+  }
+}
+
 template <typename TI, int SW, int SH, int NT>
 __device__ __forceinline__ void stage_groups(float *tile, const char *in, int64_t pitch, int X0, int Y0, int ax_lo,
-                                             int ax_hi, int ay_lo, int ay_hi, int bmode, float cval,
-                                             int reach) {
-  static_assert(SW % 4 == 0, "whole groups");
-  constexpr int G = SW / 4;
-#pragma unroll 4
-  for (int c = threadIdx.x; c < SH * G; c += NT) {
-    const int r = c / G, k = c - r * G;
-    reinterpret_cast<float4 *>(tile)[c] =
-        load_group<TI>(in, pitch, X0 + 4 * k, Y0 + r, ax_lo, ax_hi, ay_lo, ay_hi, bmode, cval, reach);
-  }
+                                             int ax_hi, int ay_lo, int ay_hi, int bmode, float cval, int reach) {
+  stage_groups_each<TI, SW, SH, NT>(in, pitch, X0, Y0, ax_lo, ax_hi, ay_lo, ay_hi, bmode, cval, reach,
+                                    [tile](int c, float4 v) { reinterpret_cast<float4 *>(tile)[c] = v; });
 }
 
 }  // namespace hgb
