@@ -12,11 +12,9 @@
 //   R  = (float)(Gx Gy - Gxy^2) - (k (float)(Gx + Gy)) (float)(Gx + Gy),
 //        every float operation rounded separately;  out = R > threshold ? 1 : 0
 // Every local operator reads through the boundary remap (CONSTANT taps read
-// 0).  Fused form: one kernel per 64 x 16 tile stages the u8 input with a
-// 2-pixel halo, forms the products on the tile plus a 1-pixel halo in shared
-// memory (a halo cell outside the image holds the products at its remapped
-// position, as the Gaussian reads them), and writes the 0/1 image: 1 byte in
-// and 1 byte out per pixel instead of the nine launches' short intermediates.
+// 0; the Gaussian reads the products at their remapped positions).  Fused form:
+// one kernel stages the u8 input with a 2-pixel halo, keeps the products in
+// registers and writes the 0/1 image: 1 byte in and 1 byte out per pixel instead of the nine launches' short intermediates.
 //
 // Unsharp (samples-public/1_Local_Operators/Unsharp/src/main.cpp:53-149,203-247,
 // 3x3): five kernels in the reference --
@@ -42,15 +40,13 @@
 #include <cstring>
 #include <mutex>
 
-#include "hgb_internal.cuh"
+#include "band.cuh"
+#include "stage_groups.cuh"
 
 namespace hgb {
 namespace {
 
 // ------------------------------------------------------------------ Harris
-constexpr int HC_TW = 64, HC_TH = 16, HC_T = 256;
-constexpr int HC_IW = HC_TW + 4, HC_IH = HC_TH + 4;  // staged input, 2-pixel halo
-constexpr int HC_DW = HC_TW + 2, HC_DH = HC_TH + 2;  // products, 1-pixel halo
 
 struct HarrisParams {
   const uint8_t *in;
@@ -93,60 +89,178 @@ __device__ __forceinline__ uint8_t hc_response(const HarrisParams &p, int gx, in
   return R > p.threshold ? 1 : 0;
 }
 
-__global__ void __launch_bounds__(HC_T) harris_fused_kernel(const __grid_constant__ HarrisParams p) {
-  __shared__ uint8_t s_in[HC_IH * HC_IW];
-  __shared__ int s_sx[HC_DH * HC_DW], s_sy[HC_DH * HC_DW], s_sxy[HC_DH * HC_DW];
-  const int b = blockIdx.z, X0 = blockIdx.x * HC_TW, Y0 = blockIdx.y * HC_TH;
-  const uint8_t *img = p.in + (int64_t)b * p.in_b;
-  const bool inside = X0 - 2 >= 0 && X0 + HC_TW + 2 <= p.w && Y0 - 2 >= 0 && Y0 + HC_TH + 2 <= p.h;
-  for (int c = threadIdx.x; c < HC_IH * HC_IW; c += HC_T) {
-    const int r = c / HC_IW, q = c - r * HC_IW;
-    s_in[c] = inside ? __ldg(img + (int64_t)(Y0 - 2 + r) * p.in_p + X0 - 2 + q)
-                     : (uint8_t)hc_in(p, img, X0 - 2 + q, Y0 - 2 + r);
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < HC_DH * HC_DW; c += HC_T) {
-    const int r = c / HC_DW, q = c - r * HC_DW;
-    const int vx = X0 - 1 + q, vy = Y0 - 1 + r;
-    int v[3][3];
-    int16_t dx = 0, dy = 0;
-    if (vx >= 0 && vx < p.w && vy >= 0 && vy < p.h) {
+// Fused form.  Pixels at least two from every edge need no boundary: their
+// whole 5 x 5 neighbourhood lies in the image.  A warp walks 128 columns of
+// TR rows of a staged byte tile, a lane four columns: per row the derivative
+// sums on six columns, their quotients, products, the Gaussian's row sums, and
+// from three of those the response of the row two above.  Everything up to the
+// sixteenths is an integer below 2^24, held exactly in FP32 and computed two
+// columns per packed f32x2 operation; the sixteenths truncate by rounding a
+// value moved to the middle of its step (x / 16 - 15/32, toward zero for either
+// sign).  The two-pixel frame takes four lanes per pixel and the
+// boundary rule at every read, in the grid's first CTAs.
+//
+// Bound by instruction issue.  One pixel per thread with 27 shared 4-byte reads
+// and int products took 90 us for 4032 x 3024; this takes 51 us (HBM floor 3.6 us).
+constexpr int HT_W = 128, HT_NT = 128, HT_SW = HT_W + 8;  // tile and staged bytes per row
+
+__device__ __forceinline__ f2 f2_both(float v) { return f2_pack(v, v); }
+
+// x / 6 truncated toward zero, |x| <= 765 (each lane): 1 / 6 rounds up in FP32,
+// so a multiple of six does not fall below its quotient, and the next quotient is
+// at least 1 / 6 away.  The truncation runs on the conversion unit, which is idle
+// otherwise.
+__device__ __forceinline__ f2 hc_sixth(f2 x) {
+  const f2 t = f2_mul(x, f2_both(0.166666672f));
+  return f2_pack(truncf(f2_lo(t)), truncf(f2_hi(t)));
+}
+
+// 1 where the response of the sixteen-fold Gaussian sums exceeds the threshold;
+// u = sum / 16 + 1.5 * 2^23 (the integer sits in the low mantissa bits), tr = gx + gy
+__device__ __forceinline__ uint32_t hc_corner(float k, float threshold, float uxf, float uyf, float uxyf, float tr) {
+  const int gx = __float_as_int(uxf) - 0x4B400000, gy = __float_as_int(uyf) - 0x4B400000,
+            gxy = __float_as_int(uxyf) - 0x4B400000;
+  const float det = __int2float_rn(gx * gy - gxy * gxy);
+  return __fsub_rn(det, __fmul_rn(__fmul_rn(k, tr), tr)) > threshold ? 1u : 0u;
+}
+
+// the response at a pixel with the boundary rule at every read, by four lanes (a
+// row of products each): the Gaussian reads the products at their remapped
+// positions (CONSTANT: 0)
+__device__ __forceinline__ uint8_t hc_frame_pixel(const HarrisParams &p, const uint8_t *img, int x, int y, int part) {
+  int a = 0, bb = 0, cc = 0;
+  const int uy = remap(p.bmode, y - 1 + part, 0, p.h);
+  if (part < 3 && uy != (int)0x80000000) {
+#pragma unroll 1
+    for (int dj = 0; dj < 3; ++dj) {
+      const int ux = remap(p.bmode, x - 1 + dj, 0, p.w);
+      if (ux == (int)0x80000000) continue;
+      int v[3][3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
+      for (int r = 0; r < 3; ++r)
 #pragma unroll
-        for (int j = 0; j < 3; ++j) v[i][j] = s_in[(r + i) * HC_IW + q + j];
+        for (int c = 0; c < 3; ++c) v[r][c] = hc_in(p, img, ux - 1 + c, uy - 1 + r);
+      int16_t dx, dy;
       hc_deriv(v, dx, dy);
-    } else if (p.bmode != HGB_BOUNDARY_CONSTANT) {
-      // the Gaussian reads the products at the remapped position
-      const int ux = remap(p.bmode, vx, 0, p.w), uy = remap(p.bmode, vy, 0, p.h);
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) v[i][j] = hc_in(p, img, ux - 1 + j, uy - 1 + i);
-      hc_deriv(v, dx, dy);
+      const int m = (part == 1 ? 2 : 1) * (dj == 1 ? 2 : 1);
+      a += (int16_t)(dx * dx) * m;
+      bb += (int16_t)(dy * dy) * m;
+      cc += (int16_t)(dx * dy) * m;
     }
-    s_sx[c] = (int16_t)(dx * dx);
-    s_sy[c] = (int16_t)(dy * dy);
-    s_sxy[c] = (int16_t)(dx * dy);
   }
-  __syncthreads();
-  const int tx = threadIdx.x % HC_TW;
+#pragma unroll
+  for (int d = 1; d < 4; d <<= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, d);
+    bb += __shfl_xor_sync(0xffffffffu, bb, d);
+    cc += __shfl_xor_sync(0xffffffffu, cc, d);
+  }
+  return hc_response(p, (int16_t)(a / 16), (int16_t)(bb / 16), (int16_t)(cc / 16));
+}
+
+template <int TR>
+__global__ void __launch_bounds__(HT_NT) harris_fused_kernel(const __grid_constant__ HarrisParams p, int tiles_x,
+                                                             int nframe) {
+  constexpr int TH = 4 * TR, SH = TH + 4, G = HT_SW / 4;
+  __shared__ __align__(16) uint32_t tile[SH * G];
+  const int b = blockIdx.z;
+  const uint8_t *img = p.in + (int64_t)b * p.in_b;
   uint8_t *out = p.out + (int64_t)b * p.out_b;
-  for (int py = threadIdx.x / HC_TW; py < HC_TH; py += HC_T / HC_TW) {
-    const int x = X0 + tx, y = Y0 + py;
-    if (x >= p.w || y >= p.h) continue;
-    int a = 0, bb = 0, cc = 0;
+  if ((int)blockIdx.x < nframe) {  // the frame, first: its threads take longest
+    const TileBand f = tile_band<2>(0, 0, p.w, p.h, p.w, p.h, true, true);
+    const int k = (blockIdx.x * HT_NT + threadIdx.x) / 4, part = threadIdx.x % 4;
+    int x = 0, y = 0;
+    if (k < f.count) tile_band_pos(f, k, x, y);
+    const uint8_t v = hc_frame_pixel(p, img, x, y, part);
+    if (k < f.count && part == 0) out[(int64_t)y * p.out_p + x] = v;
+    return;
+  }
+  const int t = (int)blockIdx.x - nframe, X0 = (t % tiles_x) * HT_W, Y0 = (t / tiles_x) * TH;
+  // bytes outside the image reach no pixel stored below
+  stage_words<G, SH, HT_NT>(tile, img, p.in_p, X0 - 4, Y0 - 2, p.w, p.h);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int x = X0 + 4 * lane, y0 = Y0 + warp * TR;
+  // rolling state of the last two rows: input (columns x - 2 .. x + 5 as biased
+  // floats 2^23 + byte; only differences are taken), column differences, and the
+  // Gaussian's row sums of the three products
+  f2 in[2][4], E[2][3], H[2][3][2];
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
+  for (int l = 0; l < 2; ++l) {
 #pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const int m = (i == 1 ? 2 : 1) * (j == 1 ? 2 : 1);
-        const int o = (py + i) * HC_DW + tx + j;
-        a += s_sx[o] * m;
-        bb += s_sy[o] * m;
-        cc += s_sxy[o] * m;
+    for (int i = 0; i < 4; ++i) in[l][i] = 0ull;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      E[l][i] = 0ull;
+      H[l][i][0] = H[l][i][1] = 0ull;
+    }
+  }
+  const uint32_t *src = &tile[warp * TR * G + lane];
+  auto row = [&](int r, int l) {  // l: parity of r, the slot of the row two above
+    const uint32_t w0 = src[r * G], w1 = src[r * G + 1], w2 = src[r * G + 2];
+    auto byte = [](uint32_t w, int q) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + q)); };
+    const f2 v[4] = {f2_pack(byte(w0, 2), byte(w0, 3)), f2_pack(byte(w1, 0), byte(w1, 1)),
+                     f2_pack(byte(w1, 2), byte(w1, 3)), f2_pack(byte(w2, 0), byte(w2, 1))};
+    f2 e[3], P[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) e[i] = f2_sub(v[i + 1], v[i]);
+    f2 d[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d[i] = f2_sub(v[i], in[l][i]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const f2 dx = hc_sixth(f2_add(f2_add(E[l][i], E[l ^ 1][i]), e[i]));
+      const f2 mid = f2_pack(f2_hi(d[i]), f2_lo(d[i + 1]));
+      const f2 dy = hc_sixth(f2_add(f2_add(d[i], mid), d[i + 1]));
+      P[0][i] = f2_mul(dx, dx);
+      P[1][i] = f2_mul(dy, dy);
+      P[2][i] = f2_mul(dx, dy);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) in[l][i] = v[i];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) E[l][i] = e[i];
+    f2 u[3][2];
+    const f2 two = f2_both(2.0f), sixteenth = f2_both(0.0625f), m = f2_both(12582912.0f);
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const f2 mid = f2_pack(f2_hi(P[a][i]), f2_lo(P[a][i + 1]));
+        const f2 h = f2_fma(two, mid, f2_add(P[a][i], P[a][i + 1]));
+        const f2 s = f2_fma(two, H[l ^ 1][a][i], f2_add(H[l][a][i], h));
+        H[l][a][i] = h;
+        f2 half;
+        if (a < 2) {  // sums of squares: not negative
+          half = f2_both(-0.46875f);
+        } else {
+          const uint32_t n = 0xBEF00000u;  // -0.46875f
+          half = f2_pack(__uint_as_float((__float_as_uint(f2_lo(s)) & 0x80000000u) ^ n),
+                         __uint_as_float((__float_as_uint(f2_hi(s)) & 0x80000000u) ^ n));
+        }
+        u[a][i] = f2_add(f2_fma(s, sixteenth, half), m);
       }
-    out[(int64_t)y * p.out_p + x] = hc_response(p, (int16_t)(a / 16), (int16_t)(bb / 16), (int16_t)(cc / 16));
+    const int y = y0 + r - 4;
+    if (r < 4 || y < 2 || y >= p.h - 2) return;
+    uint32_t o = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const f2 tr = f2_add(f2_sub(u[0][i], m), f2_sub(u[1][i], m));
+      o |= hc_corner(p.k, p.threshold, f2_lo(u[0][i]), f2_lo(u[1][i]), f2_lo(u[2][i]), f2_lo(tr)) << (16 * i);
+      o |= hc_corner(p.k, p.threshold, f2_hi(u[0][i]), f2_hi(u[1][i]), f2_hi(u[2][i]), f2_hi(tr)) << (16 * i + 8);
+    }
+    uint8_t *dst = out + (int64_t)y * p.out_p + x;
+    if (x >= 2 && x + 4 <= p.w - 2 && (reinterpret_cast<uintptr_t>(dst) & 3u) == 0) {
+      *reinterpret_cast<uint32_t *>(dst) = o;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (x + q >= 2 && x + q < p.w - 2) dst[q] = (uint8_t)(o >> (8 * q));
+    }
+  };
+#pragma unroll 1
+  for (int r = 0; r < TR + 4; r += 2) {
+    row(r, 0);
+    row(r + 1, 1);
   }
 }
 
@@ -452,8 +566,22 @@ extern "C" int hgb_harris_corner(const hgb_view *in, const hgb_view *out, float 
   p.threshold = threshold;
   cudaStream_t st = (cudaStream_t)stream;
   if (mode == 0) {
+    const int tiles_x = cdiv(p.w, HT_W);
+    const int64_t edge = 4 * ((int64_t)p.w + p.h);  // at least the frame's pixels
+    const int frame = (int)((4 * std::min<int64_t>(edge, (int64_t)p.w * p.h) + HT_NT - 1) / HT_NT);
+    // 64-row tiles (16 rows per warp, 4 more to start from) where they give every
+    // SM four CTAs, else 16-row ones (the time of a small image is the chain of
+    // rows that a warp walks); 128-row tiles are slower (one wave of uneven CTAs,
+    // 60 us against 51 us for 4032 x 3024)
+    const bool tall = (int64_t)tiles_x * cdiv(p.h, 64) * in->batch >= 4 * num_sms();
+    const int64_t ntiles = (int64_t)tiles_x * cdiv(p.h, tall ? 64 : 16);
+    HGB_REQUIRE(ntiles + frame < 0x7fffffff, "hgb_harris_corner: image too large");
+    const dim3 grid((unsigned)(ntiles + frame), 1, in->batch);
     cudaEvent_t ev = before_launch(st);
-    harris_fused_kernel<<<dim3(cdiv(p.w, HC_TW), cdiv(p.h, HC_TH), in->batch), HC_T, 0, st>>>(p);
+    if (tall)
+      harris_fused_kernel<16><<<grid, HT_NT, 0, st>>>(p, tiles_x, frame);
+    else
+      harris_fused_kernel<4><<<grid, HT_NT, 0, st>>>(p, tiles_x, frame);
     return after_launch("harris_fused_kernel", st, ev);
   }
   const size_t px = (size_t)p.w * p.h * in->batch;

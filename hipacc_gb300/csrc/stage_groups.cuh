@@ -147,4 +147,61 @@ __device__ __forceinline__ void stage_groups(float *tile, const char *in, int64_
                                     [tile](int c, float4 v) { reinterpret_cast<float4 *>(tile)[c] = v; });
 }
 
+// The same for a byte tile kept as words; bytes outside the image read 0.
+template <int G, int SH, int NT>
+__device__ __forceinline__ void stage_words(uint32_t *tile, const uint8_t *img, int64_t pitch, int X0, int Y0, int w,
+                                            int h) {
+  int r = threadIdx.x / G, k = threadIdx.x - r * G;
+  if (X0 - 4 >= 0 && X0 + 4 * G + 4 <= w && Y0 >= 0 && Y0 + SH <= h) {
+    const uint8_t *p = img + (int64_t)(Y0 + r) * pitch + X0 + 4 * k;
+    const int64_t step = (int64_t)(NT / G) * pitch + (NT % G) * 4, wrap = pitch - G * 4;
+    const uint64_t bits = reinterpret_cast<uint64_t>(img) | (uint64_t)pitch | (uint64_t)(int64_t)X0;
+    auto run = [&](auto load) {
+#pragma unroll 4
+      for (int c = threadIdx.x; c < SH * G; c += NT) {
+        tile[c] = load(p);
+        k += NT % G;
+        p += step;
+        if (k >= G) {
+          k -= G;
+          p += wrap;
+        }
+      }
+    };
+    if ((bits & 3u) == 0)
+      run([](const uint8_t *q) { return __ldg(reinterpret_cast<const uint32_t *>(q)); });
+    else
+      run([](const uint8_t *q) {
+        const unsigned s = (unsigned)(reinterpret_cast<uintptr_t>(q) & 3u);
+        const uint32_t *u = reinterpret_cast<const uint32_t *>(q - s);
+        return __funnelshift_r(__ldg(u), __ldg(u + 1), 8 * s);
+      });
+    return;
+  }
+#pragma unroll 2
+  for (int c = threadIdx.x; c < SH * G; c += NT) {
+    const int x = X0 + 4 * k, y = Y0 + r;
+    uint32_t v = 0;
+    if (y >= 0 && y < h && x + 3 >= 0 && x < w) {
+      const uint8_t *q = img + (int64_t)y * pitch + x;
+      const unsigned s = (unsigned)(reinterpret_cast<uintptr_t>(q) & 3u);
+      if (x >= 4 && x + 8 <= w) {
+        const uint32_t *u = reinterpret_cast<const uint32_t *>(q - s);
+        v = __funnelshift_r(__ldg(u), __ldg(u + 1), 8 * s);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (x + i >= 0 && x + i < w) v |= (uint32_t)__ldg(q + i) << (8 * i);
+      }
+    }
+    tile[c] = v;
+    k += NT % G;
+    r += NT / G;
+    if (k >= G) {
+      k -= G;
+      ++r;
+    }
+  }
+}
+
 }  // namespace hgb
