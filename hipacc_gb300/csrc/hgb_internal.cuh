@@ -190,6 +190,13 @@ __device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
   return d;
 }
 
+// a * b rounded on its own.  ptxas contracts mul.rn.f32x2, and fma.rn.f32x2 with a
+// -0 that it can see, with the add.rn.f32x2 that uses it (the scalar .rn forms
+// stay apart): `negative_zeros` has to come from memory, a kernel parameter say.
+// Adding -0 changes no product.
+__device__ __forceinline__ f2 f2_mul_rounded(f2 a, f2 b, f2 negative_zeros) { return f2_fma(a, b, negative_zeros); }
+constexpr f2 kNegativeZeros = 0x8000000080000000ull;
+
 // unpack 16 bytes of storage into floats
 template <typename T> struct Vec16;
 template <> struct Vec16<float> {

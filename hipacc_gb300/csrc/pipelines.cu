@@ -32,8 +32,7 @@
 // is reproduced by an exact float-float sum; a pixel whose sum lies within a
 // tiny margin of a float rounding midpoint (about 1 in 10^5) is recomputed in
 // FP64, so the result equals the double evaluation bit for bit.  Fused form:
-// one kernel per 32 x 16 tile stages the luminance with a 1-pixel halo and
-// writes the uchar4 result: 8 bytes per pixel instead of the five launches'
+// one kernel reads and writes 8 bytes per pixel instead of the five launches'
 // float intermediates.
 #include <algorithm>
 #include <cmath>
@@ -322,11 +321,9 @@ __global__ void __launch_bounds__(256) harris_response_kernel(const __grid_const
 }
 
 // ------------------------------------------------------------------ Unsharp
-constexpr int US_TW = 32, US_TH = 16, US_T = 256;
-constexpr int US_GW = US_TW + 2, US_GH = US_TH + 2;
-
 // luminance terms per byte value (host-computed, see the header comment)
 struct UnsTables {
+  float p[256];           // powf(v, c)
   float t0[256];          // 0.2126f * powf(v, c)
   float b1h[256], b1l[256];  // 0.7152 * powf(v, c) as a float pair
   float b2h[256], b2l[256];  // 0.0722 * powf(v, c) as a float pair
@@ -339,7 +336,8 @@ struct UnsharpParams {
   uchar4 *out;
   int64_t out_p, out_b;
   int w, h, bmode;
-  int tiles_x, tiles_y, ntiles;
+  int batch;
+  f2 nz;  // kNegativeZeros (f2_mul_rounded)
   const UnsTables *tab;  // device copy
   // plain launch structure: float intermediates [image][h][w]
   float *gray, *blur, *sharp, *ratio;
@@ -401,42 +399,196 @@ __device__ __forceinline__ uchar4 uns_load(const UnsharpParams &p, const uchar4 
   return cst ? make_uchar4(0, 0, 0, 0) : img[(int64_t)ry * p.in_p + rx];
 }
 
-__global__ void __launch_bounds__(US_T) unsharp_fused_kernel(const __grid_constant__ UnsharpParams p) {
-  __shared__ float t0[256], b1h[256], b1l[256], b2h[256], b2l[256];
-  __shared__ float s_g[US_GH * US_GW];
-  __shared__ uchar4 s_px[US_TH * US_TW];
-  const UnsTables &T = *p.tab;
-  for (int i = threadIdx.x; i < 256; i += US_T) {
-    t0[i] = T.t0[i];
-    b1h[i] = T.b1h[i];
-    b1l[i] = T.b1l[i];
-    b2h[i] = T.b2h[i];
-    b2l[i] = T.b2l[i];
+// Fused form.  A warp walks down a strip of 120 columns, a lane four columns
+// (the outer two lanes only supply the strip's halo), and keeps everything but
+// the power table in registers: the gray of a row is formed once, its products
+// with the mask's three weights once, and each output row adds the nine products
+// in the reference's order as its three rows pass (two partial sums roll along).
+// Additions and products run on two pixels per packed f32x2 operation.
+//
+// The power table is a copy per lane, entry v of lane l at word 32 v + l, so the
+// three lookups of a pixel hit 32 banks whatever the bytes; the products 0.7152 p
+// and 0.0722 p come from p as exact float pairs instead of four more tables (one
+// shared copy of five tables cost about 17 shared-memory cycles per pixel row of
+// a warp against 3).  The warps of one wave share the rows of the strips evenly.
+//
+// Bound by instruction issue.  One pixel per thread over 32 x 16 tiles took
+// 120 us for 4032 x 3024; this takes 55 us (HBM floor 14.4 us).
+constexpr int UF_NT = 256, UF_COLS = 120;
+
+// (float)(((double)(0.2126f p_r) + 0.7152 p_g) + 0.0722 p_b) of two pixels w0, w1
+__device__ __forceinline__ f2 uns_gray2(const float *tab, const UnsTables *T, f2 nz, uint32_t w0, uint32_t w1) {
+  // tab: the lane's column of the table
+  auto look = [tab](uint32_t w0, uint32_t w1, int k) {
+    return f2_pack(tab[((w0 >> (8 * k)) & 255u) * 32], tab[((w1 >> (8 * k)) & 255u) * 32]);
+  };
+  auto both = [](float v) { return f2_pack(v, v); };
+  constexpr float g_hi = (float)0.7152, g_lo = (float)(0.7152 - (double)(float)0.7152);
+  constexpr float b_hi = (float)0.0722, b_lo = (float)(0.0722 - (double)(float)0.0722);
+  const f2 pr = look(w0, w1, 0), pg = look(w0, w1, 1), pb = look(w0, w1, 2);
+  const f2 a = f2_mul_rounded(both(0.2126f), pr, nz);
+  // c p as a pair: hi = fl(c_hi p), lo = (c_hi p - hi) + c_lo p
+  const f2 gh = f2_mul_rounded(both(g_hi), pg, nz), bh = f2_mul_rounded(both(b_hi), pb, nz);
+  const f2 gl = f2_sub(f2_mul(both(g_lo), pg), f2_fma(both(-g_hi), pg, gh));
+  const f2 bl = f2_sub(f2_mul(both(b_lo), pb), f2_fma(both(-b_hi), pb, bh));
+  auto two_sum2 = [](f2 x, f2 y, f2 &s, f2 &e) {
+    s = f2_add(x, y);
+    const f2 yy = f2_sub(s, x);
+    e = f2_add(f2_sub(x, f2_sub(s, yy)), f2_sub(y, yy));
+  };
+  f2 s1, e1, s, e2;
+  two_sum2(a, gh, s1, e1);
+  two_sum2(s1, bh, s, e2);
+  const f2 e = f2_add(f2_add(e1, e2), f2_add(gl, bl));
+  f2 y2 = f2_add(s, e);
+  const f2 rho2 = f2_add(f2_sub(s, y2), e);  // what the rounding to y took away
+  float y[2] = {f2_lo(y2), f2_hi(y2)};
+  const float rho[2] = {f2_lo(rho2), f2_hi(rho2)};
+  bool redo[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    // within 2^-40 of a rounding midpoint, or at a power of two (whose lower
+    // midpoint is nearer): evaluate in double
+    const uint32_t u = __float_as_uint(y[i]);
+    const float half = __uint_as_float(u & 0x7f800000u) * 5.9604644775390625e-8f;  // half an ulp
+    redo[i] = (__fmaf_rn(y[i], 9.094947017729282e-13f, fabsf(rho[i])) >= half || (u & 0x007fffffu) == 0) && y[i] != 0.0f;
   }
-  // persistent: the CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...
-  for (int t = blockIdx.x; t < p.ntiles; t += gridDim.x) {
-    const int per = p.tiles_x * p.tiles_y;
-    const int b = t / per, r0 = t - b * per;
-    const int Y0 = (r0 / p.tiles_x) * US_TH, X0 = (r0 % p.tiles_x) * US_TW;
-    const uchar4 *img = p.in + (int64_t)b * p.in_b;
-    __syncthreads();  // tables staged / the previous tile's reads done
-    for (int c = threadIdx.x; c < US_GH * US_GW; c += US_T) {
-      const int r = c / US_GW, q = c - r * US_GW;
-      bool cst;
-      const uchar4 v = uns_load(p, img, X0 - 1 + q, Y0 - 1 + r, cst);
-      s_g[c] = cst ? 0.0f : uns_gray(T, t0, b1h, b1l, b2h, b2l, v.x, v.y, v.z);
-      if (r >= 1 && r <= US_TH && q >= 1 && q <= US_TW) s_px[(r - 1) * US_TW + q - 1] = v;
+  if (redo[0] || redo[1]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t w = i ? w1 : w0;
+      if (redo[i])
+        y[i] = (float)__dadd_rn(__dadd_rn((double)__ldg(&T->t0[w & 255u]), __ldg(&T->b1[w >> 8 & 255u])),
+                                __ldg(&T->b2[w >> 16 & 255u]));
     }
-    __syncthreads();
-    const int tx = threadIdx.x % US_TW;
-    uchar4 *out = p.out + (int64_t)b * p.out_b;
-    for (int py = threadIdx.x / US_TW; py < US_TH; py += US_T / US_TW) {
-      const int x = X0 + tx, y = Y0 + py;
-      if (x >= p.w || y >= p.h) continue;
-      const float g = s_g[(py + 1) * US_GW + tx + 1];
-      const float ratio = uns_ratio(g, uns_blur(&s_g[py * US_GW + tx], US_GW));
-      out[(int64_t)y * p.out_p + x] = uns_scale(s_px[py * US_TW + tx], ratio);
+    y2 = f2_pack(y[0], y[1]);
+  }
+  return y2;
+}
+
+__device__ __forceinline__ uint32_t uns_scale_word(uint32_t v, float r) {
+  // (uchar)(channel * r): truncated to an int, low byte kept; alpha copied
+  uint32_t o = v;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float c = __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440 + k)) - 8388608.0f;
+    const uint32_t t = (uint32_t)__float2int_rz(__fmul_rn(c, r));
+    o = __byte_perm(o, t, k == 0 ? 0x3214 : (k == 1 ? 0x3240 : 0x3410));
+  }
+  return o;
+}
+
+__global__ void __launch_bounds__(UF_NT) unsharp_fused_kernel(const __grid_constant__ UnsharpParams p, int strips,
+                                                              int rows_per, int segments) {
+  __shared__ __align__(16) float tab[256 * 32];
+#pragma unroll
+  for (int i = threadIdx.x; i < 256 * 8; i += UF_NT) {
+    const float v = __ldg(&p.tab->p[i >> 3]);
+    reinterpret_cast<float4 *>(tab)[i] = make_float4(v, v, v, v);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const float *tl = tab + lane;
+  const int64_t job = (int64_t)blockIdx.x * (UF_NT / 32) + (threadIdx.x >> 5);
+  const int b = (int)(job / ((int64_t)strips * segments)), jr = (int)(job - (int64_t)b * strips * segments);
+  if (b >= p.batch) return;
+  const int seg = jr / strips, x = (jr - seg * strips) * UF_COLS - 4 + 4 * lane;  // this lane's columns
+  const int y0 = seg * rows_per, y1 = min(y0 + rows_per, p.h);
+  const uint32_t *img = reinterpret_cast<const uint32_t *>(p.in) + (int64_t)b * p.in_b;
+  uint32_t *out = reinterpret_cast<uint32_t *>(p.out) + (int64_t)b * p.out_b;
+  const bool whole = x >= 0 && x + 4 <= p.w;
+  const bool stores = lane > 0 && lane < 31 && x < p.w;
+  bool in_col[4] = {true, true, true, true};  // false: a CONSTANT column, gray 0
+  int cx[4] = {x, x + 1, x + 2, x + 3};
+  if (!whole) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      // columns past the halo serve no pixel: any valid address will do
+      const int rx = x + q > p.w ? p.w - 1 : (x + q < -1 ? 0 : remap(p.bmode, x + q, 0, p.w));
+      in_col[q] = rx != (int)0x80000000;
+      cx[q] = in_col[q] ? rx : 0;
     }
+  }
+  auto load = [&](int ry, uint32_t (&w)[4]) {
+    const uint32_t *row = img + (int64_t)ry * p.in_p;
+    if (whole && (reinterpret_cast<uintptr_t>(row + x) & 15u) == 0) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + x));
+      w[0] = v.x;
+      w[1] = v.y;
+      w[2] = v.z;
+      w[3] = v.w;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) w[q] = __ldg(row + cx[q]);
+    }
+  };
+  const float m0 = 0.057118f, m1 = 0.124758f, m2 = 0.272496f;
+  auto both = [](float v) { return f2_pack(v, v); };
+  f2 one[2] = {0ull, 0ull}, two[2] = {0ull, 0ull};  // partial sums after one and two rows of their windows
+  f2 gp[2] = {0ull, 0ull};                          // gray of the row above
+  uint32_t wp[4] = {0, 0, 0, 0}, wn[4];
+  {
+    const int r0 = remap(p.bmode, y0 - 1, 0, p.h);
+    load(r0 == (int)0x80000000 ? 0 : r0, wn);
+  }
+#pragma unroll 1
+  for (int y = y0 - 1; y <= y1; ++y) {
+    uint32_t w[4] = {wn[0], wn[1], wn[2], wn[3]};
+    const bool row_in = (y >= 0 && y < p.h) || p.bmode != HGB_BOUNDARY_CONSTANT;
+    if (y < y1) {  // the next row's loads are in flight while this one computes
+      const int rn = remap(p.bmode, y + 1, 0, p.h);
+      load(rn == (int)0x80000000 ? 0 : rn, wn);
+    }
+    f2 g[2] = {uns_gray2(tl, p.tab, p.nz, w[0], w[1]), uns_gray2(tl, p.tab, p.nz, w[2], w[3])};
+    if (p.bmode == HGB_BOUNDARY_CONSTANT && (!row_in || !whole)) {
+      float v[4] = {f2_lo(g[0]), f2_hi(g[0]), f2_lo(g[1]), f2_hi(g[1])};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) v[q] = row_in && in_col[q] ? v[q] : 0.0f;
+      g[0] = f2_pack(v[0], v[1]);
+      g[1] = f2_pack(v[2], v[3]);
+    }
+    const float left = __shfl_up_sync(0xffffffffu, f2_hi(g[1]), 1);
+    const float right = __shfl_down_sync(0xffffffffu, f2_lo(g[0]), 1);
+    // columns (-1, 0), (1, 2), (3, 4) relative to x
+    const f2 go[3] = {f2_pack(left, f2_lo(g[0])), f2_pack(f2_hi(g[0]), f2_lo(g[1])), f2_pack(f2_hi(g[1]), right)};
+    f2 a0[3], a1[3], c1[2], c2[2];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      a0[i] = f2_mul_rounded(both(m0), go[i], p.nz);
+      a1[i] = f2_mul_rounded(both(m1), go[i], p.nz);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      c1[i] = f2_mul_rounded(both(m1), g[i], p.nz);
+      c2[i] = f2_mul_rounded(both(m2), g[i], p.nz);
+    }
+    f2 blur[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      // this row as the last of the window above, the middle of the next, the first of the one below
+      blur[i] = f2_add(f2_add(f2_add(two[i], a0[i]), c1[i]), a0[i + 1]);
+      two[i] = f2_add(f2_add(f2_add(one[i], a1[i]), c2[i]), a1[i + 1]);
+      one[i] = f2_add(f2_add(f2_add(0ull, a0[i]), c1[i]), a0[i + 1]);
+    }
+    if (y > y0 && stores) {  // the window centred on row y - 1 is complete
+      const float gv[4] = {f2_lo(gp[0]), f2_hi(gp[0]), f2_lo(gp[1]), f2_hi(gp[1])};
+      const float bv[4] = {f2_lo(blur[0]), f2_hi(blur[0]), f2_lo(blur[1]), f2_hi(blur[1])};
+      uint32_t o[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) o[q] = uns_scale_word(wp[q], uns_ratio(gv[q], bv[q]));
+      uint32_t *dst = out + (int64_t)(y - 1) * p.out_p + x;
+      if (x + 4 <= p.w && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
+        *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (x + q < p.w) dst[q] = o[q];
+      }
+    }
+    gp[0] = g[0];
+    gp[1] = g[1];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) wp[q] = w[q];
   }
 }
 
@@ -510,6 +662,7 @@ int unsharp_tables(const UnsTables **out) {
     const float c = 1.0f / 2.2f;
     for (int v = 0; v < 256; ++v) {
       const float pv = powf((float)v, c);
+      g_uns_host.p[v] = pv;
       g_uns_host.t0[v] = 0.2126f * pv;
       const double d1 = 0.7152 * (double)pv, d2 = 0.0722 * (double)pv;
       g_uns_host.b1[v] = d1;
@@ -635,16 +788,25 @@ extern "C" int hgb_unsharp(const hgb_view *in, const hgb_view *out, int boundary
   p.w = in->width;
   p.h = in->height;
   p.bmode = boundary;
+  p.batch = in->batch;
+  p.nz = kNegativeZeros;
   rc = unsharp_tables(&p.tab);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   if (mode == 0) {
-    p.tiles_x = cdiv(p.w, US_TW);
-    p.tiles_y = cdiv(p.h, US_TH);
-    p.ntiles = p.tiles_x * p.tiles_y * in->batch;
-    const int grid = std::min(p.ntiles, num_sms() * std::max(1, resident_ctas((const void *)unsharp_fused_kernel, US_T, 0)));
+    // one wave of warps shares the rows of the strips; a segment recomputes the
+    // gray of two rows besides its own, so it has at least two (on an image that
+    // leaves most of the GPU idle, shorter segments end sooner)
+    const int strips = cdiv(p.w, UF_COLS);
+    const int64_t warps = (int64_t)num_sms() * resident_ctas((const void *)unsharp_fused_kernel, UF_NT, 0) * (UF_NT / 32);
+    const int64_t columns = (int64_t)strips * in->batch;
+    int64_t segments = std::max<int64_t>(1, warps / columns);
+    const int rows_per = std::max(2, (int)((p.h + segments - 1) / segments));
+    segments = cdiv(p.h, rows_per);
+    const int64_t ctas = (columns * segments + UF_NT / 32 - 1) / (UF_NT / 32);
+    HGB_REQUIRE(ctas < 0x7fffffff, "hgb_unsharp: image too large");
     cudaEvent_t ev = before_launch(st);
-    unsharp_fused_kernel<<<grid, US_T, 0, st>>>(p);
+    unsharp_fused_kernel<<<(unsigned)ctas, UF_NT, 0, st>>>(p, strips, rows_per, (int)segments);
     return after_launch("unsharp_fused_kernel", st, ev);
   }
   const size_t px = (size_t)p.w * p.h * in->batch;
