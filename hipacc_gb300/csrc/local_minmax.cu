@@ -1,5 +1,6 @@
 // local_minmax.cu -- dispatch of the tiled MIN / MAX over a Domain
 // (local_minmax_kernels.cuh).
+#include <algorithm>
 #include <cstring>
 
 #include "local_minmax.h"
@@ -50,6 +51,7 @@ int run_minmax_domain(const hgb_view &in, const hgb_window &acc, const hgb_view 
   p.ih = is.height;
   p.bmode = boundary;
   p.cval = cval;
+  p.excess = std::max(0, std::max(is.width - acc.width, is.height - acc.height));
   p.flip = reduce == HGB_REDUCE_MAX ? 0x80000000u : 0u;
   p.d = d;
   const int64_t four = 4 * es;  // bytes of a thread's four outputs

@@ -28,6 +28,7 @@ struct MinMaxKernelParams {
   int ix, iy, iw, ih;  // iteration space
   int bmode, vec_out;
   float cval;
+  int excess;          // how far the iteration space exceeds the accessor window
   uint32_t flip;       // 0x80000000 for MAX: values and result change sign
   MinMaxDomain d;
 };

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(MM_NT) minmax_kernel(const __grid_constant__ M
     reinterpret_cast<uint4 *>(tile)[c] = make_uint4(u[0] ^ flip, u[1] ^ flip, u[2] ^ flip, u[3] ^ flip);
   };
   stage_groups_each<TI, SW, SH, MM_NT>(in, p.in_pitch, p.ax + i0 - HL, p.ay + j0 - R, p.ax, p.ax + p.aw, p.ay,
-                                       p.ay + p.ah, p.bmode, p.cval, R, put);
+                                       p.ay + p.ah, p.bmode, p.cval, R + p.excess, put);
   if constexpr (sizeof(TI) == 1) {  // bytes are neither; the constant may be
     const uint32_t u = __float_as_uint(p.cval);
     odd = u == 0x80000000u || (u & 0x7fffffffu) > 0x7f800000u;

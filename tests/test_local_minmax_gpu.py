@@ -79,6 +79,20 @@ def test_domain_minmax_windows(gpu, oracle):
     assert np.array_equal(_bits(out.cpu().numpy()), _bits(ref))
 
 
+@pytest.mark.parametrize("boundary", [1, 2, 3, 4])
+def test_domain_minmax_space_larger_than_window(gpu, oracle, boundary):
+    """Outputs beyond the accessor window read through the boundary at any distance."""
+    rng = np.random.default_rng(boundary)
+    img = rng.random((90, 150)).astype(np.float32)
+    out = torch.zeros((100, 160), device="cuda")
+    acc, it = (11, 7, 40, 30), (3, 5, 75, 61)
+    gpu.local_op(torch.from_numpy(img).cuda(), out, domain=DISC5, reduce=2, boundary=boundary, acc=acc, iter_space=it,
+                 const=0.3)
+    ref = np.zeros((100, 160), np.float32)
+    oracle.local_op(img, domain=DISC5, reduce=2, boundary=boundary, acc=acc, out=ref, iter_space=it, const=0.3)
+    assert np.array_equal(_bits(out.cpu().numpy()), _bits(ref))
+
+
 @pytest.mark.parametrize("red", [1, 2])
 @pytest.mark.parametrize("boundary", [0, 1, 2, 3, 4])
 @pytest.mark.parametrize("name", ["square3", "disc5", "square7", "row7", "col5", "ring3"])
