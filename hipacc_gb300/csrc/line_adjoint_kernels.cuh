@@ -17,7 +17,7 @@
 // t = rows(in) is recomputed in shared memory (the forward's operations and
 // order) instead of written to memory and read back.
 // Forward and adjoint of the separable filter: K = 9 on 4 images of 1920 x 1080
-// 502 -> 114 us, K = 5 on 4096 x 2048 689 -> 97 us.
+// 485 -> 87 us, K = 5 on 4096 x 2048 689 -> 97 us.
 //
 // Included by line_k3_9.cu and line_k11_15.cu, which compile in parallel.
 #pragma once
@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(LN_NT) line_adjoint_kernel(const __grid_consta
     if (p.part)
       stage_groups<float, SWI, SH, LN_NT>(si, (const char *)p.in + b * p.in_b, p.in_p, kT ? i0 - HL : gx, gy, 0, p.w, 0,
                                           p.h, p.bmode, kT ? p.cval : 0.0f, R);
+    stage_wait();
     __syncthreads();
     if (kT && p.part) {  // t = rows(in) on the staged rows
       for (int c = threadIdx.x; c < SH * (LN_TW / 4); c += LN_NT) {

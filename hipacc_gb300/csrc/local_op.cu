@@ -1,5 +1,6 @@
 // local_op.cu -- hgb_local_op: argument checks, mask padding, dispatch between
 // the register-blocked fast kernels and the general kernel, tile autotuning.
+#include <algorithm>
 #include <cstring>
 
 #include "autotune.h"
@@ -13,8 +14,6 @@ namespace hgb {
 int num_tile_cfgs() { return 3; }
 
 namespace {
-
-int vec_elems(int dt) { return 16 / dtype_size(dt); }
 
 template <typename TI, typename TO>
 int run_conv_typed(const ConvParams &p, int k_w, int k_h, int batch, cudaStream_t st, const char *key) {
@@ -92,10 +91,11 @@ int fill_conv_params(const hgb_view &in, const hgb_window &acc, const hgb_view &
   p->in_w = in.width;
   p->in_h = in.height;
   p->batch = in.batch;
-  p->vec_in = ((uintptr_t)in.data % 16 == 0) && (in.pitch % 16 == 0) && (in.batch_stride % 16 == 0 || in.batch == 1) &&
-              (acc.offset_x % vec_elems(in.dtype) == 0);
-  p->vec_out = ((uintptr_t)out.data % 16 == 0) && (out.pitch % 16 == 0) &&
-               (out.batch_stride % 16 == 0 || out.batch == 1) && (is.offset_x % 4 == 0);
+  p->excess = std::max(0, std::max(is.width - acc.width, is.height - acc.height));
+  // a thread stores four outputs at once
+  const int64_t four = 4 * dtype_size(out.dtype);
+  p->vec_out = ((uintptr_t)out.data + (uintptr_t)is.offset_x * dtype_size(out.dtype)) % four == 0 &&
+               out.pitch % four == 0 && (out.batch_stride % four == 0 || out.batch == 1);
   return HGB_OK;
 }
 
@@ -150,8 +150,8 @@ extern "C" int hgb_local_op(const hgb_view *in, const hgb_window *accw, const hg
   // MIN / MAX over a Domain of centred row runs (squares, discs, crosses,
   // diamonds, lines) up to 7 x 7: the tiled kernel.  Masks with weights, other
   // row shapes, larger windows and mixed storage go to the general kernel
-  // (7 x 7 disc, 6 u8 images of 1408 x 3357: 700 us there, 72 us tiled; 3 x 3,
-  // 4 f32 images of 1152 x 2870: 135 us and 39 us; a 300 x 280 image costs its
+  // (7 x 7 disc, 6 u8 images of 1408 x 3357: 697 us there, 38 us tiled; 3 x 3,
+  // 4 f32 images of 1152 x 2870: 133 us and 32 us; a 300 x 280 image costs its
   // launch in both).
   MinMaxDomain dom;
   if ((reduce == HGB_REDUCE_MIN || reduce == HGB_REDUCE_MAX) && !mask && !mask_dev && in->dtype == out->dtype &&

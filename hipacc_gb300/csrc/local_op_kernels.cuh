@@ -18,20 +18,28 @@ int launch_cfg(const ConvParams &p0, int batch, cudaStream_t st) {
   constexpr int RX = MW / 2, VI = Vec16<TI>::N;
   constexpr int SW = round_up(RX, VI) + TW + round_up(MW - 1 - RX, VI), SH = TH + MH - 1;
   ConvParams p = p0;
-  // FP32 and u8 images read through the whole-image accessor stage their tiles
-  // with TMA (the box origin X0 = i0 - round_up(RX, VI) is a multiple of 16 bytes)
-  constexpr bool kU8 = std::is_same<TI, uint8_t>::value;
-  p.use_tma = 0;
-  if ((std::is_same<TI, float>::value || kU8) && p.acc_ox == 0 && p.acc_oy == 0 && p.acc_w == p.in_w &&
-      p.acc_h == p.in_h && tma_legal(p.in, p.in_pitch, p.in_bstride, batch) &&
-      make_tensor_map_3d(&p.map, kU8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-                         (int)sizeof(TI), p.in, p.in_w, p.in_h, batch, p.in_pitch, p.in_bstride, SW, SH) == HGB_OK) {
-    p.use_tma = 1;
+  const dim3 grid(cdiv(p.is_w, TW), cdiv(p.is_h, TH), batch);
+  // images read through the whole-image accessor stage their tiles with TMA (the
+  // box origin X0 = i0 - round_up(RX, VI) is a multiple of 16 bytes)
+  constexpr CUtensorMapDataType kType = std::is_same<TI, float>::value     ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                        : std::is_same<TI, uint8_t>::value ? CU_TENSOR_MAP_DATA_TYPE_UINT8
+                                        : std::is_same<TI, __half>::value  ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                                                           : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  // The TMA form is the faster one up to 11 x 11 taps, of 16-bit storage up to 7 x 7
+  // (4 images of 1280 x 872: 3 x 3 f32 10.0 -> 6.8 us without the overhang's patch,
+  // bf16 9.6 -> 8.6 us; 11 x 11 bf16 33.8 us by TMA, 33.0 us by groups; 13 x 13 f32
+  // 61 us by TMA, 40 us by groups, whose kernel leaves the stencil more registers)
+  if (MW * MH < (sizeof(TI) == 2 ? 81 : 169) && p.acc_ox == 0 && p.acc_oy == 0 && p.acc_w == p.in_w && p.acc_h == p.in_h &&
+      tma_legal(p.in, p.in_pitch, p.in_bstride, batch) &&
+      make_tensor_map_3d(&p.map, kType, (int)sizeof(TI), p.in, p.in_w, p.in_h, batch, p.in_pitch, p.in_bstride, SW,
+                         SH) == HGB_OK) {
     p.status = device_status_word();
+    cudaEvent_t ev = before_launch(st);
+    conv_kernel<TI, TO, MW, MH, BX, BY, PX, PY, true><<<grid, BX * BY, 0, st>>>(p);
+    return after_launch("conv_kernel", st, ev);
   }
-  dim3 grid(cdiv(p.is_w, TW), cdiv(p.is_h, TH), batch);
   cudaEvent_t ev = before_launch(st);
-  conv_kernel<TI, TO, MW, MH, BX, BY, PX, PY><<<grid, BX * BY, 0, st>>>(p);
+  conv_kernel<TI, TO, MW, MH, BX, BY, PX, PY, false><<<grid, BX * BY, 0, st>>>(p);
   return after_launch("conv_kernel", st, ev);
 }
 

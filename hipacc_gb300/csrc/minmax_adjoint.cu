@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(MM_T) minmax_gather_kernel(const __grid_consta
 // halo are staged once and a row's taps come from a register window.  Bound by
 // the ALU pipe: a compare and two selects per tap (select), a compare and a
 // predicated add per tap (gather).  Forward and adjoint of the 5 x 5 disc on 8
-// images of 509 x 381: 183 -> 51 us (now its host calls); of the 7 x 7 disc on
+// images of 509 x 381: 176 -> 38 us; of the 7 x 7 disc on
 // 2309 x 2207: 779 -> 142 us.
 constexpr int MT_BX = 16, MT_NT = 128, MT_PAD = 3, MT_TW = 64, MT_SW = MT_TW + 8, MT_G = MT_SW / 4;
 
@@ -165,6 +165,7 @@ __global__ void __launch_bounds__(MT_NT) minmax_select_tile_kernel(const __grid_
   const int b = blockIdx.z, i0 = blockIdx.x * MT_TW, j0 = blockIdx.y * MT_TH;
   stage_groups<float, MT_SW, SH, MT_NT>(tile, (const char *)p.in + b * p.in_b, p.in_p, i0 - 4, j0 - R, 0, p.w, 0, p.h,
                                         p.bmode, p.cval, R);
+  stage_wait();
   __syncthreads();
   const int tx = threadIdx.x % MT_BX, ty = threadIdx.x / MT_BX;
   const float first = p.flip ? -FLT_MIN : FLT_MAX;

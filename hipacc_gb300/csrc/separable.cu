@@ -165,27 +165,29 @@ __global__ void __launch_bounds__(SP_BX *SP_BY) separable_kernel(const __grid_co
     if (X0 < 0 || X0 + SW > p.w || Y0 < 0 || Y0 + SH > p.h) {
       // cells outside the image (zero-filled by TMA): left / right columns,
       // top / bottom rows; CONSTANT cells take the constant in the storage type
-      const int nl = max(0, min(SW, -X0)), rs = max(0, min(SW, p.w - X0));
-      const int nt = max(0, min(SH, -Y0)), bs = max(0, min(SH, p.h - Y0));
-      const int ncl = nl * SH, ncr = (SW - rs) * SH, nrt = nt * SW, nrb = (SH - bs) * SW;
+      // (cells past the reach of the last outputs serve none)
+      const int cw = min(SW, p.w + R - X0), ch = min(SH, p.h + R - Y0);
+      const int nl = max(0, min(cw, -X0)), rs = max(0, min(cw, p.w - X0));
+      const int nt = max(0, min(ch, -Y0)), bs = max(0, min(ch, p.h - Y0));
+      const int ncl = nl * ch, ncr = (cw - rs) * ch, nrt = nt * cw, nrb = (ch - bs) * cw;
       for (int c = threadIdx.x; c < ncl + ncr + nrt + nrb; c += NT) {
         int r, q;
         if (c < ncl) {
           r = c / nl;
           q = c - r * nl;
         } else if (c < ncl + ncr) {
-          const int d = c - ncl, n = SW - rs;
+          const int d = c - ncl, n = cw - rs;
           r = d / n;
           q = rs + (d - r * n);
         } else if (c < ncl + ncr + nrt) {
           const int d = c - ncl - ncr;
-          r = d / SW;
-          q = d - r * SW;
+          r = d / cw;
+          q = d - r * cw;
         } else {
           const int d = c - ncl - ncr - nrt;
-          const int rr = d / SW;
+          const int rr = d / cw;
           r = bs + rr;
-          q = d - rr * SW;
+          q = d - rr * cw;
         }
         const int ry = remap(p.bmode, Y0 + r, 0, p.h), rx = remap(p.bmode, X0 + q, 0, p.w);
         tile[r * SW + q] = (ry == (int)0x80000000 || rx == (int)0x80000000)
