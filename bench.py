@@ -49,7 +49,7 @@ NSETS = 16
 # DRAM bytes (read + write) per launch from one ncu capture of each kernel on
 # this workload (profiles/ holds the summary and the command); most of each
 # kernel's output is still in L2 when the capture ends, so writes read low
-NCU_TRAFFIC = {"sobel3_tma_kernel": 16845312 + 0, "gray_bulk_kernel": 67121152 + 1238016}
+NCU_TRAFFIC = {"sobel3_tile_kernel": 16845312 + 0, "gray_bulk_kernel": 67121152 + 1238016}
 E2E_STEPS = 64  # end-to-end steps timed, independent of --steps
 METRIC = "Gpixels/s (Sobel3x3 MIRROR + u64 sum + u8 max, and RGBA->gray, 4096x4096)"
 
@@ -310,7 +310,7 @@ def run_gb300(args):
         dist.barrier()
     # per-kernel average launch duration, same stream, same rotation
     kern = {}
-    for name, gr, nbytes in (("sobel3_tma_kernel", g_sobel, SOBEL_BYTES), ("gray_bulk_kernel", g_gray, GRAY_BYTES)):
+    for name, gr, nbytes in (("sobel3_tile_kernel", g_sobel, SOBEL_BYTES), ("gray_bulk_kernel", g_gray, GRAY_BYTES)):
         reps = max(4, args.steps // NSETS // 2)
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         with torch.cuda.stream(s):

@@ -7,22 +7,19 @@
 // Kernel::reduced_data of the output with a u64 sum and a u8 max
 // (dsl/kernel.hpp:121-161).  Integer arithmetic, so every order is exact.
 //
-// Fast path (the standard 3x3 Sobel masks, TMA-legal layout): sobel3_tma_kernel
-// below -- one TMA-staged 128 x 128 tile per CTA, exact fp16x2 arithmetic, the
-// sum and max folded into workspace accumulators behind one ticket.  Fallback
-// for layouts TMA cannot address (unaligned base or pitch): sobel3_kernel,
-// which stages a 128 x 64 tile with 16-byte loads, walks rows with a three-row
-// register window and uses the separable form gx = S(x+1) - S(x-1),
-// S = top + 2 mid + bottom; gy = D(x-1) + 2 D(x) + D(x+1), D = bottom - top.
-// Other masks: sobel_generic_kernel.  The fallbacks reduce sum and max with
-// redux.sync across the warp, shared memory across the block and a last-block
-// combine of the per-block partials.
+// The standard 3x3 Sobel masks: sobel3_tile_kernel below -- one 128 x 128 tile
+// per CTA (128 x 32 on small batches), staged by TMA where the layout is legal
+// and by words otherwise, exact fp16x2 arithmetic, the sum and max folded into
+// workspace accumulators behind one ticket.  Other masks: sobel_generic_kernel,
+// which reduces sum and max with redux.sync across the warp, shared memory across
+// the block and a last-block combine of the per-block partials.
 #include <algorithm>
 
 #include <cstdio>
 
 #include "autotune.h"
 #include "reduce_common.cuh"
+#include "stage_groups.cuh"
 #include "tma.cuh"
 
 namespace hgb {
@@ -34,7 +31,7 @@ struct SobelParams {
   int64_t out_pitch, out_bstride;
   int w, h;
   int bmode, cval;
-  int vec_in, vec_out;
+  int vec_out;
   int size;
   int mx[49], my[49];
   uint64_t *sum_dev;
@@ -45,12 +42,6 @@ struct SobelParams {
 };
 
 namespace {
-
-constexpr int SB_BX = 32, SB_BY = 8, SB_PY = 8;
-constexpr int SB_TW = SB_BX * 4, SB_TH = SB_BY * SB_PY;
-constexpr int SB_HL = 16;
-constexpr int SB_SW = SB_HL + SB_TW + 16;  // bytes per staged row
-constexpr int SB_SH = SB_TH + 2;
 
 __device__ __forceinline__ void block_reduce_store(const SobelParams &p, uint32_t sum, uint32_t mx) {
   __shared__ uint32_t s_sum[32], s_max[32];
@@ -117,105 +108,13 @@ __device__ __forceinline__ int sb_load_px(const SobelParams &p, const uint8_t *i
   return img[(int64_t)ry * p.in_pitch + rx];
 }
 
-__global__ void __launch_bounds__(SB_BX *SB_BY) sobel3_kernel(const __grid_constant__ SobelParams p) {
-  __shared__ __align__(16) uint8_t tile[SB_SH * SB_SW];
-  const int b = blockIdx.z;
-  const uint8_t *img = p.in + (int64_t)b * p.in_bstride;
-  const int i0 = blockIdx.x * SB_TW, j0 = blockIdx.y * SB_TH;
-  const int X0 = i0 - SB_HL, Y0 = j0 - 1;
-  constexpr int CPR = SB_SW / 16;
-  const bool interior = X0 >= 0 && X0 + SB_SW <= p.w && Y0 >= 0 && Y0 + SB_SH <= p.h;
-  for (int c = threadIdx.x; c < SB_SH * CPR; c += SB_BX * SB_BY) {
-    const int r = c / CPR, k = c - r * CPR;
-    const int y = Y0 + r, x = X0 + k * 16;
-    uint4 v;
-    if (p.vec_in && (interior || (y >= 0 && y < p.h && x >= 0 && x + 16 <= p.w))) {
-      v = ldg16(img + (int64_t)y * p.in_pitch + x);
-    } else {
-      uint32_t wv[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t wq = 0;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) wq |= (uint32_t)sb_load_px(p, img, x + 4 * q + e, y) << (8 * e);
-        wv[q] = wq;
-      }
-      v = make_uint4(wv[0], wv[1], wv[2], wv[3]);
-    }
-    *reinterpret_cast<uint4 *>(&tile[r * SB_SW + k * 16]) = v;
-  }
-  __syncthreads();
-
-  const int tx = threadIdx.x % SB_BX, ty = threadIdx.x / SB_BX;
-  const int xs = SB_HL + 4 * tx;  // staged column of the thread's first pixel
-  int top[6], mid[6], bot[6];
-  auto load_row = [&](int r, int *v) {
-    const uint8_t *row = &tile[r * SB_SW];
-    const uint32_t w0 = *reinterpret_cast<const uint32_t *>(row + xs - 4);
-    const uint32_t w1 = *reinterpret_cast<const uint32_t *>(row + xs);
-    const uint32_t w2 = *reinterpret_cast<const uint32_t *>(row + xs + 4);
-    v[0] = w0 >> 24;
-    v[1] = w1 & 0xff;
-    v[2] = (w1 >> 8) & 0xff;
-    v[3] = (w1 >> 16) & 0xff;
-    v[4] = w1 >> 24;
-    v[5] = w2 & 0xff;
-  };
-  const int r0 = ty * SB_PY;
-  load_row(r0, top);
-  load_row(r0 + 1, mid);
-  uint32_t tsum = 0, tmax = 0;
-  uint8_t *out = p.out + (int64_t)b * p.out_bstride;
-  const int xo = i0 + 4 * tx;
-#pragma unroll
-  for (int oy = 0; oy < SB_PY; ++oy) {
-    load_row(r0 + oy + 2, bot);
-    int S[6], D[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      S[c] = top[c] + 2 * mid[c] + bot[c];
-      D[c] = bot[c] - top[c];
-    }
-    uint32_t word = 0;
-    const int yo = j0 + ty * SB_PY + oy;
-    const bool row_ok = yo < p.h;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int gx = S[q + 2] - S[q];
-      const int gy = D[q] + 2 * D[q + 1] + D[q + 2];
-      int m = abs(gx) + abs(gy);
-      m = m < 255 ? m : 255;
-      word |= (uint32_t)m << (8 * q);
-      if (row_ok && xo + q < p.w) {
-        tsum += m;
-        tmax = tmax > (uint32_t)m ? tmax : (uint32_t)m;
-      }
-    }
-    if (row_ok) {
-      uint8_t *dst = out + (int64_t)yo * p.out_pitch + xo;
-      if (p.vec_out && xo + 4 <= p.w) {
-        *reinterpret_cast<uint32_t *>(dst) = word;
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-          if (xo + q < p.w) dst[q] = (uint8_t)(word >> (8 * q));
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      top[c] = mid[c];
-      mid[c] = bot[c];
-    }
-  }
-  if (p.sum_dev || p.max_dev) block_reduce_store(p, tsum, tmax);
-}
-
-
 // ---------------------------------------------------------------------------
-// TMA path for the standard 3x3 masks.  One CTA per 128 x 128 output tile:
-// thread 0 loads the tile's 160 x 130 byte halo region with one
-// cp.async.bulk.tensor (completion on an mbarrier, bounded wait), and each of
-// the four warps runs 32 output rows of it, a lane owning four columns.  A CTA
+// The standard 3x3 masks.  One CTA per 128 x 128 output tile: thread 0 loads the
+// tile's 160 x 130 byte halo region with one cp.async.bulk.tensor (completion on
+// an mbarrier, bounded wait), and each of the four warps runs 32 output rows of
+// it, a lane owning four columns.  Layouts that TMA cannot address are staged by
+// the CTA's threads, a word at a time (4001 x 4003 with its gray: 67 -> 41 us
+// against the kernel this replaces, which staged such rows byte by byte).  A CTA
 // holds 21 KB of shared memory and 128 threads, so an SM keeps up to ten tiles
 // in flight without a software pipeline, and independent kernels of the same
 // step can share the SMs.  Cells outside the image (TMA fills them with 0)
@@ -332,17 +231,20 @@ __device__ __forceinline__ void sobel_tile(const SobelParams &p, const uint8_t *
   }
 }
 
-// Staged cells outside the image that the stencil reads (columns 15..144, all
-// rows of a tile whose first staged cell is image (X0, Y0)) get the boundary
-// rule; TMA filled them with zeros.  Regions: left columns, right columns, top
-// row, bottom rows.  Every thread of the CTA takes part.
+// Staged cells outside the image that the stencil reads (columns 15..144, SH
+// rows of a tile whose first staged cell is image (X0, Y0), up to one past the
+// image) get the boundary rule; staging filled them with zeros.  Regions: left
+// columns, right columns, top row, bottom row.  Every thread of the CTA takes
+// part.  (Patching a tile's whole overhang made a 64 x 64 image take 40 us.)
+template <int SH>
 __device__ __forceinline__ void sobel_patch(const SobelParams &p, const uint8_t *img, uint8_t *tile, int X0, int Y0) {
-  constexpr int qa = 15, qb = 145, ncol = qb - qa;
+  constexpr int qa = 15;
+  const int qb = min(145, p.w + 1 - X0), ch = min(SH, p.h + 1 - Y0), ncol = qb - qa;
   const int nl = max(0, min(qb, -X0) - qa);
   const int rs = max(qa, p.w - X0), nr = max(0, qb - rs);
   const int ntop = max(0, -Y0);
-  const int bs = max(0, p.h - Y0), nb = max(0, T_SH - bs);
-  const int n1 = nl * T_SH, n2 = n1 + nr * T_SH, n3 = n2 + ntop * ncol, n4 = n3 + nb * ncol;
+  const int bs = max(0, p.h - Y0), nb = max(0, ch - bs);
+  const int n1 = nl * ch, n2 = n1 + nr * ch, n3 = n2 + ntop * ncol, n4 = n3 + nb * ncol;
   for (int cc = threadIdx.x; cc < n4; cc += blockDim.x) {
     int r, q;
     if (cc < n1) {
@@ -366,36 +268,42 @@ __device__ __forceinline__ void sobel_patch(const SobelParams &p, const uint8_t 
   }
 }
 
-template <int T_WARPS>
-__global__ void __launch_bounds__(T_WARPS * 32) sobel3_tma_kernel(const __grid_constant__ SobelTmaParams P) {
-  constexpr int T_R = T_TH / T_WARPS;
-  __shared__ __align__(128) uint8_t tile[T_STAGE_PAD];
+template <int T_WARPS, int TH, bool TMA>
+__global__ void __launch_bounds__(T_WARPS * 32) sobel3_tile_kernel(const __grid_constant__ SobelTmaParams P) {
+  constexpr int T_R = TH / T_WARPS, SH = TH + 2, STAGE = T_SW * SH;
+  __shared__ __align__(128) uint8_t tile[(STAGE + 127) / 128 * 128];
   __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t s_sum[T_WARPS], s_max[T_WARPS];
   const SobelParams &p = P.p;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x;
   const int tx_ = t % P.tiles_x, r_ = t / P.tiles_x;
-  const int i0 = tx_ * T_TW, j0 = (r_ % P.tiles_y) * T_TH, b = r_ / P.tiles_y;
-  if (threadIdx.x == 0) {
-    mbar_init(&bar, 1);
-    mbar_fence_init();
-    mbar_expect_tx(&bar, T_STAGE);
-    tma_load_3d(tile, &P.map, i0 - 16, j0 - 1, b, &bar);
-  }
-  if (!cta_wait(&bar, 0)) {
-    if (threadIdx.x == 0) {
-      record_status(P.status, HGB_ERR_TIMEOUT);
-      mbar_wait(&bar, 0);  // the load may still land: wait once more (bounded) before leaving
-    }
-    // this CTA's partials are missing; the status word reports the launch as failed
-    if (p.sum_dev || p.max_dev)
-      if (threadIdx.x == 0) accumulate_and_publish(P.acc, P.acc + 1, P.ticket, 0, 0, p.sum_dev, p.max_dev);
-    return;
-  }
+  const int i0 = tx_ * T_TW, j0 = (r_ % P.tiles_y) * TH, b = r_ / P.tiles_y;
+  const uint8_t *img = p.in + (int64_t)b * p.in_bstride;
   const int X0 = i0 - 16, Y0 = j0 - 1;
-  if (X0 + 15 < 0 || X0 + 145 > p.w || Y0 < 0 || Y0 + T_SH > p.h) {
-    sobel_patch(p, p.in + (int64_t)b * p.in_bstride, tile, X0, Y0);
+  if constexpr (TMA) {
+    if (threadIdx.x == 0) {
+      mbar_init(&bar, 1);
+      mbar_fence_init();
+      mbar_expect_tx(&bar, STAGE);
+      tma_load_3d(tile, &P.map, i0 - 16, j0 - 1, b, &bar);
+    }
+    if (!cta_wait(&bar, 0)) {
+      if (threadIdx.x == 0) {
+        record_status(P.status, HGB_ERR_TIMEOUT);
+        mbar_wait(&bar, 0);  // the load may still land: wait once more (bounded) before leaving
+      }
+      // this CTA's partials are missing; the status word reports the launch as failed
+      if (p.sum_dev || p.max_dev)
+        if (threadIdx.x == 0) accumulate_and_publish(P.acc, P.acc + 1, P.ticket, 0, 0, p.sum_dev, p.max_dev);
+      return;
+    }
+  } else {
+    stage_words<T_SW / 4, SH, T_WARPS * 32>(reinterpret_cast<uint32_t *>(tile), img, p.in_pitch, X0, Y0, p.w, p.h);
+    __syncthreads();
+  }
+  if (X0 + 15 < 0 || X0 + 145 > p.w || Y0 < 0 || Y0 + SH > p.h) {
+    sobel_patch<SH>(p, img, tile, X0, Y0);
     __syncthreads();
   }
   uint32_t tsum = 0;
@@ -483,7 +391,7 @@ __global__ void __launch_bounds__(T_WARPS * 32) sobel3_stream_kernel(const __gri
     const int i0 = tx_ * T_TW, j0 = (r_ % P.tiles_y) * T_TH, b = r_ / P.tiles_y;
     const int X0 = i0 - 16, Y0 = j0 - 1;
     if (X0 + 15 < 0 || X0 + 145 > p.w || Y0 < 0 || Y0 + T_SH > p.h) {
-      sobel_patch(p, p.in + (int64_t)b * p.in_bstride, tile[buf], X0, Y0);
+      sobel_patch<T_SH>(p, p.in + (int64_t)b * p.in_bstride, tile[buf], X0, Y0);
       __syncthreads();
     }
     const int xo = i0 + 4 * lane, jw = j0 + warp * T_R;
@@ -609,14 +517,13 @@ extern "C" int hgb_sobel_mag(const hgb_view *in, const hgb_view *out, const int 
     p.mx[i] = mask_x[i];
     p.my[i] = mask_y[i];
   }
-  p.vec_in = ((uintptr_t)in->data % 16 == 0) && in->pitch % 16 == 0 && (in->batch == 1 || in->batch_stride % 16 == 0);
   p.vec_out = ((uintptr_t)out->data % 4 == 0) && out->pitch % 4 == 0 && (out->batch == 1 || out->batch_stride % 4 == 0);
   p.sum_dev = sum_dev;
   p.max_dev = max_dev;
   bool fast = size == 3;
   for (int i = 0; fast && i < 9; ++i) fast = mask_x[i] == kSobelX3[i] && mask_y[i] == kSobelY3[i];
-  dim3 grid = fast ? dim3(cdiv(p.w, SB_TW), cdiv(p.h, SB_TH), in->batch) : dim3(cdiv(p.w, 16), cdiv(p.h, 16), in->batch);
-  if (sum_dev || max_dev) {
+  const dim3 grid(cdiv(p.w, 16), cdiv(p.h, 16), in->batch);
+  if (!fast && (sum_dev || max_dev)) {
     const size_t nb = (size_t)grid.x * grid.y * grid.z;
     Workspace ws;
     rc = workspace_get(nb * 12 + 256, &ws);
@@ -626,24 +533,39 @@ extern "C" int hgb_sobel_mag(const hgb_view *in, const hgb_view *out, const int 
     p.ticket = ws.tickets + 0;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  if (fast && tma_legal(in->data, in->pitch, in->batch_stride, in->batch)) {
+  if (fast) {
     SobelTmaParams P;
     memset(&P, 0, sizeof(P));
     P.p = p;
     P.tiles_x = cdiv(p.w, T_TW);
     P.tiles_y = cdiv(p.h, T_TH);
-    P.ntiles = P.tiles_x * P.tiles_y * in->batch;
+    const int64_t tiles = (int64_t)P.tiles_x * P.tiles_y * in->batch;
+    HGB_REQUIRE(tiles < (1ll << 28), "hgb_sobel_mag: image too large");
+    P.ntiles = (int)tiles;
     P.status = device_status_word();
-    rc = make_tensor_map_3d(&P.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, in->data, p.w, p.h, in->batch, in->pitch,
-                            in->batch_stride, T_SW, T_SH);
-    if (rc == HGB_OK) {
-      // the streaming form always takes a ticket (it resets its tile counter)
-      Workspace ws;
-      rc = workspace_get(0, &ws);
-      if (rc) return rc;
-      P.acc = ws.acc + kSlotSobel;
-      P.ticket = ws.tickets + 0;
-      P.claim = ws.tickets + kTicketSobelClaim;
+    // the streaming form always takes a ticket (it resets its tile counter)
+    Workspace ws;
+    rc = workspace_get(0, &ws);
+    if (rc) return rc;
+    P.acc = ws.acc + kSlotSobel;
+    P.ticket = ws.tickets + 0;
+    P.claim = ws.tickets + kTicketSobelClaim;
+    // 128 x 32 tiles where the taller ones would not give every SM four CTAs:
+    // the time of a small image is one CTA's chain of rows (640 x 480 with its
+    // gray: 14.5 -> 6.0 us)
+    const bool low = P.ntiles < 4 * num_sms();
+    if (low) {
+      P.tiles_y = cdiv(p.h, 32);
+      P.ntiles = P.tiles_x * P.tiles_y * in->batch;
+    }
+    if (tma_legal(in->data, in->pitch, in->batch_stride, in->batch) &&
+        make_tensor_map_3d(&P.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, in->data, p.w, p.h, in->batch, in->pitch,
+                           in->batch_stride, T_SW, low ? 34 : T_SH) == HGB_OK) {
+      if (low) {
+        cudaEvent_t ev = before_launch(st);
+        sobel3_tile_kernel<4, 32, true><<<P.ntiles, 128, 0, st>>>(P);
+        return after_launch("sobel3_tile_kernel", st, ev);
+      }
       char key[96];
       snprintf(key, sizeof(key), "sobel3:%dx%dx%d", 1 << (32 - __builtin_clz((unsigned)p.w)),
                1 << (32 - __builtin_clz((unsigned)p.h)), in->batch);
@@ -662,17 +584,20 @@ extern "C" int hgb_sobel_mag(const hgb_view *in, const hgb_view *out, const int 
         }
         cudaEvent_t ev = before_launch(st);
         if (warps == 8)
-          sobel3_tma_kernel<8><<<P.ntiles, 256, 0, st>>>(P);
+          sobel3_tile_kernel<8, T_TH, true><<<P.ntiles, 256, 0, st>>>(P);
         else
-          sobel3_tma_kernel<4><<<P.ntiles, 128, 0, st>>>(P);
-        return after_launch("sobel3_tma_kernel", st, ev);
+          sobel3_tile_kernel<4, T_TH, true><<<P.ntiles, 128, 0, st>>>(P);
+        return after_launch("sobel3_tile_kernel", st, ev);
       });
     }
+    cudaEvent_t ev = before_launch(st);
+    if (low)
+      sobel3_tile_kernel<4, 32, false><<<P.ntiles, 128, 0, st>>>(P);
+    else
+      sobel3_tile_kernel<4, T_TH, false><<<P.ntiles, 128, 0, st>>>(P);
+    return after_launch("sobel3_tile_kernel", st, ev);
   }
   cudaEvent_t ev = before_launch(st);
-  if (fast)
-    sobel3_kernel<<<grid, SB_BX * SB_BY, 0, st>>>(p);
-  else
-    sobel_generic_kernel<<<grid, 256, 0, st>>>(p);
+  sobel_generic_kernel<<<grid, 256, 0, st>>>(p);
   return after_launch("sobel", st, ev);
 }
