@@ -126,5 +126,13 @@ def check(status: int) -> None:
         raise HgbError(status, msg)
 
 
+_fns: dict = {}  # entry points by name, resolved once
+
+
 def call(name: str, *args) -> None:
-    check(getattr(load(), name)(*args))
+    fn = _fns.get(name)
+    if fn is None:
+        fn = _fns[name] = getattr(load(), name)
+    status = fn(*args)
+    if status != OK:
+        check(status)

@@ -27,27 +27,24 @@ def view(t: torch.Tensor, rgba: bool = False) -> L.View:
     """hgb_view of a CUDA tensor (rows may be padded; the last dim must be dense)."""
     if not t.is_cuda:
         raise ValueError("hipacc_gb300 operates on CUDA tensors")
-    es = t.element_size()
+    es, shape, strides = t.element_size(), t.shape, t.stride()
     if rgba:
-        if t.dtype != torch.uint8 or t.shape[-1] != 4 or t.stride(-1) != 1 or t.stride(-2) != 4:
+        if t.dtype != torch.uint8 or shape[-1] != 4 or strides[-1] != 1 or strides[-2] != 4:
             raise ValueError("RGBA images are uint8 tensors (..., H, W, 4) with dense pixels")
-        shape = t.shape[:-1]
-        strides = t.stride()[:-1]
+        shape, strides = shape[:-1], strides[:-1]
         dt = L.U8X4
     else:
-        if t.stride(-1) != 1:
+        if strides[-1] != 1:
             raise ValueError("the innermost dimension must be dense")
-        shape, strides, dt = t.shape, t.stride(), _DT[t.dtype]
-    if len(shape) == 2:
-        b, (h, w) = 1, shape
-        bs = strides[0] * es * h
-    elif len(shape) == 3:
+        dt = _DT[t.dtype]
+    n = len(shape)
+    if n == 2:
+        h, w = shape
+        return L.View(t.data_ptr(), dt, w, h, 1, strides[0] * es, strides[0] * es * h)
+    if n == 3:
         b, h, w = shape
-        bs = strides[0] * es
-    else:
-        raise ValueError("images are (H, W) or (B, H, W)")
-    pitch = strides[-2] * es
-    return L.View(t.data_ptr(), dt, int(w), int(h), int(b), int(pitch), int(bs))
+        return L.View(t.data_ptr(), dt, w, h, b, strides[1] * es, strides[0] * es)
+    raise ValueError("images are (H, W) or (B, H, W)")
 
 
 def window(w):
@@ -56,16 +53,28 @@ def window(w):
     return C.byref(L.Window(*[int(v) for v in w]))
 
 
+# Per-call host time matters on small images: the current stream's handle comes
+# straight from torch's C layer (0.3 us; building a torch.cuda.Stream for it takes
+# 3 us), host arrays pass their address as an integer (a ctypes cast takes 1.7 us).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    """cudaStream_t of `stream`, or of the current device's current stream."""
+    if stream is None:
+        if _raw_stream is not None:
+            return _raw_stream(torch.cuda.current_device())
+        stream = torch.cuda.current_stream()
+    return stream.cuda_stream
 
 
-def _fptr(a):
-    if a is None:
-        return None
-    a = np.ascontiguousarray(a, np.float32)
-    return a.ctypes.data_as(C.c_void_p), a
+def _ptr(a):
+    """Address of a contiguous host array (the caller keeps it alive), None of None."""
+    return None if a is None else a.ctypes.data
+
+
+def _dptr(t):
+    return None if t is None else t.data_ptr()
 
 
 def init(device: int = 0) -> str:
@@ -91,9 +100,9 @@ def local_op(inp, out=None, mask=None, domain=None, size=None, reduce=SUM, bound
     d = None if domain is None else np.ascontiguousarray(domain, np.uint8)
     vi, vo = view(inp), view(out)
     L.call("hgb_local_op", C.byref(vi), window(acc), C.byref(vo), window(iter_space),
-           None if m is None else m.ctypes.data_as(C.c_void_p),
-           None if mask_dev is None else C.c_void_p(mask_dev.data_ptr()),
-           None if d is None else d.ctypes.data_as(C.c_void_p), mw, mh, reduce, boundary, float(const),
+           _ptr(m),
+           _dptr(mask_dev),
+           _ptr(d), mw, mh, reduce, boundary, float(const),
            _stream(stream))
     return out
 
@@ -106,9 +115,9 @@ def sobel_mag(inp, out=None, mask_x=SOBEL3_X, mask_y=SOBEL3_Y, boundary=MIRROR, 
     mx = np.ascontiguousarray(mask_x, np.int32)
     my = np.ascontiguousarray(mask_y, np.int32)
     vi, vo = view(inp), view(out)
-    L.call("hgb_sobel_mag", C.byref(vi), C.byref(vo), mx.ctypes.data_as(C.c_void_p), my.ctypes.data_as(C.c_void_p),
-           mx.shape[0], boundary, int(const), None if sum_out is None else C.c_void_p(sum_out.data_ptr()),
-           None if max_out is None else C.c_void_p(max_out.data_ptr()), _stream(stream))
+    L.call("hgb_sobel_mag", C.byref(vi), C.byref(vo), _ptr(mx), _ptr(my),
+           mx.shape[0], boundary, int(const), _dptr(sum_out),
+           _dptr(max_out), _stream(stream))
     return out
 
 
@@ -150,7 +159,7 @@ def reduce(inp, op=SUM, win=None, result_dev=None, stream=None):
     vi = view(inp)
     host = C.create_string_buffer(8)
     L.call("hgb_reduce", C.byref(vi), window(win), op,
-           None if result_dev is None else C.c_void_p(result_dev.data_ptr()), host, _stream(stream))
+           _dptr(result_dev), host, _stream(stream))
     raw = host.raw
     if inp.dtype in (torch.float32, torch.float16, torch.bfloat16, torch.float64):
         return struct.unpack("<d", raw)[0]
@@ -166,7 +175,7 @@ def histogram(inp, num_bins, win=None, bins=None, stream=None):
     if bins is None:
         bins = torch.empty(num_bins, dtype=torch.int32, device=inp.device)
     vi = view(inp)
-    L.call("hgb_histogram", C.byref(vi), window(win), int(num_bins), C.c_void_p(bins.data_ptr()), None,
+    L.call("hgb_histogram", C.byref(vi), window(win), int(num_bins), bins.data_ptr(), None,
            _stream(stream))
     return bins
 
@@ -177,7 +186,7 @@ def separable(inp, out=None, row_taps=None, col_taps=None, boundary=CLAMP, const
     r = np.ascontiguousarray(row_taps, np.float32)
     c = np.ascontiguousarray(col_taps if col_taps is not None else row_taps, np.float32)
     vi, vo = view(inp), view(out)
-    L.call("hgb_separable", C.byref(vi), C.byref(vo), r.ctypes.data_as(C.c_void_p), c.ctypes.data_as(C.c_void_p),
+    L.call("hgb_separable", C.byref(vi), C.byref(vo), _ptr(r), _ptr(c),
            len(r), boundary, float(const), _stream(stream))
     return out
 
@@ -187,7 +196,7 @@ def bilateral(inp, out=None, smask=None, sigma_r=0.1, boundary=CLAMP, const=0.0,
         out = torch.empty_like(inp)
     s = np.ascontiguousarray(smask, np.float32)
     vi, vo = view(inp), view(out)
-    L.call("hgb_bilateral", C.byref(vi), C.byref(vo), s.ctypes.data_as(C.c_void_p), s.shape[0], float(sigma_r),
+    L.call("hgb_bilateral", C.byref(vi), C.byref(vo), _ptr(s), s.shape[0], float(sigma_r),
            boundary, float(const), 1 if fast_weights else 0, _stream(stream))
     return out
 
@@ -216,7 +225,7 @@ class PyramidPlan:
         h = (C.c_int * self.n)(*[int(v) for v in heights])
         m = _np.ascontiguousarray(mask5, _np.float32)
         self._h = C.c_void_p()
-        L.call("hgb_pyramid_plan_create", self.n, w, h, levels, m.ctypes.data_as(C.c_void_p), boundary,
+        L.call("hgb_pyramid_plan_create", self.n, w, h, levels, _ptr(m), boundary,
                C.byref(self._h))
 
     def views(self, image, level):
@@ -254,7 +263,7 @@ class PyramidPlan:
         if buf is None:
             L.call("hgb_pyramid_plan_trace", self._h, None, 0)
         else:
-            L.call("hgb_pyramid_plan_trace", self._h, C.c_void_p(buf.data_ptr()), buf.numel() // 8)
+            L.call("hgb_pyramid_plan_trace", self._h, buf.data_ptr(), buf.numel() // 8)
 
     def collapse(self, stream=None):
         L.call("hgb_pyramid_collapse", self._h, _stream(stream))
@@ -285,16 +294,16 @@ def conv_bilateral_mse(x, t, mask, sigma, smask, boundary=CLAMP, mode=0, stream=
     mask: 7x7 float32 CUDA tensor; sigma: 1-element float32 CUDA tensor.
     Returns (loss [float64, 1], grad_x, grad_mask [7x7], grad_sigma [1])."""
     dev = x.device
-    loss = torch.zeros(1, dtype=torch.float64, device=dev)
+    loss = torch.empty(1, dtype=torch.float64, device=dev)
     gx = torch.empty_like(x)
     gm = torch.empty((7, 7), dtype=torch.float32, device=dev)
     gs = torch.empty(1, dtype=torch.float32, device=dev)
     sm = np.ascontiguousarray(smask, np.float32)
     mask = mask.contiguous()
     vx, vt, vg = view(x), view(t), view(gx)
-    L.call("hgb_conv_bilateral_mse", C.byref(vx), C.byref(vt), C.c_void_p(mask.data_ptr()), 7,
-           sm.ctypes.data_as(C.c_void_p), 9, C.c_void_p(sigma.data_ptr()), boundary, mode,
-           C.c_void_p(loss.data_ptr()), C.byref(vg), C.c_void_p(gm.data_ptr()), C.c_void_p(gs.data_ptr()),
+    L.call("hgb_conv_bilateral_mse", C.byref(vx), C.byref(vt), mask.data_ptr(), 7,
+           _ptr(sm), 9, sigma.data_ptr(), boundary, mode,
+           loss.data_ptr(), C.byref(vg), gm.data_ptr(), gs.data_ptr(),
            _stream(stream))
     return loss, gx, gm, gs
 
@@ -305,18 +314,18 @@ def local_op_adjoint(grad_out, mask, boundary=CLAMP, inp=None, want_grad_in=True
     gi = torch.empty_like(grad_out) if want_grad_in else None
     if torch.is_tensor(mask):
         mh, mw = mask.shape
-        m_host, m_dev = None, C.c_void_p(mask.contiguous().data_ptr())
+        m_host, m_dev = None, mask.contiguous().data_ptr()
     else:
         m = np.ascontiguousarray(mask, np.float32)
         mh, mw = m.shape
-        m_host, m_dev = m.ctypes.data_as(C.c_void_p), None
+        m_host, m_dev = _ptr(m), None
     gm = torch.empty((mh, mw), dtype=torch.float32, device=grad_out.device) if want_grad_mask else None
     vg = view(grad_out)
     vi = view(inp) if inp is not None else None
     vgi = view(gi) if gi is not None else None
     L.call("hgb_local_op_adjoint", None if vi is None else C.byref(vi), C.byref(vg),
            None if vgi is None else C.byref(vgi), m_host, m_dev, mw, mh, boundary,
-           None if gm is None else C.c_void_p(gm.data_ptr()), _stream(stream))
+           _dptr(gm), _stream(stream))
     return gi, gm
 
 
@@ -324,13 +333,13 @@ def bilateral_adjoint(inp, grad_out, smask, sigma_r, boundary=CLAMP, const=0.0, 
                       want_grad_sigma=True, stream=None):
     """Adjoint of the bilateral filter: (grad_in, grad_sigma [1 float]) for grad_out = dL/dy."""
     gi = torch.empty_like(grad_out) if want_grad_in else None
-    gs = torch.zeros(1, dtype=torch.float32, device=inp.device) if want_grad_sigma else None
+    gs = torch.empty(1, dtype=torch.float32, device=inp.device) if want_grad_sigma else None
     s = np.ascontiguousarray(smask, np.float32)
     vi, vg = view(inp), view(grad_out)
     vgi = view(gi) if gi is not None else None
-    L.call("hgb_bilateral_adjoint", C.byref(vi), C.byref(vg), s.ctypes.data_as(C.c_void_p), s.shape[0],
+    L.call("hgb_bilateral_adjoint", C.byref(vi), C.byref(vg), _ptr(s), s.shape[0],
            float(sigma_r), boundary, float(const), None if vgi is None else C.byref(vgi),
-           None if gs is None else C.c_void_p(gs.data_ptr()), _stream(stream))
+           _dptr(gs), _stream(stream))
     return gi, gs
 
 
@@ -340,13 +349,13 @@ def separable_adjoint(inp, grad_out, row_taps, col_taps=None, boundary=CLAMP, co
     r = np.ascontiguousarray(row_taps, np.float32)
     c = np.ascontiguousarray(col_taps if col_taps is not None else row_taps, np.float32)
     gi = torch.empty_like(grad_out) if want_grad_in else None
-    gr = torch.zeros(len(r), dtype=torch.float32, device=grad_out.device) if want_grad_taps else None
-    gc = torch.zeros(len(r), dtype=torch.float32, device=grad_out.device) if want_grad_taps else None
+    gr = torch.empty(len(r), dtype=torch.float32, device=grad_out.device) if want_grad_taps else None
+    gc = torch.empty(len(r), dtype=torch.float32, device=grad_out.device) if want_grad_taps else None
     vi, vg = view(inp), view(grad_out)
     vgi = view(gi) if gi is not None else None
-    L.call("hgb_separable_adjoint", C.byref(vi), C.byref(vg), r.ctypes.data_as(C.c_void_p),
-           c.ctypes.data_as(C.c_void_p), len(r), boundary, float(const), None if vgi is None else C.byref(vgi),
-           None if gr is None else C.c_void_p(gr.data_ptr()), None if gc is None else C.c_void_p(gc.data_ptr()),
+    L.call("hgb_separable_adjoint", C.byref(vi), C.byref(vg), _ptr(r),
+           _ptr(c), len(r), boundary, float(const), None if vgi is None else C.byref(vgi),
+           _dptr(gr), _dptr(gc),
            _stream(stream))
     return gi, gr, gc
 
@@ -357,13 +366,13 @@ def minmax_adjoint(inp, grad_out, reduce, mask=None, domain=None, size=None, bou
     if mask is not None:
         m = np.ascontiguousarray(mask, np.float32)
         mh, mw = m.shape
-        mp = m.ctypes.data_as(C.c_void_p)
+        mp = _ptr(m)
     else:
         m, mp = None, None
     if domain is not None:
         d = np.ascontiguousarray(domain, np.uint8)
         mh, mw = d.shape
-        dp = d.ctypes.data_as(C.c_void_p)
+        dp = _ptr(d)
     else:
         d, dp = None, None
     if m is None and d is None:

@@ -1,4 +1,5 @@
 // autotune.cu -- the tile-configuration cache and its JSON persistence.
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -12,10 +13,13 @@ namespace hgb {
 namespace {
 std::mutex g_mu;
 std::map<std::string, std::pair<int, float>> g_cache;
-bool g_enabled = false;
+std::atomic<bool> g_enabled{false};
+std::atomic<int> g_entries{0};  // size of g_cache
 }  // namespace
 
 bool autotune_enabled() { return g_enabled; }
+
+bool autotune_idle() { return !g_enabled && g_entries == 0; }
 
 int autotune_lookup(const char *key) {
   std::lock_guard<std::mutex> lk(g_mu);
@@ -26,6 +30,7 @@ int autotune_lookup(const char *key) {
 void autotune_store(const char *key, int cfg, float ms) {
   std::lock_guard<std::mutex> lk(g_mu);
   g_cache[key] = {cfg, ms};
+  g_entries = (int)g_cache.size();
 }
 
 }  // namespace hgb
@@ -42,6 +47,7 @@ int hgb_autotune_enable(int on) {
 int hgb_autotune_clear(void) {
   std::lock_guard<std::mutex> lk(g_mu);
   g_cache.clear();
+  g_entries = 0;
   return HGB_OK;
 }
 
@@ -91,6 +97,7 @@ int hgb_autotune_load(const char *path) {
     }
     pos = end + 1;
   }
+  g_entries = (int)g_cache.size();
   return loaded > 0 || s.find('"') == std::string::npos ? HGB_OK
                                                         : set_error(HGB_ERR_INVALID, "hgb_autotune_load: no entries");
 }

@@ -20,6 +20,9 @@ bool autotune_enabled();
 int autotune_lookup(const char *key);  // -1 when unknown
 void autotune_store(const char *key, int cfg, float ms);
 
+// Nothing to look up and nothing to tune: callers skip building their key.
+bool autotune_idle();
+
 template <typename F>
 int autotune_run(const char *key, int ncfg, cudaStream_t st, F &&launch) {
   int cfg = autotune_lookup(key);

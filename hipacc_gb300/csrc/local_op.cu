@@ -17,16 +17,21 @@ namespace {
 
 template <typename TI, typename TO>
 int run_conv_typed(const ConvParams &p, int k_w, int k_h, int batch, cudaStream_t st, const char *key) {
+  if (!key) return launch_conv<TI, TO>(p, k_w, k_h, batch, st, 0);
   const int n = num_tile_cfgs();
   return autotune_run(key, n, st, [&](int cfg) { return launch_conv<TI, TO>(p, k_w, k_h, batch, st, cfg); });
 }
 
 int run_conv(int dti, int dto, const ConvParams &p, int k_w, int k_h, int batch, cudaStream_t st) {
-  char key[128];
-  // shape class: mask, dtype and image size rounded to a power of two
-  int cls = 0;
-  while ((1 << cls) < p.is_w * (int64_t)p.is_h / 4096 && cls < 30) ++cls;
-  snprintf(key, sizeof(key), "conv/%d/%d/%dx%d/%d/b%d", dti, dto, k_w, k_h, cls, batch > 8 ? 9 : batch);
+  char text[128];
+  const char *key = nullptr;
+  if (!autotune_idle()) {
+    key = text;
+    // shape class: mask, dtype and image size rounded to a power of two
+    int cls = 0;
+    while ((1 << cls) < p.is_w * (int64_t)p.is_h / 4096 && cls < 30) ++cls;
+    snprintf(text, sizeof(text), "conv/%d/%d/%dx%d/%d/b%d", dti, dto, k_w, k_h, cls, batch > 8 ? 9 : batch);
+  }
   if (dti == HGB_F32 && dto == HGB_F32) return run_conv_typed<float, float>(p, k_w, k_h, batch, st, key);
   if (dti == HGB_BF16 && dto == HGB_BF16) return run_conv_typed<__nv_bfloat16, __nv_bfloat16>(p, k_w, k_h, batch, st, key);
   if (dti == HGB_F16 && dto == HGB_F16) return run_conv_typed<__half, __half>(p, k_w, k_h, batch, st, key);

@@ -4,6 +4,41 @@
 
 using namespace hgb;
 
+namespace {
+
+// Where the kernel leaves a host result: eight bytes of pinned host memory per
+// calling thread (a call returns after its stream is done, so a thread needs one),
+// freed with the thread.  Writing it from the kernel saves the copy back: 20 us
+// with a queued copy of 8 bytes through the C ABI, 13 us without (a call through
+// hipacc_gb300.api 26 -> 16 us).
+struct HostSlot {
+  unsigned long long *p = nullptr;
+  ~HostSlot() {
+    if (p) with_relaxed_capture([&] { return cudaFreeHost(p); });
+  }
+  unsigned long long *get() {
+    if (!p)
+      with_relaxed_capture([&] {
+        return cudaHostAlloc((void **)&p, sizeof(*p), cudaHostAllocMapped | cudaHostAllocPortable);
+      });
+    return p;  // unified addressing: the same address on every device
+  }
+  // allocation is no part of another thread's stream capture
+  template <typename F>
+  void with_relaxed_capture(F &&f) {
+    cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&m) != cudaSuccess) return;
+    if (f() != cudaSuccess) {
+      p = nullptr;
+      cudaGetLastError();
+    }
+    cudaThreadExchangeStreamCaptureMode(&m);
+  }
+};
+thread_local HostSlot t_slot;
+
+}  // namespace
+
 extern "C" int hgb_reduce(const hgb_view *in, const hgb_window *winp, int op, void *result_dev, void *result_host,
                           void *stream) {
   HGB_REQUIRE(result_dev || result_host, "hgb_reduce: no result destination");
@@ -17,13 +52,17 @@ extern "C" int hgb_reduce(const hgb_view *in, const hgb_window *winp, int op, vo
   p.partials = ws.base;
   // the 8-byte result slot sits behind the partials when no device result is given
   unsigned long long *slot = (unsigned long long *)((char *)ws.base + (size_t)grid * 16);
-  p.result_dev = result_dev ? (unsigned long long *)result_dev : slot;
+  unsigned long long *direct = result_host && !result_dev ? t_slot.get() : nullptr;
+  p.result_dev = result_dev ? (unsigned long long *)result_dev : (direct ? direct : slot);
   p.ticket = ws.tickets + 1;
   p.acc = ws.acc + kSlotReduce;
   cudaStream_t st = (cudaStream_t)stream;
   rc = reduce_launch(in->dtype, op, p, grid, st);
   if (rc) return rc;
-  if (result_host) {
+  if (direct) {
+    HGB_CHECK_CUDA(cudaStreamSynchronize(st));
+    memcpy(result_host, direct, 8);
+  } else if (result_host) {
     HGB_CHECK_CUDA(cudaMemcpyAsync(result_host, p.result_dev, 8, cudaMemcpyDeviceToHost, st));
     HGB_CHECK_CUDA(cudaStreamSynchronize(st));
   }

@@ -566,10 +566,7 @@ extern "C" int hgb_sobel_mag(const hgb_view *in, const hgb_view *out, const int 
         sobel3_tile_kernel<4, 32, true><<<P.ntiles, 128, 0, st>>>(P);
         return after_launch("sobel3_tile_kernel", st, ev);
       }
-      char key[96];
-      snprintf(key, sizeof(key), "sobel3:%dx%dx%d", 1 << (32 - __builtin_clz((unsigned)p.w)),
-               1 << (32 - __builtin_clz((unsigned)p.h)), in->batch);
-      return autotune_run(key, kSobelCfgs, st, [&](int cfg) {
+      auto launch = [&](int cfg) {
         const int per_sm = kSobelStream[cfg], warps = kSobelWarps[cfg];
         if (per_sm > 0) {
           const void *fn = warps == 8 ? (const void *)sobel3_stream_kernel<8> : (const void *)sobel3_stream_kernel<4>;
@@ -588,7 +585,12 @@ extern "C" int hgb_sobel_mag(const hgb_view *in, const hgb_view *out, const int 
         else
           sobel3_tile_kernel<4, T_TH, true><<<P.ntiles, 128, 0, st>>>(P);
         return after_launch("sobel3_tile_kernel", st, ev);
-      });
+      };
+      if (autotune_idle()) return launch(0);
+      char key[96];
+      snprintf(key, sizeof(key), "sobel3:%dx%dx%d", 1 << (32 - __builtin_clz((unsigned)p.w)),
+               1 << (32 - __builtin_clz((unsigned)p.h)), in->batch);
+      return autotune_run(key, kSobelCfgs, st, launch);
     }
     cudaEvent_t ev = before_launch(st);
     if (low)
