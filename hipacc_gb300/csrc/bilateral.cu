@@ -22,6 +22,7 @@
 #include <cmath>
 
 #include "stage.cuh"
+#include "stage_groups.cuh"
 
 namespace hgb {
 namespace {
@@ -61,8 +62,9 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 
-template <typename T, int S, bool FAST>
-__global__ void __launch_bounds__(BL_BX *BL_BY) bilateral_kernel(const __grid_constant__ BilParams p) {
+// Half-precision weights (flags bit 0).
+template <typename T, int S>
+__global__ void __launch_bounds__(BL_BX *BL_BY) bilateral_half_kernel(const __grid_constant__ BilParams p) {
   using SH_ = BilShape<T, S>;
   constexpr int R = SH_::R, HL = SH_::HL, SW = SH_::SW, SH = SH_::SH;
   __shared__ __align__(16) float tile[SH * SW];
@@ -71,29 +73,16 @@ __global__ void __launch_bounds__(BL_BX *BL_BY) bilateral_kernel(const __grid_co
   stage_tile<T, SW, SH, BL_BX * BL_BY>(tile, p.in + (int64_t)b * p.in_bstride, p.in_pitch, i0 - HL, j0 - R, 0, p.w,
                                         0, p.h, p.bmode, p.cval, p.vec_in);
   __syncthreads();
-  if constexpr (!FAST) {
-    // the FP32 path works on values scaled by q
-    for (int c = threadIdx.x; c < SH * SW; c += BL_BX * BL_BY) tile[c] = __fmul_rn(tile[c], p.q);
-    __syncthreads();
-  }
   const int tx = threadIdx.x % BL_BX, ty = threadIdx.x / BL_BX;
   constexpr int OFF = (HL - R) % 4;
   constexpr int NV = cdiv(OFF + BL_PX + S - 1, 4);
   const int cb = HL - R - OFF + tx * BL_PX;
   float ctr[BL_PX], d[BL_PX], pp[BL_PX];
-  // FP32 path: two pixels per f32x2 lane pair
-  f2 C2[BL_PX / 2], D2[BL_PX / 2], P2[BL_PX / 2];
 #pragma unroll
   for (int px = 0; px < BL_PX; ++px) {
     ctr[px] = tile[(ty + R) * SW + HL + tx * BL_PX + px];
     d[px] = 0.0f;
     pp[px] = 0.0f;
-  }
-#pragma unroll
-  for (int k = 0; k < BL_PX / 2; ++k) {
-    C2[k] = f2_pack(ctr[2 * k], ctr[2 * k + 1]);
-    D2[k] = 0ull;
-    P2[k] = 0ull;
   }
 #pragma unroll 1
   for (int my = 0; my < S; ++my) {
@@ -107,75 +96,167 @@ __global__ void __launch_bounds__(BL_BX *BL_BY) bilateral_kernel(const __grid_co
       win[4 * v + 2] = t.z;
       win[4 * v + 3] = t.w;
     }
-    if constexpr (!FAST) {
-      // window pairs starting at even (E) and odd (O) positions
-      f2 E[NV * 2], O[NV * 2];
+    // two outputs per half2: lanes (px, px+1)
+    const __half2 k2h = __float2half2_rn(p.k2);
+    __half2 c01 = __floats2half2_rn(ctr[0], ctr[1]), c23 = __floats2half2_rn(ctr[2], ctr[3]);
 #pragma unroll
-      for (int j = 0; j < NV * 2; ++j) {
-        E[j] = f2_pack(win[2 * j], win[2 * j + 1]);
-        O[j] = f2_pack(win[2 * j + 1], 2 * j + 2 < NV * 4 ? win[2 * j + 2] : 0.0f);
-      }
-#pragma unroll
-      for (int mx = 0; mx < S; ++mx) {
-        const float nl = -p.lmask[my * S + mx];
-        const f2 NL = f2_pack(nl, nl);
-#pragma unroll
-        for (int k = 0; k < BL_PX / 2; ++k) {
-          const int st = OFF + 2 * k + mx;  // window position of the pair's first pixel
-          const f2 V = (st & 1) ? O[st >> 1] : E[st >> 1];
-          const f2 df = f2_sub(V, C2[k]);
-          const f2 t = f2_fma(df, df, NL);  // d'^2 - lm (measured faster than scalar lm - d'^2)
-          const f2 sw = f2_pack(fast_exp2(-f2_lo(t)), fast_exp2(-f2_hi(t)));
-          D2[k] = f2_add(D2[k], sw);
-          P2[k] = f2_fma(sw, V, P2[k]);
-        }
-      }
-    } else {
-      // two outputs per half2: lanes (px, px+1)
-      const __half2 k2h = __float2half2_rn(p.k2);
-      __half2 c01 = __floats2half2_rn(ctr[0], ctr[1]), c23 = __floats2half2_rn(ctr[2], ctr[3]);
-#pragma unroll
-      for (int mx = 0; mx < S; ++mx) {
-        const __half2 lm = __float2half2_rn(p.lmask[my * S + mx]);
-        const __half2 v01 = __floats2half2_rn(win[OFF + mx], win[OFF + mx + 1]);
-        const __half2 v23 = __floats2half2_rn(win[OFF + mx + 2], win[OFF + mx + 3]);
-        const __half2 df01 = __hsub2(v01, c01), df23 = __hsub2(v23, c23);
-        const float2 s01 = __half22float2(h2exp2(__hfma2(__hmul2(k2h, df01), df01, lm)));
-        const float2 s23 = __half22float2(h2exp2(__hfma2(__hmul2(k2h, df23), df23, lm)));
-        d[0] += s01.x;
-        d[1] += s01.y;
-        d[2] += s23.x;
-        d[3] += s23.y;
-        pp[0] = __fmaf_rn(s01.x, win[OFF + mx], pp[0]);
-        pp[1] = __fmaf_rn(s01.y, win[OFF + mx + 1], pp[1]);
-        pp[2] = __fmaf_rn(s23.x, win[OFF + mx + 2], pp[2]);
-        pp[3] = __fmaf_rn(s23.y, win[OFF + mx + 3], pp[3]);
-      }
+    for (int mx = 0; mx < S; ++mx) {
+      const __half2 lm = __float2half2_rn(p.lmask[my * S + mx]);
+      const __half2 v01 = __floats2half2_rn(win[OFF + mx], win[OFF + mx + 1]);
+      const __half2 v23 = __floats2half2_rn(win[OFF + mx + 2], win[OFF + mx + 3]);
+      const __half2 df01 = __hsub2(v01, c01), df23 = __hsub2(v23, c23);
+      const float2 s01 = __half22float2(h2exp2(__hfma2(__hmul2(k2h, df01), df01, lm)));
+      const float2 s23 = __half22float2(h2exp2(__hfma2(__hmul2(k2h, df23), df23, lm)));
+      d[0] += s01.x;
+      d[1] += s01.y;
+      d[2] += s23.x;
+      d[3] += s23.y;
+      pp[0] = __fmaf_rn(s01.x, win[OFF + mx], pp[0]);
+      pp[1] = __fmaf_rn(s01.y, win[OFF + mx + 1], pp[1]);
+      pp[2] = __fmaf_rn(s23.x, win[OFF + mx + 2], pp[2]);
+      pp[3] = __fmaf_rn(s23.y, win[OFF + mx + 3], pp[3]);
     }
   }
   float res[BL_PX];
-  if constexpr (!FAST) {
 #pragma unroll
-    for (int k = 0; k < BL_PX / 2; ++k) {
-      res[2 * k] = __fmul_rn(__fdiv_rn(f2_lo(P2[k]), f2_lo(D2[k])), p.inv_q);
-      res[2 * k + 1] = __fmul_rn(__fdiv_rn(f2_hi(P2[k]), f2_hi(D2[k])), p.inv_q);
-    }
-  } else {
-#pragma unroll
-    for (int px = 0; px < BL_PX; ++px) res[px] = __fdiv_rn(pp[px], d[px]);
-  }
+  for (int px = 0; px < BL_PX; ++px) res[px] = __fdiv_rn(pp[px], d[px]);
   const int i = i0 + tx * BL_PX, j = j0 + ty;
   if (j < p.h && i < p.w)
     store_row<T, BL_PX>(reinterpret_cast<T *>(p.out + (int64_t)b * p.out_bstride + (int64_t)j * p.out_pitch) + i, res, i,
                         p.w, p.vec_out);
 }
 
+
+// FP32 weights.  A thread owns four (two on small images) columns of two rows, each pixel pair (rows y
+// and y + 1 of a column) one f32x2 lane pair.  The tile is kept as pairs too, cell
+// (r, x) = (v[r][x], v[r + 1][x]), so that a tap's operand for a pixel pair is one
+// aligned register pair straight from a 16-byte load: with horizontal pairs every
+// second one had to be assembled with moves, and the mask's coefficients too
+// (206 issue slots per mask row and 128 pixels against 164, where the FMA pipe and
+// the exponential unit take 208 cycles each).  Row-major tap order per pixel.
+// 13 x 13, f32 4096 x 4096: 469 us before, 425 us now, the FMA pipe and
+// the exponential unit both 72 % busy.
+constexpr int BP_NT = 256, BP_TW = 64;
+// rows of a tile with CPT columns per thread
+constexpr int bp_rows(int cpt) { return 2 * BP_NT / (BP_TW / cpt); }
+
+template <typename T, int S, int CPT>
+__global__ void __launch_bounds__(BP_NT) bilateral_kernel(const __grid_constant__ BilParams p) {
+  constexpr int R = S / 2, HL = round_up(R, 4), SW = BP_TW + 2 * HL, TH = bp_rows(CPT), SH = TH + S - 1, S2 = (S + 1) / 2 * 2;
+  constexpr int OFF = (HL - R) % 2, NC = (OFF + CPT + S - 1 + 1) / 2 * 2;  // cells of a row's window
+  extern __shared__ __align__(16) float bil_smem[];
+  f2 *cell = reinterpret_cast<f2 *>(bil_smem);             // (SH - 1) x SW pairs
+  float *tile = bil_smem + 2 * (SH - 1) * SW;              // SH x SW values
+  __shared__ __align__(16) f2 nl[S][S2];                   // -log2(mask) as pairs
+  const int b = blockIdx.z, i0 = blockIdx.x * BP_TW, j0 = blockIdx.y * TH;
+  for (int k = threadIdx.x; k < S * S2; k += BP_NT) {
+    const int y = k / S2, x = k - y * S2;
+    const float v = x < S ? -p.lmask[y * S + x] : 0.0f;
+    nl[y][x] = f2_pack(v, v);
+  }
+  const float q = p.q;  // the FP32 path works on values scaled by q
+  stage_groups_each<T, SW, SH, BP_NT>(p.in + (int64_t)b * p.in_bstride, p.in_pitch, i0 - HL, j0 - R, 0, p.w, 0, p.h,
+                                      p.bmode, p.cval, R, [=](int c, float4 v) {
+                                        reinterpret_cast<float4 *>(tile)[c] = make_float4(
+                                            __fmul_rn(v.x, q), __fmul_rn(v.y, q), __fmul_rn(v.z, q), __fmul_rn(v.w, q));
+                                      });
+  __syncthreads();
+#pragma unroll 2
+  for (int c = threadIdx.x; c < (SH - 1) * (SW / 2); c += BP_NT) {
+    const float2 lo = reinterpret_cast<const float2 *>(tile)[c], hi = reinterpret_cast<const float2 *>(tile)[c + SW / 2];
+    reinterpret_cast<float4 *>(cell)[c] = make_float4(lo.x, hi.x, lo.y, hi.y);
+  }
+  __syncthreads();
+  const int tx = threadIdx.x % (BP_TW / CPT), ty = threadIdx.x / (BP_TW / CPT);
+  f2 C[CPT], D[CPT], P[CPT];
+#pragma unroll
+  for (int k = 0; k < CPT; ++k) {
+    C[k] = cell[(2 * ty + R) * SW + HL + CPT * tx + k];
+    D[k] = P[k] = 0ull;
+  }
+  const f2 *row = cell + 2 * ty * SW + HL - R - OFF + CPT * tx;
+#pragma unroll 1
+  for (int my = 0; my < S; ++my, row += SW) {
+    f2 W[NC];
+#pragma unroll
+    for (int v = 0; v < NC / 2; ++v) {
+      const ulonglong2 t = reinterpret_cast<const ulonglong2 *>(row)[v];
+      W[2 * v] = t.x;
+      W[2 * v + 1] = t.y;
+    }
+#pragma unroll
+    for (int m2 = 0; m2 < S2 / 2; ++m2) {
+      const ulonglong2 n2 = reinterpret_cast<const ulonglong2 *>(&nl[my][0])[m2];
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        const int mx = 2 * m2 + l;
+        if (mx >= S) continue;
+        const f2 NL = l ? n2.y : n2.x;
+#pragma unroll
+        for (int k = 0; k < CPT; ++k) {
+          const f2 V = W[OFF + mx + k];
+          const f2 df = f2_sub(V, C[k]);
+          const f2 t = f2_fma(df, df, NL);  // d'^2 - lm
+          const f2 sw = f2_pack(fast_exp2(-f2_lo(t)), fast_exp2(-f2_hi(t)));
+          D[k] = f2_add(D[k], sw);
+          P[k] = f2_fma(sw, V, P[k]);
+        }
+      }
+    }
+  }
+  const int i = i0 + CPT * tx;
+  if (i >= p.w) return;
+#pragma unroll
+  for (int l = 0; l < 2; ++l) {
+    const int j = j0 + 2 * ty + l;
+    if (j >= p.h) break;
+    float res[CPT];
+#pragma unroll
+    for (int k = 0; k < CPT; ++k)
+      res[k] = __fmul_rn(l ? __fdiv_rn(f2_hi(P[k]), f2_hi(D[k])) : __fdiv_rn(f2_lo(P[k]), f2_lo(D[k])), p.inv_q);
+    T *dst = reinterpret_cast<T *>(p.out + (int64_t)b * p.out_bstride + (int64_t)j * p.out_pitch) + i;
+    if constexpr (CPT == 4) {
+      store_row<T, 4>(dst, res, i, p.w, p.vec_out);
+    } else {
+#pragma unroll
+      for (int k = 0; k < CPT; ++k)
+        if (i + k < p.w) dst[k] = Storage<T>::from_f(res[k]);
+    }
+  }
+}
+
+template <int S, int CPT>
+constexpr size_t bil_smem_bytes() {
+  constexpr int SW = BP_TW + 2 * round_up(S / 2, 4), SH = bp_rows(CPT) + S - 1;
+  return sizeof(float) * (size_t)SW * (2 * (SH - 1) + SH);
+}
+
+template <typename T, int S, int CPT>
+int launch_bil_pairs(const BilParams &p, int batch, cudaStream_t st) {
+  constexpr size_t smem = bil_smem_bytes<S, CPT>();
+  const int rc = ensure_dynamic_smem((const void *)bilateral_kernel<T, S, CPT>, smem);
+  if (rc) return rc;
+  const dim3 grid(cdiv(p.w, BP_TW), cdiv(p.h, bp_rows(CPT)), batch);
+  cudaEvent_t ev = before_launch(st);
+  bilateral_kernel<T, S, CPT><<<grid, BP_NT, smem, st>>>(p);
+  return after_launch("bilateral_kernel", st, ev);
+}
+
 template <typename T, int S, bool FAST>
 int launch_bil_s(const BilParams &p, int batch, cudaStream_t st) {
-  dim3 grid(cdiv(p.w, BL_TW), cdiv(p.h, BL_TH), batch);
-  cudaEvent_t ev = before_launch(st);
-  bilateral_kernel<T, S, FAST><<<grid, BL_BX * BL_BY, 0, st>>>(p);
-  return after_launch("bilateral_kernel", st, ev);
+  if constexpr (FAST) {
+    const dim3 grid(cdiv(p.w, BL_TW), cdiv(p.h, BL_TH), batch);
+    cudaEvent_t ev = before_launch(st);
+    bilateral_half_kernel<T, S><<<grid, BL_BX * BL_BY, 0, st>>>(p);
+    return after_launch("bilateral_half_kernel", st, ev);
+  } else {
+    // four columns per thread (64 x 32 tiles), or two (64 x 16) where those would
+    // not give every SM two CTAs: a small image's time is one thread's taps
+    // (320 x 256, 13 x 13: 12.9 us with four, 8.0 us with two)
+    if ((int64_t)cdiv(p.w, BP_TW) * cdiv(p.h, bp_rows(4)) * batch >= 2 * num_sms())
+      return launch_bil_pairs<T, S, 4>(p, batch, st);
+    return launch_bil_pairs<T, S, 2>(p, batch, st);
+  }
 }
 
 template <typename T, bool FAST>
@@ -224,7 +305,9 @@ extern "C" int hgb_bilateral(const hgb_view *in, const hgb_view *out, const floa
   p.bmode = boundary;
   p.cval = const_val;
   p.vec_in = ((uintptr_t)in->data % 16 == 0) && in->pitch % 16 == 0 && (in->batch == 1 || in->batch_stride % 16 == 0);
-  p.vec_out = ((uintptr_t)out->data % 16 == 0) && out->pitch % 16 == 0 && (out->batch == 1 || out->batch_stride % 16 == 0);
+  const int64_t four = 4 * dtype_size(out->dtype);  // a thread stores four pixels of a row
+  p.vec_out = (uintptr_t)out->data % four == 0 && out->pitch % four == 0 &&
+              (out->batch == 1 || out->batch_stride % four == 0);
   const double c_r = 0.5 / ((double)sigma_r * (double)sigma_r);
   p.k2 = (float)(-c_r * 1.4426950408889634);  // log2(e)
   p.q = (float)std::sqrt(c_r * 1.4426950408889634);
