@@ -237,6 +237,9 @@ __device__ __forceinline__ void stage_groups(float *tile, const char *in, int64_
                                     [tile](int c, float4 v) { reinterpret_cast<float4 *>(tile)[c] = v; });
 }
 __device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// tiles staged ahead: commit after staging one, then wait for all but the newest
+__device__ __forceinline__ void stage_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void stage_wait_but_newest() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 // The same for a byte tile kept as words; bytes outside the image read 0.
 template <int G, int SH, int NT>

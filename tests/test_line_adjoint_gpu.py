@@ -65,3 +65,30 @@ def test_line_mask_adjoint(gpu, oracle, shape, boundary):
             assert _close(host[0][b].cpu().numpy(), ri), (h, w)
             ref_m = ref_m + rm
         assert np.abs(host[1].cpu().numpy() - ref_m).max() <= 3e-6 * np.abs(gout).sum()
+
+
+@pytest.mark.parametrize("boundary", [0, 1, 2, 3, 4])
+@pytest.mark.parametrize("k", [3, 5, 7])
+def test_square_mask_adjoint_tiles(gpu, oracle, k, boundary):
+    """conv_adjoint.cu at the edges of its 64 x 8 and 64 x 32 tiles, on images smaller
+    than the mask and on rows off 16-byte boundaries: each gradient alone and both.
+    Pixels fold K^2 products (and a few pre-images), tap gradients at most 16 per
+    thread and tile, a warp and a CTA tree: the bounds of the line masks hold."""
+    rng = np.random.default_rng(10 * k + boundary)
+    for h, w in SIZES + [(8, 64), (9, 66)]:
+        img = rng.random((2, h, w + 1)).astype(np.float32)
+        gout = rng.normal(0, 1, (2, h, w)).astype(np.float32)
+        m = rng.random((k, k)).astype(np.float32)
+        x, g = torch.from_numpy(img).cuda()[:, :, :w], torch.from_numpy(gout).cuda()
+        gi, gm = gpu.local_op_adjoint(g, torch.from_numpy(m).cuda(), boundary=boundary, inp=x)
+        alone, _ = gpu.local_op_adjoint(g, m, boundary=boundary, want_grad_mask=False)
+        _, gm2 = gpu.local_op_adjoint(g, m, boundary=boundary, inp=x, want_grad_in=False)
+        assert torch.equal(gi, alone) and torch.equal(gm, gm2)
+        ref_m = 0.0
+        for b in range(2):
+            ri, rm = oracle.local_op_adjoint(img[b][:, :w], gout[b], m, boundary)
+            # positive masks and random signs: compare with the sum of the magnitudes too
+            scale = np.linalg.norm(oracle.local_op_adjoint(img[b][:, :w], np.abs(gout[b]), m, boundary)[0])
+            assert np.linalg.norm(gi[b].cpu().numpy() - ri) <= 2e-6 * scale, (h, w)
+            ref_m = ref_m + rm
+        assert np.abs(gm.cpu().numpy() - ref_m).max() <= 3e-6 * np.abs(gout).sum(), (h, w)
