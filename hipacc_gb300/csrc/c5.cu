@@ -57,6 +57,8 @@
 #include <cmath>
 #include <cstring>
 
+#include "conv_adjoint.h"
+#include "line_adjoint.h"
 #include "band.cuh"
 #include "reduce_common.cuh"
 #include "tma.cuh"
@@ -1076,7 +1078,13 @@ extern "C" int hgb_conv_bilateral_mse(const hgb_view *x, const hgb_view *t, cons
   const dim3 ugrid(cdiv(W, U_TW), cdiv(H, U_TH), B);
   const size_t nblk = (size_t)ugrid.x * ugrid.y * B;  // at least the CTAs of any launch below
   const int red_rows = 64;  // row blocks of the unfused mask-gradient pass
-  const size_t nparts = std::max(nblk, (size_t)B * red_rows);
+  // small batches take the tiled convolution adjoint (conv_adjoint.cu): its frame
+  // pixels go to four lanes each, where c5_conv_adjoint_kernel walks a border
+  // pixel's taps in one thread before and after its tiles (one 139 x 274 image:
+  // 29 us against 14 us, a combine included); larger batches hide that and gain from the TMA stages
+  const bool small = (int64_t)cdiv(W, 64) * cdiv(H, 32) * B < 4 * num_sms();
+  const int cgrid = small ? conv_adjoint_grid(C5_MK, W, H, B) : 0;
+  const size_t nparts = std::max(std::max(nblk, (size_t)B * red_rows), (size_t)cgrid);
   // workspace: the fused form's packed float4 per pixel (or the unfused
   // form's y1, y, a), then dy1, then the partials
   const size_t img_bytes = (size_t)ib * B * 4;
@@ -1142,7 +1150,36 @@ extern "C" int hgb_conv_bilateral_mse(const hgb_view *x, const hgb_view *t, cons
     auto wave = [&](const void *k) { return std::max(1, std::min(p.ntiles, num_sms() * resident_ctas(k, C5_T, 0))); };
     c5_forward_kernel<<<wave((const void *)c5_forward_kernel), C5_T, 0, st>>>(p);
     c5_bilateral_adjoint_kernel<<<wave((const void *)c5_bilateral_adjoint_kernel), C5_T, 0, st>>>(p);
-    c5_conv_adjoint_kernel<<<wave((const void *)c5_conv_adjoint_kernel), C5_T, 0, st>>>(p);
+    if (small) {
+      ConvAdjParams c;
+      memset(&c, 0, sizeof(c));
+      c.in = p.x;
+      c.in_p = x->pitch;
+      c.in_b = x->batch_stride;
+      c.gout = p.dy1;
+      c.gout_p = ip * 4;
+      c.gout_b = ib * 4;
+      c.gin = p.dx;
+      c.gin_p = grad_x->pitch;
+      c.gin_b = grad_x->batch_stride;
+      c.w = W;
+      c.h = H;
+      c.batch = B;
+      c.bmode = boundary;
+      c.mask_dev = mask_dev;
+      c.part = p.dm_part;
+      rc = run_conv_adjoint(C5_MK, &c, cgrid, st);
+      if (rc) return rc;
+      LineCombine lc;
+      memset(&lc, 0, sizeof(lc));
+      lc.part[0] = p.dm_part;
+      lc.out[0] = grad_mask_dev;
+      lc.taps[0] = C5_MK * C5_MK;
+      lc.nparts[0] = cgrid;
+      run_line_combine(lc, st);
+    } else {
+      c5_conv_adjoint_kernel<<<wave((const void *)c5_conv_adjoint_kernel), C5_T, 0, st>>>(p);
+    }
     return after_launch("c5 fused", st, ev);
   }
   // unfused chain, one image at a time
