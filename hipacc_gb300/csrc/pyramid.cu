@@ -414,8 +414,8 @@ __global__ void __launch_bounds__(C::NT, C::MIN_CTAS) pyr_persistent_kernel(cons
   unsigned phase = 0;
   // single == 2 (a cooperative, co-resident grid): the level-0 tiles, which
   // wait on nothing, are taken round-robin without an atomic; the later levels
-  // are claimed.  Otherwise every tile is claimed, kPyClaim consecutive tiles
-  // per atomic for persistent CTAs (the claim counter is one address for the
+  // are claimed.  Otherwise every tile is claimed, up to kPyClaim consecutive
+  // tiles per atomic for persistent CTAs (the claim counter is one address for the
   // whole launch); tiles are processed in list order.
   int claim_base = 0, claim_left = 0;
   int static_next = p.single == 2 ? (int)blockIdx.x : p.nlevel0;
@@ -442,7 +442,11 @@ __global__ void __launch_bounds__(C::NT, C::MIN_CTAS) pyr_persistent_kernel(cons
         static_next += gridDim.x;
       } else {
         if (claim_left == 0) {
-          const int chunk = p.single == 1 ? 1 : kPyClaim;
+          // several tiles per claim only while level 0 has plenty left: near its
+          // end, and in the later levels, a CTA that ran its four in turn kept
+          // the dependants of the last one waiting (one 2048 x 2048 image, eight
+          // levels: 139 us against 56 us; six photographs: 241 against 161 us)
+          const int chunk = p.single == 1 || claim_base + 8 * (int)gridDim.x >= p.nlevel0 ? 1 : kPyClaim;
           if (TRACE) tr.c1 = clock64();
           claim_base = (int)atomicAdd(p.work, (unsigned)chunk) + (p.single == 2 ? p.nlevel0 : 0);
           if (TRACE) tr.claim += clock64() - tr.c1;
