@@ -26,7 +26,8 @@
 //
 // Fused form (mode 0): three persistent kernels over 64 x 16 tiles, 16 x 16
 // threads with four horizontally adjacent pixels each, two pixels per packed
-// f32x2 operation (every lane rounded like the scalar instruction):
+// f32x2 operation (every lane rounded like the scalar instruction; the
+// bilateral adjoint takes two rows of four columns per thread instead):
 //  1. forward: x staged with a radius of 7 through the boundary; y1 on the
 //     tile plus the bilateral radius, eight cells per thread; the bilateral on
 //     u (one ex2 and four packed lane operations per tap and pixel pair); the
@@ -38,15 +39,16 @@
 //     j's own tap -o: one ex2 and ten packed operations per tap serve the
 //     neighbour term, the centre term and dL/dc.  Band pixels, whose taps
 //     cross the edge, go through the pre-images one pixel per thread, as an
-//     equal contiguous share of the batch's band list per CTA after its tiles,
+//     equal contiguous share of the batch's band list per CTA before its tiles,
 //     so the tiles cost the same and the walk has no tail of border tiles.
 //  3. convolution adjoint: grad_in as the transposed convolution away from the
 //     band of radius 3, and the mask gradient accumulated per pair of taps in
 //     packed registers; band pixels again from a flat list.
-// Every CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ...; the
-// reductions (loss, dL/dc, dL/dmask) keep per-thread and per-CTA partials in
-// a fixed assignment and are combined in FP64 in block order by the CTA that
-// takes the last ticket, so results do not change from run to run.
+// The CTAs of 1 and 2 claim chunks of up to four tiles; those of 3 walk tiles
+// blockIdx.x, blockIdx.x + gridDim.x, ....  The reductions keep their partials in
+// a fixed assignment (loss and dL/dc per chunk, dL/dmask per CTA) and are
+// combined in FP64 in that order by the CTA that takes the last ticket, so
+// results do not change from run to run.
 //
 // Unfused form (mode 1): the chain per image as a kernel-per-operator
 // framework launches it (conv, bilateral forward, loss gradient, bilateral
@@ -67,6 +69,7 @@ namespace hgb {
 namespace {
 
 constexpr int C5_T = 256;
+constexpr int BA5_T = 128;  // the fused bilateral adjoint: eight pixels per thread
 constexpr int C5_MK = 7, C5_MR = 3;  // conv mask
 constexpr int C5_BK = 9, C5_BR = 4;  // bilateral
 constexpr int C5_OUT = (int)0x80000000;  // remap result of a CONSTANT tap outside the image
@@ -123,11 +126,12 @@ struct C5Params {
   float2 *loss_part;       // per block Kahan (s, c)
   float *dc_part;          // per block
   float *dm_part;          // per block x 49
-  unsigned int *tickets;   // [0] forward, [1] bilateral adjoint, [2] conv adjoint
+  unsigned int *tickets;   // [0] forward, [1] bilateral adjoint, [2] conv adjoint; [3], [4]: chunk counters of [0], [1]
   double *loss_dev;
   float *grad_mask_dev, *grad_sigma_dev;
   int img_offset;          // image of the launch (per-image launches; 0 otherwise)
   int tiles_x, tiles_y, ntiles;  // tile grid of the launch (all images, or one image)
+  int chunk, nchunks;      // tiles per chunk and chunks of the fused forward and bilateral adjoint
 };
 
 // tile t of the launch: image, origin
@@ -142,16 +146,17 @@ __device__ __forceinline__ void tile_origin(const C5Params &p, int t, int &b, in
 }
 
 // Deterministic block-wide FP64 sum of item(0..n-1): thread t folds items
-// t, t + C5_T, ... in order, then a fixed tree over the threads.  Every thread
+// t, t + NT, ... in order, then a fixed tree over the threads.  Every thread
 // of the block calls it; every thread gets the sum.
-template <class F>
+template <int NT = C5_T, class F>
 __device__ __forceinline__ double block_sum_fixed(int n, F item, double *sh) {
   double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += C5_T) s += item(i);
+#pragma unroll 8
+  for (int i = threadIdx.x; i < n; i += NT) s += item(i);
   sh[threadIdx.x] = s;
   __syncthreads();
 #pragma unroll
-  for (int d = C5_T / 2; d > 0; d >>= 1) {
+  for (int d = NT / 2; d > 0; d >>= 1) {
     if (threadIdx.x < d) sh[threadIdx.x] += sh[threadIdx.x + d];
     __syncthreads();
   }
@@ -175,6 +180,7 @@ __device__ __forceinline__ void sigma_consts(const C5Params &p, float &c, float 
 }
 
 // block-wide sum of a float (thread 0 returns the value)
+template <int NT = C5_T>
 __device__ __forceinline__ float block_sum_f(float v, float *sbuf) {
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
@@ -182,13 +188,49 @@ __device__ __forceinline__ float block_sum_f(float v, float *sbuf) {
   __syncthreads();
   float r = 0.0f;
   if (threadIdx.x == 0)
-    for (int i = 0; i < C5_T / 32; ++i) r += sbuf[i];
+    for (int i = 0; i < NT / 32; ++i) r += sbuf[i];
   __syncthreads();
   return r;
 }
 
-// per-CTA Kahan partial of the squared error, FP64 combine by the last CTA
-__device__ __forceinline__ void loss_publish(const C5Params &p, Kahan lsum, double *dsh) {
+// A CTA's way through the chunks of consecutive tiles: the first chunk is
+// blockIdx.x, the others are claimed in launch order.  Thread 0 claims the next
+// chunk at a chunk's first tile (claim(), before a CTA barrier of that tile);
+// the chunk is read back at the last tile's end, after it.  The CTAs of an SM do
+// not advance alike, so with a fixed walk the slowest ran on alone (16 images
+// 2048 x 2048: 4664 us for the whole step, 4579 us with claims).
+struct ChunkWalk {
+  const C5Params &p;
+  unsigned int *counter;
+  int *next;  // two shared words
+  int chunk, tile, end, par = 0;
+  __device__ ChunkWalk(const C5Params &p_, unsigned int *counter_, int *next_) : p(p_), counter(counter_), next(next_) {
+    enter(blockIdx.x);
+  }
+  __device__ void enter(int c) {
+    chunk = c;
+    tile = c * p.chunk;
+    end = min(tile + p.chunk, p.ntiles);
+  }
+  __device__ bool live() const { return chunk < p.nchunks; }
+  __device__ void claim() {  // thread 0
+    if (tile == chunk * p.chunk) next[par] = min((int)(gridDim.x + atomicAdd(counter, 1u)), p.nchunks);
+  }
+  __device__ bool last() const { return tile + 1 == end; }
+  // the tile after this one, ntiles if there is none (thread 0, after claim())
+  __device__ int peek() const { return !last() ? tile + 1 : next[par] < p.nchunks ? next[par] * p.chunk : p.ntiles; }
+  __device__ void advance() {
+    if (!last()) {
+      ++tile;
+    } else {
+      enter(next[par]);
+      par ^= 1;
+    }
+  }
+};
+
+// Kahan sum of a chunk's squared errors to loss_part[chunk]
+__device__ __forceinline__ void loss_chunk(const C5Params &p, Kahan lsum, int chunk) {
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
     Kahan o;
@@ -199,15 +241,18 @@ __device__ __forceinline__ void loss_publish(const C5Params &p, Kahan lsum, doub
   __shared__ float2 kp[C5_T / 32];
   if ((threadIdx.x & 31) == 0) kp[threadIdx.x >> 5] = make_float2(lsum.s, lsum.c);
   __syncthreads();
-  const unsigned int nb = grid_blocks();
   if (threadIdx.x == 0) {
     Kahan k{0.0f, 0.0f};
     for (int i = 0; i < C5_T / 32; ++i) k = kahan_merge(k, Kahan{kp[i].x, kp[i].y});
-    p.loss_part[block_rank()] = make_float2(k.s, k.c);
+    p.loss_part[chunk] = make_float2(k.s, k.c);
   }
+}
+
+// FP64 combine of the chunks' losses by the last CTA
+__device__ __forceinline__ void loss_publish(const C5Params &p, double *dsh) {
   if (take_last_ticket(p.tickets + 0)) {
     const double s = block_sum_fixed(
-        (int)nb,
+        p.nchunks,
         [&](int i) {
           const float2 v = __ldcg(p.loss_part + i);
           return (double)v.x - (double)v.y;
@@ -216,6 +261,7 @@ __device__ __forceinline__ void loss_publish(const C5Params &p, Kahan lsum, doub
     if (threadIdx.x == 0) {
       *p.loss_dev = s * p.inv_n;
       p.tickets[0] = 0u;
+      p.tickets[3] = 0u;  // every CTA has made its last claim
     }
   }
 }
@@ -269,6 +315,7 @@ __global__ void __launch_bounds__(C5_T, 5) c5_forward_kernel(const __grid_consta
   __shared__ f2 m2[C5_MK * C5_MK];
   __shared__ __align__(16) f2 nl2[C5_BK * NL_W];
   __shared__ __align__(8) uint64_t bars[2];
+  __shared__ int s_next[2];
   double *dsh = reinterpret_cast<double *>(&xst[0][0]);  // the final combine, after the tiles
   const int W = p.w, H = p.h, bm = p.bmode;
   if (p.use_tma && threadIdx.x == 0) {
@@ -297,11 +344,12 @@ __global__ void __launch_bounds__(C5_T, 5) c5_forward_kernel(const __grid_consta
     tile_origin<F_TW, F_TH>(p, tile, b, X0, Y0);
     c5_issue(&bars[s], FX_W * FX_H * 4, xst[s], &p.map_xf, nullptr, nullptr, X0 - 8, Y0 - FX_R, b);
   };
-  if (p.use_tma && threadIdx.x == 0) issue(blockIdx.x, 0);
-  int it = 0;
-  for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x, ++it) {
+  ChunkWalk walk(p, p.tickets + 3, s_next);
+  if (p.use_tma && threadIdx.x == 0) issue(walk.tile, 0);
+  for (int it = 0; walk.live(); ++it) {
     int b, X0, Y0;
-    tile_origin<F_TW, F_TH>(p, tile, b, X0, Y0);
+    tile_origin<F_TW, F_TH>(p, walk.tile, b, X0, Y0);
+    if (threadIdx.x == 0) walk.claim();
     const float *x = p.x + (int64_t)b * p.xb;
     const bool edge = !(X0 >= 8 && X0 - 8 + FX_W <= W && Y0 >= FX_R && Y0 + F_TH + FX_R <= H);
     float *xs = xst[p.use_tma ? (it & 1) : 0];
@@ -309,10 +357,11 @@ __global__ void __launch_bounds__(C5_T, 5) c5_forward_kernel(const __grid_consta
     if (p.use_tma) {
       // the next tile's box lands while this one computes (its stage was last
       // read by the convolution of the previous tile, before a CTA barrier)
-      const bool next = tile + (int)gridDim.x < p.ntiles;
-      if (next && threadIdx.x == 0) {
+      const int next_tile = threadIdx.x == 0 ? walk.peek() : p.ntiles;
+      const bool next = next_tile < p.ntiles;
+      if (next) {
         fence_proxy_async_smem();
-        issue(tile + gridDim.x, (it & 1) ^ 1);
+        issue(next_tile, (it & 1) ^ 1);
       }
       if (!c5_wait(p, bars, it, next)) break;
       if (edge) {  // cells outside the image (zero-filled) through the boundary
@@ -437,15 +486,20 @@ __global__ void __launch_bounds__(C5_T, 5) c5_forward_kernel(const __grid_consta
         orow[gx] = make_float4(Uv[i], a, -a * uy, uy);
       }
     }
+    if (walk.last()) {
+      loss_chunk(p, lsum, walk.chunk);
+      lsum = Kahan{0.0f, 0.0f};
+    }
+    walk.advance();
   }  // tiles
-  loss_publish(p, lsum, dsh);
+  loss_publish(p, dsh);
 }
 
 // one symmetric tap of the bilateral adjoint for a pixel pair j (centre U, A =
 // a_j, B = -a_j u_yj) and its neighbour pair p = j - o (Pu, Pa, PB = -a_p
-// u_yp); s = {sum e a_p, sum e d (u_j a_p - a_p u_yp), sum e d a_j (u_p -
-// u_yj), the same times d} with d = u_j - u_p
-__device__ __forceinline__ void adj_tap(f2 Pu, f2 Pa, f2 PB, f2 U, f2 A, f2 B, f2 NL, f2 (&s)[4]) {
+// u_yp); s = {sum e a_p, sum e d (u_j a_p - a_p u_yp) + e d a_j (u_p - u_yj),
+// the latter's second term times d} with d = u_j - u_p
+__device__ __forceinline__ void adj_tap(f2 Pu, f2 Pa, f2 PB, f2 U, f2 A, f2 B, f2 NL, f2 (&s)[3]) {
   const f2 d = f2_sub(U, Pu);
   const f2 t = f2_fma(d, d, NL);
   const f2 e = f2_pack(ex2f(-f2_lo(t)), ex2f(-f2_hi(t)));
@@ -453,8 +507,8 @@ __device__ __forceinline__ void adj_tap(f2 Pu, f2 Pa, f2 PB, f2 U, f2 A, f2 B, f
   s[0] = f2_fma(e, Pa, s[0]);
   s[1] = f2_fma(h, f2_fma(U, Pa, PB), s[1]);
   const f2 wd = f2_mul(h, f2_fma(A, Pu, B));
-  s[2] = f2_add(s[2], wd);
-  s[3] = f2_fma(wd, d, s[3]);
+  s[1] = f2_add(s[1], wd);
+  s[2] = f2_fma(wd, d, s[2]);
 }
 
 // dL/dy1 of a band pixel j through the pre-images, from the forward's packed
@@ -504,17 +558,25 @@ __device__ float bil_adj_band(const C5Params &p, const float4 *pk, int jy, int j
   return __fmaf_rn(C2S, ctr, dn);
 }
 
-__global__ void __launch_bounds__(C5_T, 4) c5_bilateral_adjoint_kernel(const __grid_constant__ C5Params p) {
-  // per staged position k of a row: (u_k, u_k+1, a_k, a_k+1) and (B_k, B_k+1),
-  // so that a pixel pair's neighbours at any offset are one aligned load each
-  __shared__ __align__(16) float4 sq[FY_H * SQ_W];
-  __shared__ __align__(16) f2 sb[FY_H * SB_W];
+// Bound by the FMA pipe (ten packed operations per tap and pixel pair) as far as the
+// shared-memory loads and the staging let it.  A thread owns four columns of two
+// rows, each pair of rows one f32x2 lane pair: twelve 24-byte loads per mask row serve
+// 36 taps of pixel pairs, where two horizontal pairs of one row took eleven for 18.
+// Four CTAs of 128 threads per SM (five leave 96 registers: 4430 us against 4327 for
+// the whole step).  16 images 2048 x 2048, forward and convolution adjoint
+// included: 4579 us with horizontal pairs, 4293 us now.
+__global__ void __launch_bounds__(BA5_T, 4) c5_bilateral_adjoint_kernel(const __grid_constant__ C5Params p) {
+  // per staged cell of row r: (u_r, u_r+1, a_r, a_r+1) and (B_r, B_r+1) of its
+  // column, so that a pixel pair's neighbours at any offset are one aligned load each
+  __shared__ __align__(16) float4 sq[(FY_H - 1) * SQ_W];
+  __shared__ __align__(16) f2 sb[(FY_H - 1) * SB_W];
   __shared__ __align__(16) f2 nl2[C5_BK * NL_W];
   __shared__ float lsm[C5_BK * C5_BK];
   __shared__ float sbuf[32];
+  __shared__ int s_next[2];
   double *dsh = reinterpret_cast<double *>(sq);  // the final combine, after the tiles
   const int W = p.w, H = p.h;
-  for (int i = threadIdx.x; i < C5_BK * NL_W; i += C5_T) {
+  for (int i = threadIdx.x; i < C5_BK * NL_W; i += BA5_T) {
     const int oy = i / NL_W, ox = i - oy * NL_W;
     const float n = ox < C5_BK ? -p.lsm[oy * C5_BK + ox] : 0.0f;
     nl2[i] = f2_pack(n, n);
@@ -526,70 +588,14 @@ __global__ void __launch_bounds__(C5_T, 4) c5_bilateral_adjoint_kernel(const __g
   const float inv_q3 = inv_q * inv_q * inv_q;
   const int tx = threadIdx.x % F_GX, ty = threadIdx.x / F_GX;
   float dc = 0.0f;
-  for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x) {
-    int b, X0, Y0;
-    tile_origin<F_TW, F_TH>(p, tile, b, X0, Y0);
-    const float4 *pk = p.pk + (int64_t)b * p.ib;
-    __syncthreads();  // the previous tile's reads are done
-    // in-image cells of rows Y0-4 .., columns X0-4 ..: two positions per item
-    for (int it = threadIdx.x; it < FY_H * (FY_W / 2); it += C5_T) {
-      const int r = it / (FY_W / 2), k = (it - r * (FY_W / 2)) * 2;
-      const int gy = Y0 - C5_BR + r, gx = X0 - C5_BR + k;
-      if (gy < 0 || gy >= H) continue;
-      const float4 *src = pk + (int64_t)gy * p.ip;
-      const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      const float4 v0 = (gx >= 0 && gx < W) ? __ldg(src + gx) : z;
-      const float4 v1 = (gx + 1 >= 0 && gx + 1 < W) ? __ldg(src + gx + 1) : z;
-      const float4 v2 = (gx + 2 >= 0 && gx + 2 < W) ? __ldg(src + gx + 2) : z;
-      sq[r * SQ_W + skew8(k)] = make_float4(v0.x, v1.x, v0.y, v1.y);
-      sq[r * SQ_W + skew8(k + 1)] = make_float4(v1.x, v2.x, v1.y, v2.y);
-      sb[r * SB_W + skew16(k)] = f2_pack(v0.z, v1.z);
-      sb[r * SB_W + skew16(k + 1)] = f2_pack(v1.z, v2.z);
-    }
-    __syncthreads();
-    const int jx0 = X0 + 4 * tx, jy = Y0 + ty;
-    if (jx0 >= C5_BR && jx0 + 3 < W - C5_BR && jy >= C5_BR && jy < H - C5_BR) {
-      // skewed position 4 tx + s of a row = base + s + (s < 4 ? 0 : s < 8 ? k1 : k2)
-      const int q1 = tx & 1, b1 = (tx & 3) == 3, b2 = (tx & 3) >= 2;
-      const int qbase = 4 * tx + (tx >> 1), bbase = 4 * tx + (tx >> 2);
-      const int ce_q = (ty + C5_BR) * SQ_W + qbase + q1, ce_b = (ty + C5_BR) * SB_W + bbase + b1;
-      const float4 J0 = sq[ce_q + 4], J1 = sq[ce_q + 6];
-      const f2 U0 = f2_pack(J0.x, J0.y), U1 = f2_pack(J1.x, J1.y);
-      const f2 A0 = f2_pack(J0.z, J0.w), A1 = f2_pack(J1.z, J1.w);
-      const f2 B0 = sb[ce_b + 4], B1 = sb[ce_b + 6];
-      f2 s0[4] = {0ull, 0ull, 0ull, 0ull}, s1[4] = {0ull, 0ull, 0ull, 0ull};
-#pragma unroll 3
-      for (int oy = 0; oy < C5_BK; ++oy) {
-        // neighbours p = j - o: row ty + 8 - oy, positions 4 tx + s, s = 0 .. 10;
-        // pair 0 takes tap ox = 8 - s, pair 1 tap ox = 10 - s
-        const int row = ty + 2 * C5_BR - oy;
-        const float4 *qr = &sq[row * SQ_W + qbase];
-        const f2 *br = &sb[row * SB_W + bbase];
-        f2 NL[NL_W];
-        nl_row(&nl2[oy * NL_W], NL);
-#pragma unroll
-        for (int s = 0; s <= 2 * C5_BR + 2; ++s) {
-          const float4 P = qr[s + (s < 4 ? 0 : s < 8 ? q1 : 1)];
-          const f2 Pu = f2_pack(P.x, P.y), Pa = f2_pack(P.z, P.w), PB = br[s + (s < 4 ? 0 : s < 8 ? b1 : b2)];
-          if (s <= 2 * C5_BR) adj_tap(Pu, Pa, PB, U0, A0, B0, NL[2 * C5_BR - s], s0);
-          if (s >= 2) adj_tap(Pu, Pa, PB, U1, A1, B1, NL[2 * C5_BR + 2 - s], s1);
-        }
-      }
-      // dL/dy1 = sum e a_p - C2S (neighbour sum + centre sum); dL/dc share -s3 / q^3
-      const float4 o = make_float4(f2_lo(s0[0]) - C2S * (f2_lo(s0[1]) + f2_lo(s0[2])),
-                                   f2_hi(s0[0]) - C2S * (f2_hi(s0[1]) + f2_hi(s0[2])),
-                                   f2_lo(s1[0]) - C2S * (f2_lo(s1[1]) + f2_lo(s1[2])),
-                                   f2_hi(s1[0]) - C2S * (f2_hi(s1[1]) + f2_hi(s1[2])));
-      *reinterpret_cast<float4 *>(p.dy1 + (int64_t)b * p.ib + (int64_t)jy * p.ip + jx0) = o;
-      dc = __fmaf_rn(-inv_q3, (f2_lo(s0[3]) + f2_hi(s0[3])) + (f2_lo(s1[3]) + f2_hi(s1[3])), dc);
-    }
-  }  // tiles
-  // band pixels of every image of the batch: an equal contiguous share per CTA
+  __syncthreads();  // lsm
+  // band pixels of every image of the batch: an equal contiguous share per CTA,
+  // ahead of the tiles, whose claims then even out the end
   {
     const int per = band_size(W, H, C5_BR);
     int64_t k0, k1;
     cta_share((int64_t)per * p.batch, k0, k1);
-    for (int64_t k = k0 + threadIdx.x; k < k1; k += C5_T) {
+    for (int64_t k = k0 + threadIdx.x; k < k1; k += BA5_T) {
       const int b = (int)(k / per);
       int jy, jx;
       band_pos((int)(k - (int64_t)b * per), W, H, C5_BR, jy, jx);
@@ -597,15 +603,96 @@ __global__ void __launch_bounds__(C5_T, 4) c5_bilateral_adjoint_kernel(const __g
       p.dy1[(int64_t)b * p.ib + (int64_t)jy * p.ip + jx] = g;
     }
   }
-  const float bdc = block_sum_f(dc, sbuf);
-  const unsigned int nb = grid_blocks();
-  if (threadIdx.x == 0) p.dc_part[block_rank()] = bdc;
+  {
+    const float s = block_sum_f<BA5_T>(dc, sbuf);
+    if (threadIdx.x == 0) p.dc_part[p.nchunks + blockIdx.x] = s;
+    dc = 0.0f;
+  }
+  for (ChunkWalk walk(p, p.tickets + 4, s_next); walk.live(); walk.advance()) {
+    int b, X0, Y0;
+    tile_origin<F_TW, F_TH>(p, walk.tile, b, X0, Y0);
+    const float4 *pk = p.pk + (int64_t)b * p.ib;
+    __syncthreads();  // the previous tile's reads are done
+    if (threadIdx.x == 0) walk.claim();
+    // in-image cells of rows Y0-4 .., columns X0-4 ..: four cells of a column per item
+    for (int it = threadIdx.x; it < (FY_H / 4) * FY_W; it += BA5_T) {
+      const int g = it / FY_W, c = it - g * FY_W, r = 4 * g;
+      const int gy = Y0 - C5_BR + r, gx = X0 - C5_BR + c;
+      if (gx < 0 || gx >= W) continue;
+      const float4 *src = pk + (int64_t)gy * p.ip + gx;
+      float4 v[5];
+#pragma unroll
+      for (int i = 0; i < 5; ++i)
+        v[i] = gy + i >= 0 && gy + i < H ? __ldg(src + (int64_t)i * p.ip) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (r + i == FY_H - 1) break;
+        sq[(r + i) * SQ_W + skew8(c)] = make_float4(v[i].x, v[i + 1].x, v[i].y, v[i + 1].y);
+        sb[(r + i) * SB_W + skew16(c)] = f2_pack(v[i].z, v[i + 1].z);
+      }
+    }
+    __syncthreads();
+    // columns jx0 .. jx0 + 3 of rows jy and jy + 1 (a lane pair each); the band's
+    // first row below may be jy + 1, which then only goes along
+    const int jx0 = X0 + 4 * tx, jy = Y0 + 2 * ty;
+    if (jx0 >= C5_BR && jx0 + 3 < W - C5_BR && jy >= C5_BR && jy < H - C5_BR) {
+      // skewed position 4 tx + s of a row = base + s + (s < 4 ? 0 : s < 8 ? k1 : k2)
+      const int q1 = tx & 1, b1 = (tx & 3) == 3, b2 = (tx & 3) >= 2;
+      const int qbase = 4 * tx + (tx >> 1), bbase = 4 * tx + (tx >> 2);
+      const float4 *ce_q = &sq[(2 * ty + C5_BR) * SQ_W + qbase + q1];
+      const f2 *ce_b = &sb[(2 * ty + C5_BR) * SB_W + bbase + b1];
+      f2 U[4], A[4], B[4], s[4][3];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 J = ce_q[4 + i];
+        U[i] = f2_pack(J.x, J.y);
+        A[i] = f2_pack(J.z, J.w);
+        B[i] = ce_b[4 + i];
+        s[i][0] = s[i][1] = s[i][2] = 0ull;
+      }
+#pragma unroll 3
+      for (int oy = 0; oy < C5_BK; ++oy) {
+        // neighbours p = j - o: cell row 2 ty + 8 - oy, positions 4 tx + v, v = 0 .. 11;
+        // column i takes tap ox = 8 + i - v
+        const int row = 2 * ty + 2 * C5_BR - oy;
+        const float4 *qr = &sq[row * SQ_W + qbase];
+        const f2 *br = &sb[row * SB_W + bbase];
+        f2 NL[NL_W];
+        nl_row(&nl2[oy * NL_W], NL);
+#pragma unroll
+        for (int v = 0; v <= 2 * C5_BR + 3; ++v) {
+          const float4 P = qr[v + (v < 4 ? 0 : v < 8 ? q1 : 1)];
+          const f2 Pu = f2_pack(P.x, P.y), Pa = f2_pack(P.z, P.w), PB = br[v + (v < 4 ? 0 : v < 8 ? b1 : b2)];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (v >= i && v <= 2 * C5_BR + i) adj_tap(Pu, Pa, PB, U[i], A[i], B[i], NL[2 * C5_BR + i - v], s[i]);
+        }
+      }
+      // dL/dy1 = sum e a_p - C2S (neighbour and centre sum); dL/dc share -s2 / q^3
+      float *dst = p.dy1 + (int64_t)b * p.ib + (int64_t)jy * p.ip + jx0;
+      const auto lo = [&](int i) { return f2_lo(s[i][0]) - C2S * f2_lo(s[i][1]); };
+      const auto hi = [&](int i) { return f2_hi(s[i][0]) - C2S * f2_hi(s[i][1]); };
+      *reinterpret_cast<float4 *>(dst) = make_float4(lo(0), lo(1), lo(2), lo(3));
+      float w = (f2_lo(s[0][2]) + f2_lo(s[1][2])) + (f2_lo(s[2][2]) + f2_lo(s[3][2]));
+      if (jy + 1 < H - C5_BR) {
+        *reinterpret_cast<float4 *>(dst + p.ip) = make_float4(hi(0), hi(1), hi(2), hi(3));
+        w += (f2_hi(s[0][2]) + f2_hi(s[1][2])) + (f2_hi(s[2][2]) + f2_hi(s[3][2]));
+      }
+      dc = __fmaf_rn(-inv_q3, w, dc);
+    }
+    if (walk.last()) {
+      const float s = block_sum_f<BA5_T>(dc, sbuf);
+      if (threadIdx.x == 0) p.dc_part[walk.chunk] = s;
+      dc = 0.0f;
+    }
+  }  // tiles
   if (take_last_ticket(p.tickets + 1)) {
-    const double s = block_sum_fixed((int)nb, [&](int i) { return (double)__ldcg(p.dc_part + i); }, dsh);
+    const double s = block_sum_fixed<BA5_T>(p.nchunks + (int)gridDim.x, [&](int i) { return (double)__ldcg(p.dc_part + i); }, dsh);
     if (threadIdx.x == 0) {
       const double sg = (double)__ldg(p.sigma_dev);
       *p.grad_sigma_dev = (float)(s * (-1.0 / (sg * sg * sg)));
       p.tickets[1] = 0u;
+      p.tickets[4] = 0u;  // every CTA has made its last claim
     }
   }
 }
@@ -1084,7 +1171,15 @@ extern "C" int hgb_conv_bilateral_mse(const hgb_view *x, const hgb_view *t, cons
   // 29 us against 14 us, a combine included); larger batches hide that and gain from the TMA stages
   const bool small = (int64_t)cdiv(W, 64) * cdiv(H, 32) * B < 4 * num_sms();
   const int cgrid = small ? conv_adjoint_grid(C5_MK, W, H, B) : 0;
-  const size_t nparts = std::max(std::max(nblk, (size_t)B * red_rows), (size_t)cgrid);
+  // chunks of up to four tiles, at least some 16 per CTA (shorter ones would add to the
+  // combine of their partials, longer ones to the wait for the last)
+  const int ftiles = cdiv(W, F_TW) * cdiv(H, F_TH) * B;
+  const int fgrid = num_sms() * resident_ctas((const void *)c5_bilateral_adjoint_kernel, BA5_T, 0);
+  const int chunk = std::max(1, std::min(4, ftiles / (16 * std::max(1, fgrid))));
+  const int nchunks = cdiv(ftiles, chunk);
+  // dL/dc has a partial per chunk and one per CTA for its share of the band
+  const size_t nparts =
+      std::max(std::max(nblk, (size_t)B * red_rows), std::max((size_t)cgrid, (size_t)nchunks + std::min(nchunks, fgrid)));
   // workspace: the fused form's packed float4 per pixel (or the unfused
   // form's y1, y, a), then dy1, then the partials
   const size_t img_bytes = (size_t)ib * B * 4;
@@ -1146,10 +1241,15 @@ extern "C" int hgb_conv_bilateral_mse(const hgb_view *x, const hgb_view *t, cons
     // persistent grids: one wave of resident CTAs walking the tiles
     p.tiles_x = cdiv(W, F_TW);
     p.tiles_y = cdiv(H, F_TH);
-    p.ntiles = p.tiles_x * p.tiles_y * B;
-    auto wave = [&](const void *k) { return std::max(1, std::min(p.ntiles, num_sms() * resident_ctas(k, C5_T, 0))); };
-    c5_forward_kernel<<<wave((const void *)c5_forward_kernel), C5_T, 0, st>>>(p);
-    c5_bilateral_adjoint_kernel<<<wave((const void *)c5_bilateral_adjoint_kernel), C5_T, 0, st>>>(p);
+    p.ntiles = ftiles;
+    p.chunk = chunk;
+    p.nchunks = nchunks;
+    auto wave = [&](const void *k, int work) {
+      return std::max(1, std::min(work, num_sms() * resident_ctas(k, C5_T, 0)));
+    };
+    const int agrid = std::max(1, std::min(nchunks, fgrid));
+    c5_forward_kernel<<<wave((const void *)c5_forward_kernel, nchunks), C5_T, 0, st>>>(p);
+    c5_bilateral_adjoint_kernel<<<agrid, BA5_T, 0, st>>>(p);
     if (small) {
       ConvAdjParams c;
       memset(&c, 0, sizeof(c));
@@ -1178,7 +1278,7 @@ extern "C" int hgb_conv_bilateral_mse(const hgb_view *x, const hgb_view *t, cons
       lc.nparts[0] = cgrid;
       run_line_combine(lc, st);
     } else {
-      c5_conv_adjoint_kernel<<<wave((const void *)c5_conv_adjoint_kernel), C5_T, 0, st>>>(p);
+      c5_conv_adjoint_kernel<<<wave((const void *)c5_conv_adjoint_kernel, p.ntiles), C5_T, 0, st>>>(p);
     }
     return after_launch("c5 fused", st, ev);
   }
