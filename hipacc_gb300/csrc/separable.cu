@@ -22,8 +22,14 @@
 // of an FP32 tile, so more CTAs per SM); cells outside the image, which TMA
 // fills with zeros, are patched with the boundary rule (a CONSTANT cell holds
 // the constant in the storage type).  Other layouts stage an FP32 tile with
-// 16-byte global loads.  Both passes run packed f32x2 fused multiply-adds on
-// pairs of adjacent outputs, keeping each output's tap order.
+// 16-byte global loads, in an instantiation of their own (f32 1023 x 767, 9 taps: 8.5
+// us with both stagings in one kernel, 7.2 us now).  Both passes run packed f32x2 fused
+// multiply-adds on pairs of adjacent outputs, keeping each output's tap order.
+// 16-bit tiles take eight outputs per lane in the row pass (row_pass8); for FP32
+// ones, whose lanes would read 32 bytes apart, four remain.  bf16, four outputs
+// per lane against eight: 13 taps 4 x 1920 x 1080 22.3 against 19.0 us, 9 taps
+// 8192 x 8192 97.3 against 96.0 us: there the chain of tile load, row pass and
+// column pass, with a barrier between each, bounds a tile more than their instructions.
 #include <algorithm>
 #include <type_traits>
 
@@ -131,7 +137,44 @@ __device__ __forceinline__ void row_pass(const SepParams &p, const TT *tile, flo
   }
 }
 
-template <typename T, int K>
+// 16-byte units of a row-buffer row: unit u of four columns lies at sep_unit(u), so that
+// both a lane with two adjacent units (row_pass8's stores) and one with a unit (the
+// column pass) meet eight bank groups per eight lanes
+__device__ __forceinline__ int sep_unit(int u) { return u ^ ((u >> 3) & 1); }
+
+// row pass over a 16-bit tile: 8 outputs per lane, two rows per warp.  A lane's 24
+// cells are three 16-byte loads, and a tap pair, which must be in registers (a packed
+// operation takes no constant operand), serves four operations instead of two.
+template <typename TT, int K, int SW, int SH>
+__device__ __forceinline__ void row_pass8(const SepParams &p, const TT *tile, float *rowb, int j0) {
+  constexpr int R = K / 2, OFF = 8 - R;  // outputs 8 l ..: cells 8 l + OFF ..
+  const int l = threadIdx.x % 16;
+  float *dst = rowb + 4 * sep_unit(2 * l);
+  const int dhi = 4 * (sep_unit(2 * l + 1) - sep_unit(2 * l));
+  for (int r = threadIdx.x / 16; r < SH; r += SP_BX * SP_BY / 16) {
+    float win[24];
+#pragma unroll
+    for (int v = 0; v < 3; ++v)
+      Vec16<TT>::unpack(*reinterpret_cast<const uint4 *>(&tile[r * SW + 8 * (l + v)]), win + 8 * v);
+    f2 a[4];
+#pragma unroll
+    for (int pp = 0; pp < 4; ++pp) a[pp] = 0ull;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int pp = 0; pp < 4; ++pp)
+        a[pp] = f2_fma(p.row2[k], f2_pack(win[OFF + 2 * pp + k], win[OFF + 2 * pp + k + 1]), a[pp]);
+    const int ay = j0 - R + r;
+    if (p.bmode == HGB_BOUNDARY_CONSTANT && (ay < 0 || ay >= p.h))
+#pragma unroll
+      for (int pp = 0; pp < 4; ++pp) a[pp] = f2_pack(p.cval, p.cval);
+    float *o = dst + r * SP_TW;
+    *reinterpret_cast<float4 *>(o) = make_float4(f2_lo(a[0]), f2_hi(a[0]), f2_lo(a[1]), f2_hi(a[1]));
+    *reinterpret_cast<float4 *>(o + dhi) = make_float4(f2_lo(a[2]), f2_hi(a[2]), f2_lo(a[3]), f2_hi(a[3]));
+  }
+}
+
+template <typename T, int K, bool TMA>
 __global__ void __launch_bounds__(SP_BX *SP_BY) separable_kernel(const __grid_constant__ SepParams p) {
   using S = SepShape<T, K>;
   constexpr int R = S::R, HL = S::HL, SW = S::SW, SH = S::SH;
@@ -144,8 +187,10 @@ __global__ void __launch_bounds__(SP_BX *SP_BY) separable_kernel(const __grid_co
   const int X0 = i0 - HL, Y0 = j0 - R;
   const char *img = p.in + (int64_t)b * p.in_bstride;
   const int tx = threadIdx.x % SP_BX, ty = threadIdx.x / SP_BX;
+  constexpr bool kWide = TMA && sizeof(T) == 2;  // row_pass8, with its layout of the row buffer
+  static_assert(!kWide || (HL == 8 && SW == SP_TW + 16), "a lane's window is 24 cells from 8 l");
   float *rowb;
-  if (p.use_tma) {
+  if constexpr (TMA) {
     // the tile stays in the storage type; the row pass widens as it reads
     T *tile = reinterpret_cast<T *>(base);
     rowb = reinterpret_cast<float *>(base + S::tile_tma);
@@ -196,7 +241,10 @@ __global__ void __launch_bounds__(SP_BX *SP_BY) separable_kernel(const __grid_co
       }
     }
     __syncthreads();
-    row_pass<T, K, SW, SH, HL>(p, tile, rowb, j0, tx, ty);
+    if constexpr (kWide)
+      row_pass8<T, K, SW, SH>(p, tile, rowb, j0);
+    else
+      row_pass<T, K, SW, SH, HL>(p, tile, rowb, j0, tx, ty);
   } else {
     float *tile = reinterpret_cast<float *>(base);
     rowb = reinterpret_cast<float *>(base + S::tile_ldg);
@@ -206,6 +254,7 @@ __global__ void __launch_bounds__(SP_BX *SP_BY) separable_kernel(const __grid_co
   }
   __syncthreads();
   // ---- column pass: 4 x 4 outputs per thread
+  const float *colb = rowb + ty * SP_PY * SP_TW + 4 * (kWide ? sep_unit(tx) : tx);
   f2 c2[SP_PY][SP_PX / 2];
 #pragma unroll
   for (int oy = 0; oy < SP_PY; ++oy)
@@ -213,7 +262,7 @@ __global__ void __launch_bounds__(SP_BX *SP_BY) separable_kernel(const __grid_co
     for (int pp = 0; pp < SP_PX / 2; ++pp) c2[oy][pp] = 0ull;
 #pragma unroll
   for (int r = 0; r < SP_PY + K - 1; ++r) {
-    const float4 t = *reinterpret_cast<const float4 *>(&rowb[(ty * SP_PY + r) * SP_TW + tx * SP_PX]);
+    const float4 t = *reinterpret_cast<const float4 *>(colb + r * SP_TW);
     const f2 v01 = f2_pack(t.x, t.y), v23 = f2_pack(t.z, t.w);
 #pragma unroll
     for (int oy = 0; oy < SP_PY; ++oy) {
@@ -260,11 +309,12 @@ int launch_sep_k(const SepParams &p0, int batch, cudaStream_t st) {
     p.status = device_status_word();
   }
   const size_t smem = p.use_tma ? S::smem_tma : S::smem_ldg;
-  const int rc = ensure_dynamic_smem((const void *)separable_kernel<T, K>, smem);
+  const auto kern = p.use_tma ? separable_kernel<T, K, true> : separable_kernel<T, K, false>;
+  const int rc = ensure_dynamic_smem((const void *)kern, smem);
   if (rc) return rc;
   dim3 grid(cdiv(p.w, SP_TW), cdiv(p.h, SP_TH), batch);
   cudaEvent_t ev = before_launch(st);
-  separable_kernel<T, K><<<grid, SP_BX * SP_BY, smem, st>>>(p);
+  kern<<<grid, SP_BX * SP_BY, smem, st>>>(p);
   return after_launch("separable_kernel", st, ev);
 }
 
