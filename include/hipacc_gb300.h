@@ -405,9 +405,9 @@ HGB_API int hgb_bilateral_adjoint(const hgb_view *in, const hgb_view *grad_out, 
  *   NULL, k floats each, device)        = dL/drow_taps, dL/dcol_taps, combined in
  *                                         FP64 in a fixed order.
  * Same taps / k / boundary / const_val as the forward (const_val recomputes t;
- * the tap gradients count CONSTANT taps outside as reading 0).  Composed from
- * hgb_local_op and hgb_local_op_adjoint; uses the library workspace (8 bytes
- * per pixel): calls sharing it must be ordered on one stream. */
+ * the tap gradients count CONSTANT taps outside as reading 0).  Uses the
+ * library workspace (4 bytes per pixel for odd k from 3 to 15, else 8, with
+ * rows padded to 16 bytes): calls sharing it must be ordered on one stream. */
 HGB_API int hgb_separable_adjoint(const hgb_view *in, const hgb_view *grad_out, const float *row_taps,
                                   const float *col_taps, int k, int boundary, float const_val,
                                   const hgb_view *grad_in, float *grad_row_dev, float *grad_col_dev, void *stream);
@@ -422,7 +422,7 @@ HGB_API int hgb_separable_adjoint(const hgb_view *in, const hgb_view *grad_out, 
  * for convolve); nothing flows when no tap replaced the initial value or when
  * the winner was a CONSTANT tap outside the image.  grad_in is gathered per
  * pixel in a fixed order (deterministic).  FP32 storage, masks up to 15 x 15.
- * Uses the library workspace (1 byte per pixel). */
+ * Uses the library workspace (1 byte per pixel, rows padded to whole words). */
 HGB_API int hgb_local_op_minmax_adjoint(const hgb_view *in, const hgb_view *grad_out, const hgb_view *grad_in,
                                         const float *mask, const uint8_t *domain, int mask_w, int mask_h,
                                         int reduce, int boundary, float const_val, void *stream);
