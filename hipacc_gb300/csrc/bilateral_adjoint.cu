@@ -32,9 +32,9 @@
 //  1. bpk_forward_kernel: the bilateral over 64 x 16 tiles, four pixels per
 //     thread, two per packed f32x2 operation; it writes per pixel the float4
 //     (u, a, -a u_y, u_y) with u = q in, u_y = q y, a = g / W;
-//  2. bpk_adjoint_kernel: persistent CTAs over the tiles; staged rows hold
-//     pairs (u_k, u_k+1, a_k, a_k+1) and (B_k, B_k+1), skewed against bank
-//     conflicts; one ex2 and ten packed lane operations per tap serve the
+//  2. bpk_adjoint_kernel: persistent CTAs over the tiles; staged cells hold
+//     the pairs of two rows, (u_r, u_r+1, a_r, a_r+1) and (B_r, B_r+1), skewed
+//     against bank conflicts; one ex2 and ten packed lane operations per tap serve the
 //     neighbour term, the centre term and dL/dc; pixels within the radius of
 //     an edge take the pre-image path from a flat band list (band.cuh), an
 //     equal share per CTA after its tiles;
@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(BA_T) bil_adjoint_kernel(const __grid_constant
 }
 
 // ---------------------------------------------------------------- packed form
+constexpr int BPA_T = 128;  // threads of the packed adjoint: eight pixels each
 constexpr int BP_TW = 64, BP_TH = 16, BP_GX = BP_TW / 4, BP_SW = BP_TW + 16;  // staged in: columns X0-8 ..
 constexpr float BP_C2S = 1.3862943611198906f;                                  // 2 ln 2
 
@@ -309,9 +310,9 @@ __global__ void __launch_bounds__(BA_T) bpk_forward_kernel(const __grid_constant
 }
 
 // one symmetric tap for a pixel pair: centre (U, A = a_j, B = -a_j u_yj),
-// neighbour pair (Pu, Pa, PB); s = {sum e a_p, sum e d (u_j a_p - a_p u_yp),
-// sum e d a_j (u_p - u_yj), the same times d}, d = u_j - u_p
-__device__ __forceinline__ void bpk_tap(f2 Pu, f2 Pa, f2 PB, f2 U, f2 A, f2 B, f2 NL, f2 (&s)[4]) {
+// neighbour pair (Pu, Pa, PB); s = {sum e a_p, sum e d (u_j a_p - a_p u_yp) +
+// e d a_j (u_p - u_yj), the latter's second term times d}, d = u_j - u_p
+__device__ __forceinline__ void bpk_tap(f2 Pu, f2 Pa, f2 PB, f2 U, f2 A, f2 B, f2 NL, f2 (&s)[3]) {
   const f2 d = f2_sub(U, Pu);
   const f2 t = f2_fma(d, d, NL);
   const f2 e = f2_pack(ex2_approx(-f2_lo(t)), ex2_approx(-f2_hi(t)));
@@ -319,8 +320,8 @@ __device__ __forceinline__ void bpk_tap(f2 Pu, f2 Pa, f2 PB, f2 U, f2 A, f2 B, f
   s[0] = f2_fma(e, Pa, s[0]);
   s[1] = f2_fma(h, f2_fma(U, Pa, PB), s[1]);
   const f2 wd = f2_mul(h, f2_fma(A, Pu, B));
-  s[2] = f2_add(s[2], wd);
-  s[3] = f2_fma(wd, d, s[3]);
+  s[1] = f2_add(s[1], wd);
+  s[2] = f2_fma(wd, d, s[2]);
 }
 
 // dL/din of a band pixel j through the pre-images, from the packed values;
@@ -374,23 +375,28 @@ template <int K>
 struct BpkShape {
   static constexpr int R = K / 2, FW = BP_TW + 2 * R, FH = BP_TH + 2 * R;  // staged positions: columns X0-R ..
   static constexpr int SQW = FW + FW / 8, SBW = FW + FW / 16;               // skewed row strides
-  static constexpr size_t smem = (size_t)FH * SQW * 16 + (size_t)FH * SBW * 8 + 128;
+  static constexpr size_t smem = (size_t)(FH - 1) * SQW * 16 + (size_t)(FH - 1) * SBW * 8 + 128;
 };
 __device__ __forceinline__ int bp_sk8(int k) { return k + (k >> 3); }
 __device__ __forceinline__ int bp_sk16(int k) { return k + (k >> 4); }
 
+// Bound by the FMA pipe, as the differentiation step's adjoint.  A thread owns four
+// columns of two rows, each pair of rows one f32x2 lane pair, so that K + 3 loads of 24
+// bytes per mask row serve 4 K taps of pixel pairs; two horizontal pairs of one row took
+// K + 2 for 2 K.  Forward filter and its adjoint, 9 x 9, 4096 x 4096: 1217 us with
+// horizontal pairs in both, 1088 us now; 7 x 7, two images 1531 x 1203: 215 against 181 us.
 template <int K>
-__global__ void __launch_bounds__(BA_T) bpk_adjoint_kernel(const __grid_constant__ BilAdjParams p) {
+__global__ void __launch_bounds__(BPA_T, 4) bpk_adjoint_kernel(const __grid_constant__ BilAdjParams p) {
   using S = BpkShape<K>;
   constexpr int R = S::R, FW = S::FW, FH = S::FH, SQW = S::SQW, SBW = S::SBW, NLW = K + 1;
   extern __shared__ __align__(16) uint8_t bpk_dsm[];
-  float4 *sq = reinterpret_cast<float4 *>(bpk_dsm);                    // (u_k, u_k+1, a_k, a_k+1)
-  f2 *sb = reinterpret_cast<f2 *>(bpk_dsm + (size_t)FH * SQW * 16);  // (B_k, B_k+1)
+  float4 *sq = reinterpret_cast<float4 *>(bpk_dsm);                    // (u_r, u_r+1, a_r, a_r+1)
+  f2 *sb = reinterpret_cast<f2 *>(bpk_dsm + (size_t)(FH - 1) * SQW * 16);  // (B_r, B_r+1)
   __shared__ __align__(16) f2 nl2[K * NLW];
   __shared__ float lm[K * K];
-  __shared__ double s_dc[BA_T / 32];
+  __shared__ double s_dc[BPA_T / 32];
   const int W = p.w, H = p.h;
-  for (int i = threadIdx.x; i < K * NLW; i += BA_T) {
+  for (int i = threadIdx.x; i < K * NLW; i += BPA_T) {
     const int oy = i / NLW, ox = i - oy * NLW;
     const float n = ox < K ? -p.lm[oy * K + ox] : 0.0f;
     nl2[i] = f2_pack(n, n);
@@ -403,56 +409,72 @@ __global__ void __launch_bounds__(BA_T) bpk_adjoint_kernel(const __grid_constant
     bp_tile(p, t, b, X0, Y0);
     const float4 *pk = p.pk + (int64_t)b * W * H;
     __syncthreads();  // the previous tile's reads are done (and nl2 / lm written)
-    // in-image cells of rows Y0-R .., columns X0-R ..: two positions per item
-    for (int it = threadIdx.x; it < FH * (FW / 2); it += BA_T) {
-      const int r = it / (FW / 2), k = (it - r * (FW / 2)) * 2;
-      const int gy = Y0 - R + r, gx = X0 - R + k;
-      if (gy < 0 || gy >= H) continue;
-      const float4 *src = pk + (int64_t)gy * W;
-      const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      const float4 v0 = (gx >= 0 && gx < W) ? src[gx] : z;
-      const float4 v1 = (gx + 1 >= 0 && gx + 1 < W) ? src[gx + 1] : z;
-      const float4 v2 = (gx + 2 >= 0 && gx + 2 < W) ? src[gx + 2] : z;
-      sq[r * SQW + bp_sk8(k)] = make_float4(v0.x, v1.x, v0.y, v1.y);
-      sq[r * SQW + bp_sk8(k + 1)] = make_float4(v1.x, v2.x, v1.y, v2.y);
-      sb[r * SBW + bp_sk16(k)] = f2_pack(v0.z, v1.z);
-      sb[r * SBW + bp_sk16(k + 1)] = f2_pack(v1.z, v2.z);
+    // in-image columns of rows Y0-R .., zero outside: four cells of a column per item
+    for (int it = threadIdx.x; it < cdiv(FH - 1, 4) * FW; it += BPA_T) {
+      const int g = it / FW, c = it - g * FW, r = 4 * g;
+      const int gy = Y0 - R + r, gx = X0 - R + c;
+      if (gx < 0 || gx >= W) continue;
+      const float4 *src = pk + (int64_t)gy * W + gx;
+      float4 v[5];
+#pragma unroll
+      for (int i = 0; i < 5; ++i)
+        v[i] = gy + i >= 0 && gy + i < H ? src[(int64_t)i * W] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (r + i >= FH - 1) break;
+        sq[(r + i) * SQW + bp_sk8(c)] = make_float4(v[i].x, v[i + 1].x, v[i].y, v[i + 1].y);
+        sb[(r + i) * SBW + bp_sk16(c)] = f2_pack(v[i].z, v[i + 1].z);
+      }
     }
     __syncthreads();
-    const int jx0 = X0 + 4 * tx, jy = Y0 + ty;
-    if (jx0 >= band_left(R) && jx0 + 3 < W - R && jy >= R && jy < H - R) {
-      // positions 4 tx + s of a row: pair pp's centre at s = R + 2 pp, its
-      // neighbours for tap ox at s = 2R + 2 pp - ox
-      const int cq = (ty + R) * SQW, cb = (ty + R) * SBW;
-      const float4 J0 = sq[cq + bp_sk8(4 * tx + R)], J1 = sq[cq + bp_sk8(4 * tx + R + 2)];
-      const f2 U0 = f2_pack(J0.x, J0.y), U1 = f2_pack(J1.x, J1.y);
-      const f2 A0 = f2_pack(J0.z, J0.w), A1 = f2_pack(J1.z, J1.w);
-      const f2 B0 = sb[cb + bp_sk16(4 * tx + R)], B1 = sb[cb + bp_sk16(4 * tx + R + 2)];
-      f2 s0[4] = {0ull, 0ull, 0ull, 0ull}, s1[4] = {0ull, 0ull, 0ull, 0ull};
+    // columns jx0 .. jx0 + 3 of rows jy and jy + 1 (a lane pair each), of which one may be the band's
+    const int jx0 = X0 + 4 * tx, jy = Y0 + 2 * ty;
+    if (jx0 >= band_left(R) && jx0 + 3 < W - R && jy + 1 >= R && jy < H - R) {
+      // skewed position 4 tx + s of a row: base + s + (4 (tx & 1) + s) / 8, and base + s + (4 (tx & 3) + s) / 16
+      const int q1 = tx & 1, b1 = (tx & 3) == 3, b2 = (tx & 3) >= 2, b3 = (tx & 3) >= 1;
+      const auto pq = [&](int v) { return v + (v < 4 ? 0 : v < 8 ? q1 : v < 12 ? 1 : 1 + q1); };
+      const auto pb = [&](int v) { return v + (v < 4 ? 0 : v < 8 ? b1 : v < 12 ? b2 : b3); };
+      const float4 *ce_q = sq + (2 * ty + R) * SQW + 4 * tx + (tx >> 1);
+      const f2 *ce_b = sb + (2 * ty + R) * SBW + 4 * tx + (tx >> 2);
+      f2 U[4], A[4], B[4], s[4][3];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 J = ce_q[pq(R + i)];
+        U[i] = f2_pack(J.x, J.y);
+        A[i] = f2_pack(J.z, J.w);
+        B[i] = ce_b[pb(R + i)];
+        s[i][0] = s[i][1] = s[i][2] = 0ull;
+      }
 #pragma unroll 1
       for (int oy = 0; oy < K; ++oy) {
-        const int row = ty + 2 * R - oy;
-        const float4 *qr = sq + row * SQW;
-        const f2 *br = sb + row * SBW;
+        // neighbours p = j - o: cell row 2 ty + 2R - oy, positions 4 tx + v; column i takes tap ox = 2R + i - v
+        const float4 *qr = ce_q + (R - oy) * SQW;
+        const f2 *br = ce_b + (R - oy) * SBW;
         f2 NL[NLW];
         bp_nl_row(&nl2[oy * NLW], NL);
 #pragma unroll
-        for (int s = 0; s <= 2 * R + 2; ++s) {
-          const int pos = 4 * tx + s;
-          const float4 P = qr[bp_sk8(pos)];
-          const f2 Pu = f2_pack(P.x, P.y), Pa = f2_pack(P.z, P.w), PB = br[bp_sk16(pos)];
-          if (s <= 2 * R) bpk_tap(Pu, Pa, PB, U0, A0, B0, NL[2 * R - s], s0);
-          if (s >= 2) bpk_tap(Pu, Pa, PB, U1, A1, B1, NL[2 * R + 2 - s], s1);
+        for (int v = 0; v <= 2 * R + 3; ++v) {
+          const float4 P = qr[pq(v)];
+          const f2 Pu = f2_pack(P.x, P.y), Pa = f2_pack(P.z, P.w), PB = br[pb(v)];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (v >= i && v <= 2 * R + i) bpk_tap(Pu, Pa, PB, U[i], A[i], B[i], NL[2 * R + i - v], s[i]);
         }
       }
-      if (p.gin) {
-        float *gi = p.gin + (int64_t)b * p.gi_b + (int64_t)jy * p.gi_p + jx0;
-        gi[0] = f2_lo(s0[0]) - BP_C2S * (f2_lo(s0[1]) + f2_lo(s0[2]));
-        gi[1] = f2_hi(s0[0]) - BP_C2S * (f2_hi(s0[1]) + f2_hi(s0[2]));
-        gi[2] = f2_lo(s1[0]) - BP_C2S * (f2_lo(s1[1]) + f2_lo(s1[2]));
-        gi[3] = f2_hi(s1[0]) - BP_C2S * (f2_hi(s1[1]) + f2_hi(s1[2]));
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        if (jy + l < R || jy + l >= H - R) continue;
+        float w = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w += l ? f2_hi(s[i][2]) : f2_lo(s[i][2]);
+        dc = __fmaf_rn(-p.inv_q3, w, dc);
+        if (p.gin) {
+          float *gi = p.gin + (int64_t)b * p.gi_b + (int64_t)(jy + l) * p.gi_p + jx0;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            gi[i] = l ? f2_hi(s[i][0]) - BP_C2S * f2_hi(s[i][1]) : f2_lo(s[i][0]) - BP_C2S * f2_lo(s[i][1]);
+        }
       }
-      dc = __fmaf_rn(-p.inv_q3, (f2_lo(s0[3]) + f2_hi(s0[3])) + (f2_lo(s1[3]) + f2_hi(s1[3])), dc);
     }
   }
   // band pixels of every image: an equal contiguous share per CTA
@@ -460,7 +482,7 @@ __global__ void __launch_bounds__(BA_T) bpk_adjoint_kernel(const __grid_constant
     const int per = band_size(W, H, R);
     int64_t k0, k1;
     cta_share((int64_t)per * p.batch, k0, k1);
-    for (int64_t k = k0 + threadIdx.x; k < k1; k += BA_T) {
+    for (int64_t k = k0 + threadIdx.x; k < k1; k += BPA_T) {
       const int b = (int)(k / per);
       int jy, jx;
       band_pos((int)(k - (int64_t)b * per), W, H, R, jy, jx);
@@ -476,7 +498,7 @@ __global__ void __launch_bounds__(BA_T) bpk_adjoint_kernel(const __grid_constant
   __syncthreads();
   if (threadIdx.x == 0) {
     double sum = 0.0;
-    for (int i = 0; i < BA_T / 32; ++i) sum += s_dc[i];
+    for (int i = 0; i < BPA_T / 32; ++i) sum += s_dc[i];
     p.dc_part[blockIdx.x] = sum;
   }
 }
@@ -494,10 +516,10 @@ int launch_bpk(const BilAdjParams &p0, cudaStream_t st) {
   const size_t smem = BpkShape<K>::smem;
   int rc = ensure_dynamic_smem(kern, smem);
   if (rc) return rc;
-  const int grid = std::max(1, std::min(p.ntiles, num_sms() * resident_ctas(kern, BA_T, smem)));
+  const int grid = std::max(1, std::min(p.ntiles, num_sms() * resident_ctas(kern, BPA_T, smem)));
   cudaEvent_t ev = before_launch(st);
   bpk_forward_kernel<K><<<fgrid, BA_T, 0, st>>>(p);
-  bpk_adjoint_kernel<K><<<grid, BA_T, smem, st>>>(p);
+  bpk_adjoint_kernel<K><<<grid, BPA_T, smem, st>>>(p);
   if (p.grad_sigma) bil_adjoint_combine_kernel<<<1, BA_T, 0, st>>>(p, grid);
   return after_launch("bpk_adjoint_kernel", st, ev);
 }
