@@ -22,14 +22,10 @@
 // of an FP32 tile, so more CTAs per SM); cells outside the image, which TMA
 // fills with zeros, are patched with the boundary rule (a CONSTANT cell holds
 // the constant in the storage type).  Other layouts stage an FP32 tile with
-// 16-byte global loads, in an instantiation of their own (f32 1023 x 767, 9 taps: 8.5
-// us with both stagings in one kernel, 7.2 us now).  Both passes run packed f32x2 fused
-// multiply-adds on pairs of adjacent outputs, keeping each output's tap order.
-// 16-bit tiles take eight outputs per lane in the row pass (row_pass8); for FP32
-// ones, whose lanes would read 32 bytes apart, four remain.  bf16, four outputs
-// per lane against eight: 13 taps 4 x 1920 x 1080 22.3 against 19.0 us, 9 taps
-// 8192 x 8192 97.3 against 96.0 us: there the chain of tile load, row pass and
-// column pass, with a barrier between each, bounds a tile more than their instructions.
+// 16-byte global loads.  Both passes run packed f32x2 fused multiply-adds on
+// pairs of adjacent outputs, keeping each output's tap order.  With few taps the chain
+// of tile load, row pass and column pass, with a barrier between each, bounds a
+// tile more than their instructions.
 #include <algorithm>
 #include <type_traits>
 
@@ -40,6 +36,11 @@ namespace hgb {
 namespace {
 
 constexpr int kSepMaxK = 15;
+// 16-bit tiles staged by TMA take row_pass8 from 11 taps on.  bf16, four outputs per lane
+// against eight: 15 taps 2 x 1920 x 1080 14.3 / 12.8 us, 13 taps 4 x 1920 x 1080 20.5 /
+// 18.5, 11 taps 19.8 / 17.4; but 9 taps 8192 x 8192 93.8 / 95.7, 3 taps (f16) 8 x 1024 x
+// 1024 9.8 / 10.2: with few taps the wider window's loads and conversions weigh more.
+constexpr int kSepWideK = 11;
 
 struct SepParams {
   CUtensorMap map;  // storage-type tensor map of the input when use_tma
@@ -174,7 +175,7 @@ __device__ __forceinline__ void row_pass8(const SepParams &p, const TT *tile, fl
   }
 }
 
-template <typename T, int K, bool TMA>
+template <typename T, int K, bool WIDE>
 __global__ void __launch_bounds__(SP_BX *SP_BY) separable_kernel(const __grid_constant__ SepParams p) {
   using S = SepShape<T, K>;
   constexpr int R = S::R, HL = S::HL, SW = S::SW, SH = S::SH;
@@ -187,10 +188,9 @@ __global__ void __launch_bounds__(SP_BX *SP_BY) separable_kernel(const __grid_co
   const int X0 = i0 - HL, Y0 = j0 - R;
   const char *img = p.in + (int64_t)b * p.in_bstride;
   const int tx = threadIdx.x % SP_BX, ty = threadIdx.x / SP_BX;
-  constexpr bool kWide = TMA && sizeof(T) == 2;  // row_pass8, with its layout of the row buffer
-  static_assert(!kWide || (HL == 8 && SW == SP_TW + 16), "a lane's window is 24 cells from 8 l");
+  static_assert(!WIDE || (HL == 8 && SW == SP_TW + 16), "a lane's window is 24 cells from 8 l");
   float *rowb;
-  if constexpr (TMA) {
+  if (WIDE || p.use_tma) {
     // the tile stays in the storage type; the row pass widens as it reads
     T *tile = reinterpret_cast<T *>(base);
     rowb = reinterpret_cast<float *>(base + S::tile_tma);
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(SP_BX *SP_BY) separable_kernel(const __grid_co
       }
     }
     __syncthreads();
-    if constexpr (kWide)
+    if constexpr (WIDE)
       row_pass8<T, K, SW, SH>(p, tile, rowb, j0);
     else
       row_pass<T, K, SW, SH, HL>(p, tile, rowb, j0, tx, ty);
@@ -254,7 +254,6 @@ __global__ void __launch_bounds__(SP_BX *SP_BY) separable_kernel(const __grid_co
   }
   __syncthreads();
   // ---- column pass: 4 x 4 outputs per thread
-  const float *colb = rowb + ty * SP_PY * SP_TW + 4 * (kWide ? sep_unit(tx) : tx);
   f2 c2[SP_PY][SP_PX / 2];
 #pragma unroll
   for (int oy = 0; oy < SP_PY; ++oy)
@@ -262,7 +261,8 @@ __global__ void __launch_bounds__(SP_BX *SP_BY) separable_kernel(const __grid_co
     for (int pp = 0; pp < SP_PX / 2; ++pp) c2[oy][pp] = 0ull;
 #pragma unroll
   for (int r = 0; r < SP_PY + K - 1; ++r) {
-    const float4 t = *reinterpret_cast<const float4 *>(colb + r * SP_TW);
+    const float4 t = *reinterpret_cast<const float4 *>(
+        &rowb[(ty * SP_PY + r) * SP_TW + (WIDE ? 4 * sep_unit(tx) : tx * SP_PX)]);
     const f2 v01 = f2_pack(t.x, t.y), v23 = f2_pack(t.z, t.w);
 #pragma unroll
     for (int oy = 0; oy < SP_PY; ++oy) {
@@ -309,7 +309,10 @@ int launch_sep_k(const SepParams &p0, int batch, cudaStream_t st) {
     p.status = device_status_word();
   }
   const size_t smem = p.use_tma ? S::smem_tma : S::smem_ldg;
-  const auto kern = p.use_tma ? separable_kernel<T, K, true> : separable_kernel<T, K, false>;
+  auto kern = separable_kernel<T, K, false>;
+  if constexpr (sizeof(T) == 2 && K >= kSepWideK) {
+    if (p.use_tma) kern = separable_kernel<T, K, true>;
+  }
   const int rc = ensure_dynamic_smem((const void *)kern, smem);
   if (rc) return rc;
   dim3 grid(cdiv(p.w, SP_TW), cdiv(p.h, SP_TH), batch);
