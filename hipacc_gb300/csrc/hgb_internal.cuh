@@ -33,6 +33,22 @@ int after_launch(const char *kernel, cudaStream_t stream, cudaEvent_t start);
 // returns a started event when timing is on (else nullptr)
 cudaEvent_t before_launch(cudaStream_t stream);
 
+// While it lives, this thread may allocate although a stream of the process is being
+// captured (a capture in the default mode refuses that and is lost).
+class RelaxedCapture {
+ public:
+  RelaxedCapture() { on_ = cudaThreadExchangeStreamCaptureMode(&mode_) == cudaSuccess; }
+  ~RelaxedCapture() {
+    if (on_) cudaThreadExchangeStreamCaptureMode(&mode_);
+  }
+  RelaxedCapture(const RelaxedCapture &) = delete;
+  RelaxedCapture &operator=(const RelaxedCapture &) = delete;
+
+ private:
+  cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+  bool on_ = false;
+};
+
 // ---------------------------------------------------------------- workspace
 // Per-device scratch owned by the library: reduction partials, tickets,
 // work-lists.  The ticket region is zeroed once at allocation and every

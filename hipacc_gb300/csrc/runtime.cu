@@ -80,12 +80,21 @@ int workspace_get(size_t bytes, Workspace *ws) {
   std::lock_guard<std::mutex> lk(g_mu);
   DeviceState &st = dev_state(dev);
   if (!st.ws.tickets) {
-    // accumulators first (8-byte aligned), tickets behind them
+    // accumulators first (8-byte aligned), tickets behind them.  The device's first
+    // call may be under stream capture: nothing here touches a captured stream.
+    const RelaxedCapture relaxed;
     void *t = nullptr;
     const size_t nb = kAcc * sizeof(unsigned long long) + kTickets * sizeof(unsigned int);
-    HGB_CHECK_CUDA(cudaMalloc(&t, nb));
-    HGB_CHECK_CUDA(cudaMemset(t, 0, nb));
-    HGB_CHECK_CUDA(cudaDeviceSynchronize());
+    cudaStream_t own = nullptr;
+    HGB_CHECK_CUDA(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+    cudaError_t e = cudaMalloc(&t, nb);
+    if (e == cudaSuccess) e = cudaMemsetAsync(t, 0, nb, own);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(own);
+    cudaStreamDestroy(own);
+    if (e != cudaSuccess) {
+      cudaFree(t);
+      return cuda_error(e, "workspace_get");
+    }
     st.ws.acc = (unsigned long long *)t;
     st.ws.tickets = (unsigned int *)((char *)t + kAcc * sizeof(unsigned long long));
   }
