@@ -170,8 +170,8 @@ int check_view(const hgb_view *v, const char *name) {
     return set_error(HGB_ERR_INVALID, std::string(name) + ": pitch smaller than a row");
   if (v->batch > 1 && v->batch_stride < v->pitch * v->height)
     return set_error(HGB_ERR_INVALID, std::string(name) + ": batch_stride smaller than an image");
-  if (((uintptr_t)v->data) % es != 0 || v->pitch % es != 0)
-    return set_error(HGB_ERR_INVALID, std::string(name) + ": misaligned data or pitch");
+  if (((uintptr_t)v->data) % es != 0 || v->pitch % es != 0 || (v->batch > 1 && v->batch_stride % es != 0))
+    return set_error(HGB_ERR_INVALID, std::string(name) + ": misaligned data, pitch or batch stride");
   return HGB_OK;
 }
 

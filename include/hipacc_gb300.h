@@ -83,6 +83,7 @@ typedef struct hgb_view {
   int32_t batch;        /* images, >= 1 */
   int64_t pitch;        /* bytes between rows */
   int64_t batch_stride; /* bytes between images (ignored when batch == 1) */
+                        /* data, pitch and batch_stride: whole elements */
 } hgb_view;
 
 /* Accessor window / IterationSpace ROI (HipaccAccessorBase,
