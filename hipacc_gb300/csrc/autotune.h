@@ -7,7 +7,7 @@
 // size class) key with autotuning on times every configuration with CUDA
 // events and keeps the fastest.  Choices can be saved to and loaded from a
 // JSON file.  While a stream is being captured nothing is timed: the stored
-// choice (or configuration 0) is used.
+// choice (or the operator's untuned configuration) is used.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -23,17 +23,18 @@ void autotune_store(const char *key, int cfg, float ms);
 // Nothing to look up and nothing to tune: callers skip building their key.
 bool autotune_idle();
 
+// `untuned`: the configuration of a key without a choice while tuning is off
 template <typename F>
-int autotune_run(const char *key, int ncfg, cudaStream_t st, F &&launch) {
+int autotune_run(const char *key, int ncfg, cudaStream_t st, F &&launch, int untuned = 0) {
   int cfg = autotune_lookup(key);
   if (cfg >= 0 && cfg < ncfg) return launch(cfg);
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   cudaStreamIsCapturing(st, &cs);
-  if (!autotune_enabled() || ncfg <= 1 || cs != cudaStreamCaptureStatusNone) return launch(0);
+  if (!autotune_enabled() || ncfg <= 1 || cs != cudaStreamCaptureStatusNone) return launch(untuned);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  int best = 0;
+  int best = untuned;
   float best_ms = 3.0e38f;
   for (int c = 0; c < ncfg; ++c) {
     int rc = launch(c);  // warm-up, also surfaces launch errors

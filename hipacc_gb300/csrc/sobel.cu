@@ -135,20 +135,21 @@ struct SobelTmaParams {
   unsigned int *claim;      // tile counter of the streaming form, zero at rest
 };
 
-// The tile is 128 x 128 outputs in every configuration.  The autotuner picks
-// the rows per warp (32 rows for 4 warps, or 16 rows for 8 warps: a shorter
-// serial stencil per warp after the tile lands, twice the warps per SM) and the
-// launch form:
+// The tile is 128 x 128 outputs, or 128 x 32 in the last configuration
+// (kSobelLow: one CTA of four warps per tile, for small images).  Of the tall
+// tiles the autotuner picks the rows per warp (32 rows for 4 warps, or 16 rows
+// for 8 warps: a shorter serial stencil per warp after the tile lands, twice the
+// warps per SM) and the launch form:
 //   one-shot (kSobelStream 0): one CTA per tile, every tile's copy issued at
 //     launch;
 //   streaming (kSobelStream = CTAs per SM): a few CTAs per SM claim tiles from
 //     a counter, each with two stage buffers, so that the next tile's copy
 //     lands while the current one is computed.  Tiles go to the CTAs that are
 //     free, and the SMs keep room for an independent kernel of the same step.
-constexpr int T_TW = 128, T_TH = 128;
+constexpr int T_TW = 128, T_TH = 128, T_LOW = 32;
 constexpr int kSobelWarps[] = {4, 8, 4, 4, 8};
 constexpr int kSobelStream[] = {0, 0, 2, 3, 2};
-constexpr int kSobelCfgs = 5;
+constexpr int kSobelLow = 5, kSobelCfgs = 6;
 constexpr int T_SW = 160, T_SH = T_TH + 2, T_STAGE = T_SW * T_SH;
 constexpr int T_STAGE_PAD = (T_STAGE + 127) / 128 * 128;
 
@@ -552,21 +553,32 @@ extern "C" int hgb_sobel_mag(const hgb_view *in, const hgb_view *out, const int 
     P.claim = ws.tickets + kTicketSobelClaim;
     // 128 x 32 tiles where the taller ones would not give every SM four CTAs:
     // the time of a small image is one CTA's chain of rows (640 x 480 with its
-    // gray: 14.5 -> 6.0 us)
+    // gray: 14.5 -> 6.0 us).  A tuned or loaded choice goes before this rule.
     const bool low = P.ntiles < 4 * num_sms();
-    if (low) {
-      P.tiles_y = cdiv(p.h, 32);
+    int rows = 0;
+    auto set_rows = [&](int r) {
+      P.tiles_y = cdiv(p.h, r);
       P.ntiles = P.tiles_x * P.tiles_y * in->batch;
-    }
+      rows = r;
+    };
+    auto map_rows = [&](int r) {
+      set_rows(r);
+      return make_tensor_map_3d(&P.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, in->data, p.w, p.h, in->batch, in->pitch,
+                                in->batch_stride, T_SW, r + 2);
+    };
     if (tma_legal(in->data, in->pitch, in->batch_stride, in->batch) &&
-        make_tensor_map_3d(&P.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, in->data, p.w, p.h, in->batch, in->pitch,
-                           in->batch_stride, T_SW, low ? 34 : T_SH) == HGB_OK) {
-      if (low) {
-        cudaEvent_t ev = before_launch(st);
-        sobel3_tile_kernel<4, 32, true><<<P.ntiles, 128, 0, st>>>(P);
-        return after_launch("sobel3_tile_kernel", st, ev);
-      }
+        map_rows(low ? T_LOW : T_TH) == HGB_OK) {
       auto launch = [&](int cfg) {
+        const int want = cfg == kSobelLow ? T_LOW : T_TH;
+        if (rows != want) {
+          const int e = map_rows(want);
+          if (e) return e;
+        }
+        if (cfg == kSobelLow) {
+          cudaEvent_t ev = before_launch(st);
+          sobel3_tile_kernel<4, T_LOW, true><<<P.ntiles, 128, 0, st>>>(P);
+          return after_launch("sobel3_tile_kernel", st, ev);
+        }
         const int per_sm = kSobelStream[cfg], warps = kSobelWarps[cfg];
         if (per_sm > 0) {
           const void *fn = warps == 8 ? (const void *)sobel3_stream_kernel<8> : (const void *)sobel3_stream_kernel<4>;
@@ -586,15 +598,17 @@ extern "C" int hgb_sobel_mag(const hgb_view *in, const hgb_view *out, const int 
           sobel3_tile_kernel<4, T_TH, true><<<P.ntiles, 128, 0, st>>>(P);
         return after_launch("sobel3_tile_kernel", st, ev);
       };
-      if (autotune_idle()) return launch(0);
+      const int untuned = low ? kSobelLow : 0;
+      if (autotune_idle()) return launch(untuned);
       char key[96];
       snprintf(key, sizeof(key), "sobel3:%dx%dx%d", 1 << (32 - __builtin_clz((unsigned)p.w)),
                1 << (32 - __builtin_clz((unsigned)p.h)), in->batch);
-      return autotune_run(key, kSobelCfgs, st, launch);
+      return autotune_run(key, kSobelCfgs, st, launch, untuned);
     }
+    set_rows(low ? T_LOW : T_TH);
     cudaEvent_t ev = before_launch(st);
     if (low)
-      sobel3_tile_kernel<4, 32, false><<<P.ntiles, 128, 0, st>>>(P);
+      sobel3_tile_kernel<4, T_LOW, false><<<P.ntiles, 128, 0, st>>>(P);
     else
       sobel3_tile_kernel<4, T_TH, false><<<P.ntiles, 128, 0, st>>>(P);
     return after_launch("sobel3_tile_kernel", st, ev);
