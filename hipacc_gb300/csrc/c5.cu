@@ -1179,7 +1179,7 @@ extern "C" int hgb_conv_bilateral_mse(const hgb_view *x, const hgb_view *t, cons
   const int nchunks = cdiv(ftiles, chunk);
   // dL/dc has a partial per chunk and one per CTA for its share of the band
   const size_t nparts =
-      std::max(std::max(nblk, (size_t)B * red_rows), std::max((size_t)cgrid, (size_t)nchunks + std::min(nchunks, fgrid)));
+      std::max(std::max(nblk, (size_t)B * red_rows), std::max(2 * (size_t)cgrid, (size_t)nchunks + std::min(nchunks, fgrid)));
   // workspace: the fused form's packed float4 per pixel (or the unfused
   // form's y1, y, a), then dy1, then the partials
   const size_t img_bytes = (size_t)ib * B * 4;
@@ -1267,12 +1267,12 @@ extern "C" int hgb_conv_bilateral_mse(const hgb_view *x, const hgb_view *t, cons
       c.batch = B;
       c.bmode = boundary;
       c.mask_dev = mask_dev;
-      c.part = p.dm_part;
+      c.part = (double *)(parts + (nparts * 12 + 7) / 8 * 8);  // in dm_part's place: 2 cgrid <= nparts
       rc = run_conv_adjoint(C5_MK, &c, cgrid, st);
       if (rc) return rc;
       LineCombine lc;
       memset(&lc, 0, sizeof(lc));
-      lc.part[0] = p.dm_part;
+      lc.part[0] = c.part;
       lc.out[0] = grad_mask_dev;
       lc.taps[0] = C5_MK * C5_MK;
       lc.nparts[0] = cgrid;

@@ -11,7 +11,7 @@
 // thread keeps 4 x 4 (4 x 1) pixels.  grad_in: each staged row is read once and
 // serves all the thread's rows, two pixels per packed f32x2 operation.  grad_m: a
 // row of in, the same way, against the thread's grad_out, two taps per packed
-// operation, in registers that live across the CTA's tiles.  The next tile is
+// operation; a tile's sums join the warp's compensated ones (tap_fold.cuh).  The next tile is
 // staged (asynchronous copies) while this one computes.  Any row alignment.
 //
 // Bound by load latency and issue at 16 to 24 warps per SM (the mask gradient's
@@ -25,6 +25,7 @@
 #include "band.cuh"
 #include "conv_adjoint.h"
 #include "stage_groups.cuh"
+#include "tap_fold.cuh"
 
 namespace hgb {
 namespace {
@@ -107,19 +108,15 @@ __global__ void __launch_bounds__(CA_NT, K == 3 ? 6 : (K == 5 ? 5 : 4)) conv_adj
   extern __shared__ __align__(16) float ca_stage[];  // two buffers of [grad_out][in]: the next tile lands meanwhile
   __shared__ __align__(16) f2 m2[K][2 * NP];  // mask pairs (m, m), an even count per row
   __shared__ float msk[K * K];
-  __shared__ float red[CA_NT / 32][K * K];
+  __shared__ TapSum sum[CA_NT / 32][K * K];  // mask gradient of each warp's pixels
   for (int i = threadIdx.x; i < K * 2 * NP; i += CA_NT) {
     const int y = i / (2 * NP), x = i - y * (2 * NP);
     const float m = x < K ? (p.mask_dev ? __ldg(p.mask_dev + y * K + x) : p.mask[y * K + x]) : 0.0f;
     m2[y][x] = f2_pack(m, m);
     if (x < K) msk[y * K + x] = m;
   }
+  for (int i = threadIdx.x; i < CA_NT / 32 * K * K; i += CA_NT) (&sum[0][0])[i] = TapSum{0.0f, 0.0f};
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  f2 DM[K][NP];  // mask gradient per pair of taps (my, 2 op), (my, 2 op + 1)
-#pragma unroll
-  for (int i = 0; i < K; ++i)
-#pragma unroll
-    for (int j = 0; j < NP; ++j) DM[i][j] = 0ull;
   auto origin = [&](int t, int &b, int &i0, int &j0) {
     const int per = p.tiles_x * p.tiles_y;
     b = t / per;
@@ -203,7 +200,12 @@ __global__ void __launch_bounds__(CA_NT, K == 3 ? 6 : (K == 5 ? 5 : 4)) conv_adj
         }
       }
     }
-    if (p.part && x < p.w && y0 < p.h) {
+    if (p.part) {
+      f2 DM[K][NP];  // mask gradient per pair of taps (my, 2 op), (my, 2 op + 1)
+#pragma unroll
+      for (int i = 0; i < K; ++i)
+#pragma unroll
+        for (int j = 0; j < NP; ++j) DM[i][j] = 0ull;
       if (x + 4 <= p.w && y0 + PY <= p.h) {
         f2 GG[PY][4];
 #pragma unroll
@@ -231,7 +233,7 @@ __global__ void __launch_bounds__(CA_NT, K == 3 ? 6 : (K == 5 ? 5 : 4)) conv_adj
               }
           }
         }
-      } else {  // groups that leave the image: only the pixels inside
+      } else if (x < p.w) {  // groups that leave the image: only the pixels inside
 #pragma unroll 1
         for (int oy = 0; oy < PY && y0 + oy < p.h; ++oy)
 #pragma unroll 1
@@ -248,25 +250,19 @@ __global__ void __launch_bounds__(CA_NT, K == 3 ? 6 : (K == 5 ? 5 : 4)) conv_adj
                                     DM[my][op]);
           }
       }
+      float dm[K * K];
+#pragma unroll
+      for (int o = 0; o < K * K; ++o) {
+        const f2 v = DM[o / K][o % K >> 1];
+        dm[o] = (o % K & 1) ? f2_hi(v) : f2_lo(v);
+      }
+      fold_taps(dm, sum[threadIdx.x >> 5], 0, K * K);
     }
     __syncthreads();  // this buffer is read before the tile after the next is staged into it
   }
   if (!p.part) return;
-#pragma unroll
-  for (int my = 0; my < K; ++my)
-#pragma unroll
-    for (int mx = 0; mx < K; ++mx) {
-      float v = (mx & 1) ? f2_hi(DM[my][mx >> 1]) : f2_lo(DM[my][mx >> 1]);
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][my * K + mx] = v;
-    }
   __syncthreads();
-  for (int o = threadIdx.x; o < K * K; o += CA_NT) {
-    float v = 0.0f;
-    for (int w = 0; w < CA_NT / 32; ++w) v += red[w][o];
-    p.part[(size_t)o * gridDim.x + blockIdx.x] = v;
-  }
+  for (int o = threadIdx.x; o < K * K; o += CA_NT) p.part[(size_t)o * gridDim.x + blockIdx.x] = tap_total(sum, o);
 }
 
 using ConvAdjKernel = void (*)(ConvAdjParams);

@@ -14,7 +14,7 @@ struct ConvAdjParams {
   int tiles_x, tiles_y, ntiles;
   const float *mask_dev;                             // K x K taps on the device, or null
   float mask[49];
-  float *part;                                       // [taps][CTAs] partials of the mask gradient, or null
+  double *part;                                      // [taps][CTAs] partials of the mask gradient, or null
 };
 
 bool conv_adjoint_size(int k);  // 3, 5 or 7

@@ -17,7 +17,7 @@ __global__ void __launch_bounds__(256) line_combine_kernel(const __grid_constant
     a = 1;
   }
   double s = 0.0;
-  for (int k = threadIdx.x; k < c.nparts[a]; k += 256) s += (double)__ldcg(c.part[a] + (size_t)o * c.nparts[a] + k);
+  for (int k = threadIdx.x; k < c.nparts[a]; k += 256) s += __ldcg(c.part[a] + (size_t)o * c.nparts[a] + k);
   sh[threadIdx.x] = s;
   __syncthreads();
   for (int d = 128; d > 0; d >>= 1) {

@@ -15,7 +15,7 @@ struct LineAdjParams {
   float mask[15];
   float cval;
   float row[15];                                     // row taps that recompute t (column form of the separable filter)
-  float *part;                                       // [taps][CTAs] partials of the tap gradient, or null
+  double *part;                                      // [taps][CTAs] partials of the tap gradient, or null
 };
 
 enum LineForm { kLineRow = 0, kLineCol = 1, kLineColOfRows = 2 };
@@ -31,7 +31,7 @@ template <int K>
 LineKernel line_kernel_k(LineForm f, bool dev, int py);  // line_k*.cu; py rows per thread, 4 or 1
 
 struct LineCombine {  // up to two tap gradients, summed in FP64 in a fixed order
-  const float *part[2];
+  const double *part[2];
   float *out[2];
   int taps[2], nparts[2];
 };

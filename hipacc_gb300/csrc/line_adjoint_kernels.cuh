@@ -11,7 +11,8 @@
 // One pass: a CTA walks 64 x 32 tiles (64 x 8 on small batches), stages grad_out (zero outside the image)
 // and in (through the boundary) with the halo of one axis, and a thread keeps
 // 4 x 4 (4 x 1) pixels: grad_in from register windows, the tap gradient in one packed
-// f32x2 accumulator per tap that lives across the CTA's tiles.  The general
+// f32x2 accumulator per tap, which joins the warp's compensated sums after each tile
+// (tap_fold.cuh).  The general
 // kernels (local_adjoint.cu) read every tap from global memory and walk the
 // images once per tap.  In the column form of a separable filter the row pass
 // t = rows(in) is recomputed in shared memory (the forward's operations and
@@ -25,6 +26,7 @@
 #include "band.cuh"
 #include "line_adjoint.h"
 #include "stage_groups.cuh"
+#include "tap_fold.cuh"
 
 namespace hgb {
 
@@ -57,16 +59,14 @@ __global__ void __launch_bounds__(LN_NT) line_adjoint_kernel(const __grid_consta
   __shared__ __align__(16) float si[SH * SWI];
   __shared__ __align__(16) float st[kT ? SH * LN_TW : 4];
   __shared__ float sm[DEV ? K : 1];
-  __shared__ float red[LN_NT / 32][K];
+  __shared__ TapSum sum[LN_NT / 32][K];  // tap gradient of each warp's pixels
   if (DEV) {
     if (threadIdx.x < K) sm[threadIdx.x] = __ldg(p.mask_dev + threadIdx.x);
     __syncthreads();
   }
   auto tap = [&](int k) { return DEV ? sm[k] : p.mask[k]; };
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  f2 gm[K];  // tap gradients: even and odd pixels of the pairs
-#pragma unroll
-  for (int k = 0; k < K; ++k) gm[k] = 0ull;
+  if (threadIdx.x < LN_NT / 32 * K) (&sum[0][0])[threadIdx.x] = TapSum{0.0f, 0.0f};
   for (int t = blockIdx.x; t < p.ntiles; t += gridDim.x) {
     const int per = p.tiles_x * p.tiles_y, b = t / per, rt = t - b * per, by = rt / p.tiles_x;
     const int i0 = (rt - by * p.tiles_x) * LN_TW, j0 = by * LN_TH;
@@ -151,8 +151,13 @@ __global__ void __launch_bounds__(LN_NT) line_adjoint_kernel(const __grid_consta
           }
         }
       }
-      // ---- tap gradient
-      if (p.part) {
+    }
+    // ---- tap gradient
+    if (p.part) {
+      f2 gm[K];  // even and odd pixels of the pairs
+#pragma unroll
+      for (int k = 0; k < K; ++k) gm[k] = 0ull;
+      if (x < p.w && y0 < p.h) {
         if (x + 4 <= p.w && y0 + LN_PY <= p.h) {
           f2 g0[LN_PY], g1[LN_PY];
 #pragma unroll
@@ -204,6 +209,10 @@ __global__ void __launch_bounds__(LN_NT) line_adjoint_kernel(const __grid_consta
             }
         }
       }
+      float v[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[k] = f2_lo(gm[k]) + f2_hi(gm[k]);
+      fold_taps(v, sum[threadIdx.x >> 5], 0, K);
     }
     // ---- near a border: a pixel with other pre-images sums over all of them, a
     // band pixel per thread, only the taps that reach back into the image.  On
@@ -245,19 +254,8 @@ __global__ void __launch_bounds__(LN_NT) line_adjoint_kernel(const __grid_consta
     __syncthreads();  // the tile is read before the next one is staged
   }
   if (!p.part) return;
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    float v = f2_lo(gm[k]) + f2_hi(gm[k]);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < K) {
-    float v = 0.0f;
-    for (int w = 0; w < LN_NT / 32; ++w) v += red[w][threadIdx.x];
-    p.part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = v;
-  }
+  // the tiles end with a barrier
+  if (threadIdx.x < K) p.part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = tap_total(sum, threadIdx.x);
 }
 
 template <int K, int PY>

@@ -453,9 +453,9 @@ extern "C" int hgb_local_op_adjoint(const hgb_view *in, const hgb_view *grad_out
     memset(&c, 0, sizeof(c));
     if (grad_mask_dev) {
       Workspace ws;
-      rc = workspace_get((size_t)n * grid * sizeof(float) + 64, &ws);
+      rc = workspace_get((size_t)n * grid * sizeof(double) + 64, &ws);
       if (rc) return rc;
-      l.part = (float *)ws.base;
+      l.part = (double *)ws.base;
       c.part[0] = l.part;
       c.out[0] = grad_mask_dev;
       c.taps[0] = n;
@@ -538,9 +538,9 @@ extern "C" int hgb_local_op_adjoint(const hgb_view *in, const hgb_view *grad_out
     memset(&lc, 0, sizeof(lc));
     if (grad_mask_dev) {
       Workspace ws;
-      rc = workspace_get((size_t)K * K * grid * sizeof(float) + 64, &ws);
+      rc = workspace_get((size_t)K * K * grid * sizeof(double) + 64, &ws);
       if (rc) return rc;
-      c.part = (float *)ws.base;
+      c.part = (double *)ws.base;
       lc.part[0] = c.part;
       lc.out[0] = grad_mask_dev;
       lc.taps[0] = K * K;

@@ -42,9 +42,10 @@ int separable_adjoint_tiles(const hgb_view *in, const hgb_view *grad_out, const 
   const int64_t gt_p = ((int64_t)p.w + 3) / 4 * 16, gt_b = gt_p * p.h;
   const size_t gt_bytes = want_gt ? (size_t)gt_b * p.batch : 0;
   Workspace ws;
-  int rc = workspace_get(gt_bytes + (size_t)k * (g1 + g2) * sizeof(float) + 64, &ws);
+  int rc = workspace_get(gt_bytes + (size_t)k * (g1 + g2) * sizeof(double) + 64, &ws);
   if (rc) return rc;
-  float *gt = (float *)ws.base, *part1 = (float *)((char *)ws.base + gt_bytes), *part2 = part1 + (size_t)k * g1;
+  float *gt = (float *)ws.base;
+  double *part1 = (double *)((char *)ws.base + gt_bytes), *part2 = part1 + (size_t)k * g1;
   LineCombine c;
   memset(&c, 0, sizeof(c));
   int n = 0;
