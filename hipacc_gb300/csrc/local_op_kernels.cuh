@@ -25,18 +25,24 @@ int launch_cfg(const ConvParams &p0, int batch, cudaStream_t st) {
                                         : std::is_same<TI, uint8_t>::value ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                                         : std::is_same<TI, __half>::value  ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                                            : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  // The TMA form is the faster one up to 11 x 11 taps, of 16-bit storage up to 7 x 7
-  // (4 images of 1280 x 872: 3 x 3 f32 10.0 -> 6.8 us without the overhang's patch,
-  // bf16 9.6 -> 8.6 us; 11 x 11 bf16 33.8 us by TMA, 33.0 us by groups; 13 x 13 f32
-  // 61 us by TMA, 40 us by groups, whose kernel leaves the stencil more registers)
-  if (MW * MH < (sizeof(TI) == 2 ? 81 : 169) && p.acc_ox == 0 && p.acc_oy == 0 && p.acc_w == p.in_w && p.acc_h == p.in_h &&
-      tma_legal(p.in, p.in_pitch, p.in_bstride, batch) &&
-      make_tensor_map_3d(&p.map, kType, (int)sizeof(TI), p.in, p.in_w, p.in_h, batch, p.in_pitch, p.in_bstride, SW,
-                         SH) == HGB_OK) {
-    p.status = device_status_word();
-    cudaEvent_t ev = before_launch(st);
-    conv_kernel<TI, TO, MW, MH, BX, BY, PX, PY, true><<<grid, BX * BY, 0, st>>>(p);
-    return after_launch("conv_kernel", st, ev);
+  // The TMA form is the faster one up to 11 x 11 taps.  13 x 13 goes by groups, whose
+  // kernel leaves the stencil more registers (TMA / groups, 4096 x 4096: f32 176 / 127,
+  // bf16 176 / 134, u8 173 / 133 us; 4 x 1280 x 872 63 / 42, 59 / 43, 59 / 42 us).  16-bit
+  // masks of 9 x 9 and 11 x 11 take TMA where every SM has four tiles: bf16 9 x 9 64.7 /
+  // 70.7 us on 4096 x 4096, 132 / 142 on 32 x 1024 x 1024, 23.1 / 24.7 on 16 x 512 x 512, but
+  // 14.6 / 14.1 on 1920 x 1080 and 8.7 / 8.0 on 640 x 480; 11 x 11 110 / 113, 230 / 241, 35.6 /
+  // 37.2, 22.7 / 23.4 and 10.6 / 10.6.
+  if constexpr (MW * MH < 169) {
+    const bool enough = sizeof(TI) != 2 || MW * MH < 81 || (int64_t)grid.x * grid.y * grid.z >= 4 * num_sms();
+    if (enough && p.acc_ox == 0 && p.acc_oy == 0 && p.acc_w == p.in_w && p.acc_h == p.in_h &&
+        tma_legal(p.in, p.in_pitch, p.in_bstride, batch) &&
+        make_tensor_map_3d(&p.map, kType, (int)sizeof(TI), p.in, p.in_w, p.in_h, batch, p.in_pitch, p.in_bstride, SW,
+                           SH) == HGB_OK) {
+      p.status = device_status_word();
+      cudaEvent_t ev = before_launch(st);
+      conv_kernel<TI, TO, MW, MH, BX, BY, PX, PY, true><<<grid, BX * BY, 0, st>>>(p);
+      return after_launch("conv_kernel", st, ev);
+    }
   }
   cudaEvent_t ev = before_launch(st);
   conv_kernel<TI, TO, MW, MH, BX, BY, PX, PY, false><<<grid, BX * BY, 0, st>>>(p);
