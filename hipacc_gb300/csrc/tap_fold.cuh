@@ -75,12 +75,13 @@ __device__ __forceinline__ void fold_taps(const T (&v)[N], TapSum *sum, int base
   }
 }
 
-// sum of a tap over the CTA's warps
+// sum of a tap over the CTA's warps (FP64 only at the end: its additions take long)
 template <int W, int N>
 __device__ __forceinline__ double tap_total(const TapSum (&sum)[W][N], int tap) {
-  double v = 0.0;
-  for (int w = 0; w < W; ++w) v += (double)sum[w][tap].s + (double)sum[w][tap].c;
-  return v;
+  TapSum v = sum[0][tap];
+#pragma unroll
+  for (int w = 1; w < W; ++w) v = tap_add(v, sum[w][tap]);
+  return (double)v.s + (double)v.c;
 }
 
 }  // namespace hgb
