@@ -468,14 +468,18 @@ extern "C" int hgb_local_op_adjoint(const hgb_view *in, const hgb_view *grad_out
     return after_launch("line_adjoint", st, ev);
   }
   // Both gradients of a 3 x 3, 5 x 5 or 7 x 7 mask: the fused kernel where TMA can
-  // address both images and 64 x 32 tiles would give every SM four CTAs (8 images
-  // of 1024 x 1024, MIRROR: 41 / 66 / 96 us for the three masks against 49 / 67 /
-  // 123 us tiled); the tiled kernel of conv_adjoint.cu elsewhere (2 images of 2049 x
-  // 2051: 46 / 66 / 99 us against 89 / 130 / 224 us for the pair of kernels that
-  // took other layouts; one image of 200 x 160: 4.6 / - / 6.8 us against 20 us and
-  // more) and for one gradient alone (7 x 7 on 4096 x 2048: 48 us against 95 and 114 us).
+  // address both images and there are enough 64 x 32 tiles, three for every two SMs (3 x 3)
+  // or four per SM; else the tiled kernel of conv_adjoint.cu.  Fused / tiled, MIRROR, for
+  // the three masks: 8 images of 1024 x 1024 (4096 tiles) 41.5 / 50.7, 65.6 / 66.3, 95.9 /
+  // 118.6 us; 1024 x 1024 (512) 12.4 / 16.1, 18.7 / 18.7, 24.6 / 24.7; 1280 x 720 (460) 12.0 /
+  // 14.4, 17.4 / 17.7, 23.9 / 21.1; 300 of 64 x 64 (600) 19.0 / 20.8, 34.6 / 31.0, 54.0 / 47.3;
+  // 768 x 768 (288) 11.1 / 13.2, 16.1 / 14.3, 21.0 / 17.5; 640 x 480 (150) 9.9 / 9.9, 15.3 /
+  // 11.2, 18.8 / 12.7.  Layouts off TMA always take the tiled one (2 images of 2049 x 2051:
+  // 45 / 64 / 96 us against 89 / 130 / 224 us for the pair of kernels that took them before),
+  // and so does one gradient alone (7 x 7 on 4096 x 2048: 45 and 49 us against 95 and 114 us).
+  const int64_t tiles = (int64_t)cdiv(p.w, 64) * cdiv(p.h, 32) * p.batch;
   if (grad_in && grad_mask_dev && mask_w == mask_h && (K == 3 || K == 5 || K == 7) && p.w >= 8 && p.h >= 8 &&
-      (int64_t)cdiv(p.w, 64) * cdiv(p.h, 32) * p.batch >= 4 * num_sms() &&
+      2 * tiles >= (K == 3 ? 3 : 8) * num_sms() &&
       tma_legal(p.gout, grad_out->pitch, grad_out->batch_stride, p.batch) &&
       tma_legal(p.in, in->pitch, in->batch_stride, p.batch)) {
     AdjFusedParams P;

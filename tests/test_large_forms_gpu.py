@@ -65,7 +65,7 @@ def _floats(seed, h=H, w=W, signed=False):
 @pytest.mark.parametrize("k", [3, 5, 7])
 @pytest.mark.parametrize("h,w", [(41, 132), (33, 64)])
 def test_fused_square_mask_adjoint(gpu, oracle, k, boundary, h, w):
-    """adj_fused_kernel: both gradients, rows of whole 16 bytes, from 4 SMs' worth of 64 x 32 tiles on."""
+    """adj_fused_kernel: both gradients, rows of whole 16 bytes, four 64 x 32 tiles per SM."""
     n = _batch(math.ceil(w / 64) * math.ceil(h / 32), 4 * SMS)
     img, gout = _floats(k, h, w), _floats(k + 100, h, w, True)
     m = np.random.default_rng(k).random((k, k)).astype(np.float32)
@@ -77,6 +77,25 @@ def test_fused_square_mask_adjoint(gpu, oracle, k, boundary, h, w):
     for b, c in enumerate(_weights(n)):
         ri, rm = oracle.local_op_adjoint(img[b].numpy(), gout[b].numpy(), m, boundary)
         scale = np.linalg.norm(oracle.local_op_adjoint(img[b].numpy(), gout[b].abs().numpy(), m, boundary)[0])
+        assert _close(got[b], ri, scale), b
+        ref_m = ref_m + c * rm
+    assert np.abs(gm.cpu().numpy() - ref_m).max() <= 3e-6 * g.abs().double().sum().item()
+
+
+@pytest.mark.parametrize("k", [3, 5, 7])
+@pytest.mark.parametrize("step", [-1, 0])
+def test_square_mask_adjoint_about_the_line(gpu, oracle, step, k):
+    """The last batch of the tiled kernel and the first of the fused one: 1.5 (3 x 3) or 4 tiles per SM."""
+    h, w = 41, 132  # 6 tiles
+    n = _batch(6, -(-3 * SMS // 2) if k == 3 else 4 * SMS) + step
+    img, gout = _floats(k + 4, h, w), _floats(k + 104, h, w, True)
+    m = np.random.default_rng(k).random((k, k)).astype(np.float32)
+    x, g = _copies(img, n), _copies(gout, n)
+    gi, gm = gpu.local_op_adjoint(g, m, boundary=3, inp=x)
+    got, ref_m = _check_copies(gi), 0.0
+    for b, c in enumerate(_weights(n)):
+        ri, rm = oracle.local_op_adjoint(img[b].numpy(), gout[b].numpy(), m, 3)
+        scale = np.linalg.norm(oracle.local_op_adjoint(img[b].numpy(), gout[b].abs().numpy(), m, 3)[0])
         assert _close(got[b], ri, scale), b
         ref_m = ref_m + c * rm
     assert np.abs(gm.cpu().numpy() - ref_m).max() <= 3e-6 * g.abs().double().sum().item()
