@@ -130,10 +130,8 @@ __global__ void __launch_bounds__(BL_BX *BL_BY) bilateral_half_kernel(const __gr
 // FP32 weights.  A thread owns four (two on small images) columns of two rows, each pixel pair (rows y
 // and y + 1 of a column) one f32x2 lane pair.  The tile is kept as pairs too, cell
 // (r, x) = (v[r][x], v[r + 1][x]), so that a tap's operand for a pixel pair is one
-// aligned register pair straight from a 16-byte load: with horizontal pairs every
-// second one had to be assembled with moves, and the mask's coefficients too
-// (206 issue slots per mask row and 128 pixels against 164, where the FMA pipe and
-// the exponential unit take 208 cycles each).  Row-major tap order per pixel.
+// aligned register pair straight from a 16-byte load: of horizontal pairs every
+// second one has to be assembled from two.  Row-major tap order per pixel.
 // 13 x 13, f32 4096 x 4096: 469 us before, 425 us now, the FMA pipe and
 // the exponential unit both 72 % busy.
 constexpr int BP_NT = 256, BP_TW = 64;

@@ -14,11 +14,11 @@
 // operation; a tile's sums join the warp's compensated ones (tap_fold.cuh).  The next tile is
 // staged (asynchronous copies) while this one computes.  Any row alignment.
 //
-// Bound by load latency and issue at 16 to 24 warps per SM (the mask gradient's
-// registers), not by the FMA pipe (2 K^2 lane operations per pixel, 24 us for 7 x 7 on
-// 8.4 Mpx, which takes 86 us).  Two kernels without a register block over rows took
-// the layouts and forms that come here before: 7 x 7 on 2 images of 2049 x 2051 224 us,
-// now 99 us.
+// Bound by instruction fetch (the unrolled passes) and latencies at 16 to 24 warps per SM
+// (the mask gradient's registers): 7 x 7 keeps 42 % of the issue slots and of the FMA pipe
+// busy, its first stall is no_instruction.  Its 2 K^2 lane operations per pixel are 24 us of
+// the 88 us that 8.4 Mpx take.  Two kernels without a register block over rows took the
+// layouts and forms that come here before: 7 x 7 on 2 images of 2049 x 2051 224 us, now 96 us.
 #include <algorithm>
 #include <cstring>
 

@@ -17,8 +17,10 @@
 // images once per tap.  In the column form of a separable filter the row pass
 // t = rows(in) is recomputed in shared memory (the forward's operations and
 // order) instead of written to memory and read back.
+// Bound by the wait for each tile's loads and by latencies at 6 to 9 CTAs per SM (issue
+// slots 49 to 53 % busy, first stall long_scoreboard): a tile is staged, then computed.
 // Forward and adjoint of the separable filter: K = 9 on 4 images of 1920 x 1080
-// 485 -> 87 us, K = 5 on 4096 x 2048 689 -> 97 us.
+// 485 -> 87 us, K = 5 on 4096 x 2048 689 -> 90 us.
 //
 // Included by line_k3_9.cu and line_k11_15.cu, which compile in parallel.
 #pragma once

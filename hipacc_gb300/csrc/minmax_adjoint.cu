@@ -125,9 +125,10 @@ __global__ void __launch_bounds__(MM_T) minmax_gather_kernel(const __grid_consta
 // 64 x 8 PY pixels per CTA, a thread per 4 x PY (PY = 4, fewer on small
 // batches).  The general kernels above spend
 // a remap and a global load on every tap of every pixel; here the tile and its
-// halo are staged once and a row's taps come from a register window.  Bound by
-// the ALU pipe: a compare and two selects per tap (select), a compare and a
-// predicated add per tap (gather).  Forward and adjoint of the 5 x 5 disc on 8
+// halo are staged once and a row's taps come from a register window.  Select is
+// bound by the ALU pipe (a compare and two selects per tap: 85 % busy on 8 images of
+// 1024 x 1024), gather by its loads (first stall long_scoreboard, issue slots 64 %
+// busy, ALU pipe 40 %).  Forward and adjoint of the 5 x 5 disc on 8
 // images of 509 x 381: 176 -> 38 us; of the 7 x 7 disc on
 // 2309 x 2207: 779 -> 142 us.
 constexpr int MT_BX = 16, MT_NT = 128, MT_PAD = 3, MT_TW = 64, MT_SW = MT_TW + 8, MT_G = MT_SW / 4;

@@ -99,8 +99,10 @@ __device__ __forceinline__ uint8_t hc_response(const HarrisParams &p, int gx, in
 // sign).  The two-pixel frame takes four lanes per pixel and the
 // boundary rule at every read, in the grid's first CTAs.
 //
-// Bound by instruction issue.  One pixel per thread with 27 shared 4-byte reads
-// and int products took 90 us for 4032 x 3024; this takes 51 us (HBM floor 3.6 us).
+// Bound by instructions at 20 warps per SM (83 registers): issue slots 58 % busy, the
+// FMA pipe, which a packed operation holds for two cycles, 50 %.  One pixel per thread
+// with 27 shared 4-byte reads and int products took 90 us for 4032 x 3024; this takes
+// 51 us (HBM floor 3.6 us).
 constexpr int HT_W = 128, HT_NT = 128, HT_SW = HT_W + 8;  // tile and staged bytes per row
 
 __device__ __forceinline__ f2 f2_both(float v) { return f2_pack(v, v); }
@@ -412,8 +414,8 @@ __device__ __forceinline__ uchar4 uns_load(const UnsharpParams &p, const uchar4 
 // shared copy of five tables cost about 17 shared-memory cycles per pixel row of
 // a warp against 3).  The warps of one wave share the rows of the strips evenly.
 //
-// Bound by instruction issue.  One pixel per thread over 32 x 16 tiles took
-// 120 us for 4032 x 3024; this takes 55 us (HBM floor 14.4 us).
+// Bound by instruction issue (72 % of the slots busy).  One pixel per thread over
+// 32 x 16 tiles took 120 us for 4032 x 3024; this takes 55 us (HBM floor 14.4 us).
 constexpr int UF_NT = 256, UF_COLS = 120;
 
 // (float)(((double)(0.2126f p_r) + 0.7152 p_g) + 0.0722 p_b) of two pixels w0, w1

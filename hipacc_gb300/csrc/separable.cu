@@ -37,9 +37,11 @@ namespace {
 
 constexpr int kSepMaxK = 15;
 // 16-bit tiles staged by TMA take row_pass8 from 11 taps on.  bf16, four outputs per lane
-// against eight: 15 taps 2 x 1920 x 1080 14.3 / 12.8 us, 13 taps 4 x 1920 x 1080 20.5 /
-// 18.5, 11 taps 19.8 / 17.4; but 9 taps 8192 x 8192 93.8 / 95.7, 3 taps (f16) 8 x 1024 x
-// 1024 9.8 / 10.2: with few taps the wider window's loads and conversions weigh more.
+// against eight, 8192 x 8192: 15 taps 153.9 / 130.3 us, 13 taps 136.4 / 118.0, 11 taps 129.3 /
+// 109.8; but 9 taps 95.5 / 97.5, 7 taps 82.0 / 83.2, 5 taps 67.8 / 70.6: with few taps the
+// wider window's loads and conversions weigh more.  4096 x 4096, 4 x 1920 x 1080, 8 x 1024 x
+// 1024 and f16 draw the same line (f16 has 7 taps 2 to 5 % in favour of eight); on 640 x 480
+// the two are within 3 %.
 constexpr int kSepWideK = 11;
 
 struct SepParams {

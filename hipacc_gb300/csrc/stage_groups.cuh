@@ -2,12 +2,12 @@
 // row alignment and any boundary, four columns at a time.
 //
 // Rows [Y0, Y0 + SH) x columns [X0, X0 + SW) of an accessor window are copied
-// into `tile` (row pitch SW floats).  A group of four columns that lies inside
-// the window is loaded whole: one vector load where its address allows it,
-// else the aligned 32-bit words around it, shifted into place (u8 and 16-bit
-// rows of odd length start at any byte).  Only groups that leave the window
-// evaluate the boundary remap (lib/AST/BorderHandling.cpp:41-120), so a border
-// tile costs little more than an inner one.
+// into `tile` (row pitch SW floats).  In a tile inside the window every group of
+// four columns is loaded whole: one vector load where the rows' alignment allows
+// it, else the aligned words around it, shifted into place (u8 and 16-bit rows of
+// odd length start at any byte).  A border tile evaluates the boundary remap
+// (lib/AST/BorderHandling.cpp:41-120) once per row and column and loads every
+// group element by element through those tables.
 //
 // Why: the per-element staging this replaces spent a remap (two compares and
 // often a branch per axis) and one byte load on every staged cell, ~21 cells

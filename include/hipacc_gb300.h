@@ -284,7 +284,9 @@ HGB_API int hgb_unsharp(const hgb_view *in, const hgb_view *out, int boundary, i
  *   f32/f16/bf16 MIN/MAX/PROD -> folded in float, delivered widened to a double
  *   f64 -> double
  * `result_dev` (device, 8 bytes) and/or `result_host` (8 bytes; the call then
- * synchronises the stream). */
+ * synchronises the stream).  A thread's first call for a host result alone pins
+ * 8 bytes of host memory, which the kernel writes and which are freed when the
+ * thread ends; where they cannot be had the result is copied back instead. */
 HGB_API int hgb_reduce(const hgb_view *in, const hgb_window *win, int op, void *result_dev, void *result_host,
                void *stream);
 
