@@ -133,7 +133,9 @@ __global__ void __launch_bounds__(BL_BX *BL_BY) bilateral_half_kernel(const __gr
 // aligned register pair straight from a 16-byte load: of horizontal pairs every
 // second one has to be assembled from two.  Row-major tap order per pixel.
 // 13 x 13, f32 4096 x 4096: 469 us before, 425 us now, the FMA pipe and
-// the exponential unit both 72 % busy.
+// the exponential unit both 72 % busy.  The values are scaled as the pairs form, so
+// that f32 tiles are staged by asynchronous copies (3 x 3, 4096 x 4096: 53 us, 61 us with
+// values scaled on their way through registers).
 constexpr int BP_NT = 256, BP_TW = 64;
 // rows of a tile with CPT columns per thread
 constexpr int bp_rows(int cpt) { return 2 * BP_NT / (BP_TW / cpt); }
@@ -152,17 +154,16 @@ __global__ void __launch_bounds__(BP_NT) bilateral_kernel(const __grid_constant_
     const float v = x < S ? -p.lmask[y * S + x] : 0.0f;
     nl[y][x] = f2_pack(v, v);
   }
-  const float q = p.q;  // the FP32 path works on values scaled by q
-  stage_groups_each<T, SW, SH, BP_NT>(p.in + (int64_t)b * p.in_bstride, p.in_pitch, i0 - HL, j0 - R, 0, p.w, 0, p.h,
-                                      p.bmode, p.cval, R, [=](int c, float4 v) {
-                                        reinterpret_cast<float4 *>(tile)[c] = make_float4(
-                                            __fmul_rn(v.x, q), __fmul_rn(v.y, q), __fmul_rn(v.z, q), __fmul_rn(v.w, q));
-                                      });
+  stage_groups<T, SW, SH, BP_NT>(tile, p.in + (int64_t)b * p.in_bstride, p.in_pitch, i0 - HL, j0 - R, 0, p.w, 0, p.h,
+                                 p.bmode, p.cval, R);
+  stage_wait();
   __syncthreads();
+  const float q = p.q;  // the FP32 path works on values scaled by q
 #pragma unroll 2
   for (int c = threadIdx.x; c < (SH - 1) * (SW / 2); c += BP_NT) {
     const float2 lo = reinterpret_cast<const float2 *>(tile)[c], hi = reinterpret_cast<const float2 *>(tile)[c + SW / 2];
-    reinterpret_cast<float4 *>(cell)[c] = make_float4(lo.x, hi.x, lo.y, hi.y);
+    reinterpret_cast<float4 *>(cell)[c] =
+        make_float4(__fmul_rn(lo.x, q), __fmul_rn(hi.x, q), __fmul_rn(lo.y, q), __fmul_rn(hi.y, q));
   }
   __syncthreads();
   const int tx = threadIdx.x % (BP_TW / CPT), ty = threadIdx.x / (BP_TW / CPT);
@@ -249,9 +250,12 @@ int launch_bil_s(const BilParams &p, int batch, cudaStream_t st) {
     return after_launch("bilateral_half_kernel", st, ev);
   } else {
     // four columns per thread (64 x 32 tiles), or two (64 x 16) where those would
-    // not give every SM two CTAs: a small image's time is one thread's taps
-    // (320 x 256, 13 x 13: 12.9 us with four, 8.0 us with two)
-    if ((int64_t)cdiv(p.w, BP_TW) * cdiv(p.h, bp_rows(4)) * batch >= 2 * num_sms())
+    // not give every SM four CTAs: a small image's time is one thread's taps, and up
+    // to a few tiles per SM the last wave counts.  f32, four / two, 9 x 9 and 13 x 13:
+    // 320 x 256 7.9 / 5.5 and 12.9 / 8.3 us, 1024 x 1024 19.8 / 18.1 and 36.2 / 32.5, 4 of
+    // 640 x 480 20.6 / 20.6 and 37.1 / 36.2; 1920 x 1080 31.6 / 32.6 and 59.6 / 59.6, 4096 x
+    // 4096 215.6 / 229.1 and 426 / 434
+    if ((int64_t)cdiv(p.w, BP_TW) * cdiv(p.h, bp_rows(4)) * batch >= 4 * num_sms())
       return launch_bil_pairs<T, S, 4>(p, batch, st);
     return launch_bil_pairs<T, S, 2>(p, batch, st);
   }

@@ -216,9 +216,9 @@ def test_sobel_tall_tiles(gpu, oracle, pad, boundary):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("size", [3, 5, 7, 9, 11, 13])
 def test_bilateral_four_columns(gpu, oracle, size, dtype):
-    """Four columns per thread (from 2 SMs' worth of 64 x 32 tiles on) against the two-column form of a
+    """Four columns per thread (from four 64 x 32 tiles per SM on) against the two-column form of a
     single image, which the oracle checks elsewhere: the same taps in the same order."""
-    n = _batch(9, 2 * SMS)
+    n = _batch(9, 4 * SMS)
     img = _floats(size).to(dtype)
     sm = oracle.spatial_mask(size, size / 4.0)
     for boundary in (0, 1, 2, 3, 4):
