@@ -272,29 +272,43 @@ __device__ __forceinline__ void stage_words(uint32_t *tile, const uint8_t *img, 
       });
     return;
   }
-#pragma unroll 2
+  // Border tiles: first the words with four columns to spare and those outside, with
+  // the loads of eight words in flight, then the few words at the left and right
+  // edges byte by byte.  (One loop with both kinds kept two words in flight: 250 x 250
+  // Sobel 6.6 us.)
+#pragma unroll 8
   for (int c = threadIdx.x; c < SH * G; c += NT) {
     const int x = X0 + 4 * k, y = Y0 + r;
+    const bool row = y >= 0 && y < h, spare = row && x >= 4 && x + 8 <= w;
     uint32_t v = 0;
-    if (y >= 0 && y < h && x + 3 >= 0 && x < w) {
+    if (spare) {
       const uint8_t *q = img + (int64_t)y * pitch + x;
       const unsigned s = (unsigned)(reinterpret_cast<uintptr_t>(q) & 3u);
-      if (x >= 4 && x + 8 <= w) {
-        const uint32_t *u = reinterpret_cast<const uint32_t *>(q - s);
-        v = __funnelshift_r(__ldg(u), __ldg(u + 1), 8 * s);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (x + i >= 0 && x + i < w) v |= (uint32_t)__ldg(q + i) << (8 * i);
-      }
+      const uint32_t *u = reinterpret_cast<const uint32_t *>(q - s);
+      v = __funnelshift_r(__ldg(u), __ldg(u + 1), 8 * s);
     }
-    tile[c] = v;
+    if (spare || !row || x + 3 < 0 || x >= w) tile[c] = v;
     k += NT % G;
     r += NT / G;
     if (k >= G) {
       k -= G;
       ++r;
     }
+  }
+  // words of each row that hold an edge: the one at column 0 and the last two, from x
+  // > w - 8 on (X0 is a multiple of 4)
+  const int kl = -X0 / 4, kr = (max(w - 7, 0) + 3) / 4 - X0 / 4;
+#pragma unroll 2
+  for (int c = threadIdx.x; c < 3 * SH; c += NT) {
+    const int e = c / SH, rr = c - e * SH, kk = e == 0 ? kl : kr + e - 1;
+    const int x = X0 + 4 * kk, y = Y0 + rr;
+    if (kk < 0 || kk >= G || y < 0 || y >= h || x >= w || (x >= 4 && x + 8 <= w)) continue;
+    const uint8_t *q = img + (int64_t)y * pitch + x;
+    uint32_t v = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (x + i < w) v |= (uint32_t)__ldg(q + i) << (8 * i);
+    tile[rr * G + kk] = v;
   }
 }
 
