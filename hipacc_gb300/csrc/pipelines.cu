@@ -127,27 +127,37 @@ __device__ __forceinline__ uint32_t hc_corner(float k, float threshold, float ux
 
 // the response at a pixel with the boundary rule at every read, by four lanes (a
 // row of products each): the Gaussian reads the products at their remapped
-// positions (CONSTANT: 0)
+// positions (CONSTANT: 0, as products of pixels that read 0).  The rows and columns
+// are remapped first, so that a lane's 27 loads are in flight together (one product
+// after the other took the smallest images from 4.9 to 6.4 us with CONSTANT).
 __device__ __forceinline__ uint8_t hc_frame_pixel(const HarrisParams &p, const uint8_t *img, int x, int y, int part) {
   int a = 0, bb = 0, cc = 0;
-  const int uy = remap(p.bmode, y - 1 + part, 0, p.h);
-  if (part < 3 && uy != (int)0x80000000) {
-#pragma unroll 1
-    for (int dj = 0; dj < 3; ++dj) {
-      const int ux = remap(p.bmode, x - 1 + dj, 0, p.w);
-      if (ux == (int)0x80000000) continue;
-      int v[3][3];
+  const int uy = part < 3 ? remap(p.bmode, y - 1 + part, 0, p.h) : (int)0x80000000;
+  int row[3], col[3][3];  // negative: reads 0
 #pragma unroll
-      for (int r = 0; r < 3; ++r)
+  for (int r = 0; r < 3; ++r) row[r] = uy < 0 ? uy : remap(p.bmode, uy - 1 + r, 0, p.h);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) v[r][c] = hc_in(p, img, ux - 1 + c, uy - 1 + r);
-      int16_t dx, dy;
-      hc_deriv(v, dx, dy);
-      const int m = (part == 1 ? 2 : 1) * (dj == 1 ? 2 : 1);
-      a += (int16_t)(dx * dx) * m;
-      bb += (int16_t)(dy * dy) * m;
-      cc += (int16_t)(dx * dy) * m;
-    }
+  for (int dj = 0; dj < 3; ++dj) {
+    const int ux = remap(p.bmode, x - 1 + dj, 0, p.w);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) col[dj][c] = ux < 0 ? ux : remap(p.bmode, ux - 1 + c, 0, p.w);
+  }
+  int v[3][3][3];
+#pragma unroll
+  for (int dj = 0; dj < 3; ++dj)
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        v[dj][r][c] = (row[r] | col[dj][c]) < 0 ? 0 : __ldg(img + (int64_t)row[r] * p.in_p + col[dj][c]);
+#pragma unroll
+  for (int dj = 0; dj < 3; ++dj) {
+    int16_t dx, dy;
+    hc_deriv(v[dj], dx, dy);
+    const int m = (part == 1 ? 2 : 1) * (dj == 1 ? 2 : 1);
+    a += (int16_t)(dx * dx) * m;
+    bb += (int16_t)(dy * dy) * m;
+    cc += (int16_t)(dx * dy) * m;
   }
 #pragma unroll
   for (int d = 1; d < 4; d <<= 1) {
@@ -725,18 +735,22 @@ extern "C" int hgb_harris_corner(const hgb_view *in, const hgb_view *out, float 
     const int64_t edge = 4 * ((int64_t)p.w + p.h);  // at least the frame's pixels
     const int frame = (int)((4 * std::min<int64_t>(edge, (int64_t)p.w * p.h) + HT_NT - 1) / HT_NT);
     // 64-row tiles (16 rows per warp, 4 more to start from) where they give every
-    // SM four CTAs, else 16-row ones (the time of a small image is the chain of
-    // rows that a warp walks); 128-row tiles are slower (one wave of uneven CTAs,
-    // 60 us against 51 us for 4032 x 3024)
-    const bool tall = (int64_t)tiles_x * cdiv(p.h, 64) * in->batch >= 4 * num_sms();
-    const int64_t ntiles = (int64_t)tiles_x * cdiv(p.h, tall ? 64 : 16);
+    // SM four CTAs, else 16-row ones, or 8-row ones where five quarters of the SMs have
+    // one (the time of a small image is the chain of rows that a warp walks: 640 x 480
+    // 5.95 us with 16 rows, 5.4 with 8; 800 x 600 5.97 and 6.4); 128-row tiles are slower
+    // (one wave of uneven CTAs, 60 us against 51 us for 4032 x 3024 at the time)
+    const int64_t per_row = (int64_t)tiles_x * in->batch;
+    const int rows = per_row * cdiv(p.h, 64) >= 4 * num_sms() ? 64 : 4 * per_row * cdiv(p.h, 16) > 5 * num_sms() ? 16 : 8;
+    const int64_t ntiles = (int64_t)tiles_x * cdiv(p.h, rows);
     HGB_REQUIRE(ntiles + frame < 0x7fffffff, "hgb_harris_corner: image too large");
     const dim3 grid((unsigned)(ntiles + frame), 1, in->batch);
     cudaEvent_t ev = before_launch(st);
-    if (tall)
+    if (rows == 64)
       harris_fused_kernel<16><<<grid, HT_NT, 0, st>>>(p, tiles_x, frame);
-    else
+    else if (rows == 16)
       harris_fused_kernel<4><<<grid, HT_NT, 0, st>>>(p, tiles_x, frame);
+    else
+      harris_fused_kernel<2><<<grid, HT_NT, 0, st>>>(p, tiles_x, frame);
     return after_launch("harris_fused_kernel", st, ev);
   }
   const size_t px = (size_t)p.w * p.h * in->batch;
