@@ -426,7 +426,8 @@ __device__ __forceinline__ uchar4 uns_load(const UnsharpParams &p, const uchar4 
 //
 // Bound by instruction issue (72 % of the slots busy).  One pixel per thread over
 // 32 x 16 tiles took 120 us for 4032 x 3024; this takes 55 us (HBM floor 14.4 us).
-constexpr int UF_NT = 256, UF_COLS = 120;
+constexpr int UF_NT = 256;
+constexpr int uf_cols(int np) { return 30 * 2 * np; }  // columns of a strip with np pairs per lane
 
 // (float)(((double)(0.2126f p_r) + 0.7152 p_g) + 0.0722 p_b) of two pixels w0, w1
 __device__ __forceinline__ f2 uns_gray2(const float *tab, const UnsTables *T, f2 nz, uint32_t w0, uint32_t w1) {
@@ -490,117 +491,145 @@ __device__ __forceinline__ uint32_t uns_scale_word(uint32_t v, float r) {
   return o;
 }
 
+template <int NP>
 __global__ void __launch_bounds__(UF_NT) unsharp_fused_kernel(const __grid_constant__ UnsharpParams p, int strips,
                                                               int rows_per, int segments) {
+  constexpr int CPL = 2 * NP;  // columns per lane
   __shared__ __align__(16) float tab[256 * 32];
-#pragma unroll
-  for (int i = threadIdx.x; i < 256 * 8; i += UF_NT) {
-    const float v = __ldg(&p.tab->p[i >> 3]);
-    reinterpret_cast<float4 *>(tab)[i] = make_float4(v, v, v, v);
-  }
-  __syncthreads();
   const int lane = threadIdx.x & 31;
   const float *tl = tab + lane;
   const int64_t job = (int64_t)blockIdx.x * (UF_NT / 32) + (threadIdx.x >> 5);
-  const int b = (int)(job / ((int64_t)strips * segments)), jr = (int)(job - (int64_t)b * strips * segments);
-  if (b >= p.batch) return;
-  const int seg = jr / strips, x = (jr - seg * strips) * UF_COLS - 4 + 4 * lane;  // this lane's columns
+  const int64_t per = (int64_t)strips * segments;
+  // (a 64-bit division takes several times a 32-bit one)
+  const int b = (int)((job | per) >> 32 ? job / per : (int64_t)((unsigned)job / (unsigned)per)), jr = (int)(job - b * per);
+  const bool idle = b >= p.batch;
+  const int seg = jr / strips, x = (jr - seg * strips) * uf_cols(NP) - CPL + CPL * lane;  // this lane's columns
   const int y0 = seg * rows_per, y1 = min(y0 + rows_per, p.h);
   const uint32_t *img = reinterpret_cast<const uint32_t *>(p.in) + (int64_t)b * p.in_b;
   uint32_t *out = reinterpret_cast<uint32_t *>(p.out) + (int64_t)b * p.out_b;
-  const bool whole = x >= 0 && x + 4 <= p.w;
+  const bool whole = x >= 0 && x + CPL <= p.w;
   const bool stores = lane > 0 && lane < 31 && x < p.w;
-  bool in_col[4] = {true, true, true, true};  // false: a CONSTANT column, gray 0
-  int cx[4] = {x, x + 1, x + 2, x + 3};
+  bool in_col[CPL];  // false: a CONSTANT column, gray 0
+  int cx[CPL];
+#pragma unroll
+  for (int q = 0; q < CPL; ++q) {
+    in_col[q] = true;
+    cx[q] = x + q;
+  }
   if (!whole) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < CPL; ++q) {
       // columns past the halo serve no pixel: any valid address will do
       const int rx = x + q > p.w ? p.w - 1 : (x + q < -1 ? 0 : remap(p.bmode, x + q, 0, p.w));
       in_col[q] = rx != (int)0x80000000;
       cx[q] = in_col[q] ? rx : 0;
     }
   }
-  auto load = [&](int ry, uint32_t (&w)[4]) {
+  auto load = [&](int ry, uint32_t (&w)[CPL]) {
     const uint32_t *row = img + (int64_t)ry * p.in_p;
-    if (whole && (reinterpret_cast<uintptr_t>(row + x) & 15u) == 0) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + x));
-      w[0] = v.x;
-      w[1] = v.y;
-      w[2] = v.z;
-      w[3] = v.w;
+    if (whole && (reinterpret_cast<uintptr_t>(row + x) & (4 * CPL - 1)) == 0) {
+      if constexpr (NP == 2) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(row + x));
+        w[0] = v.x;
+        w[1] = v.y;
+        w[2] = v.z;
+        w[3] = v.w;
+      } else {
+        const uint2 v = __ldg(reinterpret_cast<const uint2 *>(row + x));
+        w[0] = v.x;
+        w[1] = v.y;
+      }
     } else {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) w[q] = __ldg(row + cx[q]);
+      for (int q = 0; q < CPL; ++q) w[q] = __ldg(row + cx[q]);
     }
   };
   const float m0 = 0.057118f, m1 = 0.124758f, m2 = 0.272496f;
   auto both = [](float v) { return f2_pack(v, v); };
-  f2 one[2] = {0ull, 0ull}, two[2] = {0ull, 0ull};  // partial sums after one and two rows of their windows
-  f2 gp[2] = {0ull, 0ull};                          // gray of the row above
-  uint32_t wp[4] = {0, 0, 0, 0}, wn[4];
-  {
+  f2 one[NP], two[NP];  // partial sums after one and two rows of their windows
+  f2 gp[NP];            // gray of the row above
+  uint32_t wp[CPL], wn[CPL];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) one[i] = two[i] = gp[i] = 0ull;
+#pragma unroll
+  for (int q = 0; q < CPL; ++q) wp[q] = wn[q] = 0;
+  if (!idle) {  // the first row's loads are in flight while the table is copied
     const int r0 = remap(p.bmode, y0 - 1, 0, p.h);
     load(r0 == (int)0x80000000 ? 0 : r0, wn);
   }
+#pragma unroll
+  for (int i = threadIdx.x; i < 256 * 8; i += UF_NT) {
+    const float v = __ldg(&p.tab->p[i >> 3]);
+    reinterpret_cast<float4 *>(tab)[i] = make_float4(v, v, v, v);
+  }
+  __syncthreads();
+  if (idle) return;
 #pragma unroll 1
   for (int y = y0 - 1; y <= y1; ++y) {
-    uint32_t w[4] = {wn[0], wn[1], wn[2], wn[3]};
+    uint32_t w[CPL];
+#pragma unroll
+    for (int q = 0; q < CPL; ++q) w[q] = wn[q];
     const bool row_in = (y >= 0 && y < p.h) || p.bmode != HGB_BOUNDARY_CONSTANT;
     if (y < y1) {  // the next row's loads are in flight while this one computes
       const int rn = remap(p.bmode, y + 1, 0, p.h);
       load(rn == (int)0x80000000 ? 0 : rn, wn);
     }
-    f2 g[2] = {uns_gray2(tl, p.tab, p.nz, w[0], w[1]), uns_gray2(tl, p.tab, p.nz, w[2], w[3])};
+    f2 g[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) g[i] = uns_gray2(tl, p.tab, p.nz, w[2 * i], w[2 * i + 1]);
     if (p.bmode == HGB_BOUNDARY_CONSTANT && (!row_in || !whole)) {
-      float v[4] = {f2_lo(g[0]), f2_hi(g[0]), f2_lo(g[1]), f2_hi(g[1])};
 #pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = row_in && in_col[q] ? v[q] : 0.0f;
-      g[0] = f2_pack(v[0], v[1]);
-      g[1] = f2_pack(v[2], v[3]);
+      for (int i = 0; i < NP; ++i)
+        g[i] = f2_pack(row_in && in_col[2 * i] ? f2_lo(g[i]) : 0.0f, row_in && in_col[2 * i + 1] ? f2_hi(g[i]) : 0.0f);
     }
-    const float left = __shfl_up_sync(0xffffffffu, f2_hi(g[1]), 1);
+    const float left = __shfl_up_sync(0xffffffffu, f2_hi(g[NP - 1]), 1);
     const float right = __shfl_down_sync(0xffffffffu, f2_lo(g[0]), 1);
-    // columns (-1, 0), (1, 2), (3, 4) relative to x
-    const f2 go[3] = {f2_pack(left, f2_lo(g[0])), f2_pack(f2_hi(g[0]), f2_lo(g[1])), f2_pack(f2_hi(g[1]), right)};
-    f2 a0[3], a1[3], c1[2], c2[2];
+    f2 go[NP + 1];  // columns (-1, 0), (1, 2), .. relative to x
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
+    for (int i = 0; i <= NP; ++i)
+      go[i] = f2_pack(i == 0 ? left : f2_hi(g[i > 0 ? i - 1 : 0]), i == NP ? right : f2_lo(g[i < NP ? i : 0]));
+    f2 a0[NP + 1], a1[NP + 1], c1[NP], c2[NP];
+#pragma unroll
+    for (int i = 0; i <= NP; ++i) {
       a0[i] = f2_mul_rounded(both(m0), go[i], p.nz);
       a1[i] = f2_mul_rounded(both(m1), go[i], p.nz);
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < NP; ++i) {
       c1[i] = f2_mul_rounded(both(m1), g[i], p.nz);
       c2[i] = f2_mul_rounded(both(m2), g[i], p.nz);
     }
-    f2 blur[2];
+    f2 blur[NP];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < NP; ++i) {
       // this row as the last of the window above, the middle of the next, the first of the one below
       blur[i] = f2_add(f2_add(f2_add(two[i], a0[i]), c1[i]), a0[i + 1]);
       two[i] = f2_add(f2_add(f2_add(one[i], a1[i]), c2[i]), a1[i + 1]);
       one[i] = f2_add(f2_add(f2_add(0ull, a0[i]), c1[i]), a0[i + 1]);
     }
     if (y > y0 && stores) {  // the window centred on row y - 1 is complete
-      const float gv[4] = {f2_lo(gp[0]), f2_hi(gp[0]), f2_lo(gp[1]), f2_hi(gp[1])};
-      const float bv[4] = {f2_lo(blur[0]), f2_hi(blur[0]), f2_lo(blur[1]), f2_hi(blur[1])};
-      uint32_t o[4];
+      uint32_t o[CPL];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) o[q] = uns_scale_word(wp[q], uns_ratio(gv[q], bv[q]));
+      for (int q = 0; q < CPL; ++q) {
+        const f2 G = gp[q / 2], B = blur[q / 2];
+        o[q] = uns_scale_word(wp[q], q & 1 ? uns_ratio(f2_hi(G), f2_hi(B)) : uns_ratio(f2_lo(G), f2_lo(B)));
+      }
       uint32_t *dst = out + (int64_t)(y - 1) * p.out_p + x;
-      if (x + 4 <= p.w && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
-        *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+      if (x + CPL <= p.w && (reinterpret_cast<uintptr_t>(dst) & (4 * CPL - 1)) == 0) {
+        if constexpr (NP == 2)
+          *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+        else
+          *reinterpret_cast<uint2 *>(dst) = make_uint2(o[0], o[1]);
       } else {
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int q = 0; q < CPL; ++q)
           if (x + q < p.w) dst[q] = o[q];
       }
     }
-    gp[0] = g[0];
-    gp[1] = g[1];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) wp[q] = w[q];
+    for (int i = 0; i < NP; ++i) gp[i] = g[i];
+#pragma unroll
+    for (int q = 0; q < CPL; ++q) wp[q] = w[q];
   }
 }
 
@@ -613,6 +642,40 @@ __device__ __forceinline__ bool us_pixel(const UnsharpParams &p, int &x, int &y,
 }
 __device__ __forceinline__ int64_t us_at(const UnsharpParams &p, int b, int x, int y) {
   return ((int64_t)b * p.h + y) * p.w + x;
+}
+
+using UnsharpKernel = void (*)(UnsharpParams, int, int, int);
+UnsharpKernel unsharp_kernel(int np) { return np == 2 ? unsharp_fused_kernel<2> : unsharp_fused_kernel<1>; }
+
+// Pairs per lane and rows per warp.  A warp's rows (two more than it stores) run one
+// after another, in 0.30 us + 0.47 us (two pairs) or 0.26 us (one pair) per CTA on the
+// SM, measured on 64 x 64 to 4032 x 3024; the least sum over the CTAs per SM wins.  One
+// pair also leaves less of a strip empty on narrow images.  4032 x 3024 54 us (60 us
+// with one pair), 1920 x 1080 13.7 us (15.0 us in one full wave of two pairs), 1280 x 720
+// 9.3 us (10.3), 640 x 480 6.0 us (6.4), 64 x 64 3.5 us (5.1).
+struct UnsharpShape {
+  int np, strips, rows, segments;
+  int64_t ctas;
+};
+UnsharpShape unsharp_shape(int w, int h, int batch) {
+  constexpr int kWarps = UF_NT / 32;
+  UnsharpShape best = {};
+  int64_t least = -1;
+  for (int np = 2; np >= 1; --np) {
+    const int strips = cdiv(w, uf_cols(np)), fit = resident_ctas((const void *)unsharp_kernel(np), UF_NT, 0);
+    const int64_t columns = (int64_t)strips * batch, sms = num_sms();
+    for (int c = 1; c <= fit; ++c) {
+      const int64_t most = std::max<int64_t>(1, c * sms * kWarps / columns);  // segments
+      const int rows = (int)((h + most - 1) / most), segments = cdiv(h, rows);
+      const int64_t ctas = (columns * segments + kWarps - 1) / kWarps;
+      const int64_t cost = (rows + 2) * (30 + (np == 2 ? 47 : 26) * ((ctas + sms - 1) / sms));
+      if (least < 0 || cost < least) {
+        least = cost;
+        best = {np, strips, rows, segments, ctas};
+      }
+    }
+  }
+  return best;
 }
 
 __global__ void __launch_bounds__(256) unsharp_gray_kernel(const __grid_constant__ UnsharpParams p) {
@@ -810,19 +873,10 @@ extern "C" int hgb_unsharp(const hgb_view *in, const hgb_view *out, int boundary
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   if (mode == 0) {
-    // one wave of warps shares the rows of the strips; a segment recomputes the
-    // gray of two rows besides its own, so it has at least two (on an image that
-    // leaves most of the GPU idle, shorter segments end sooner)
-    const int strips = cdiv(p.w, UF_COLS);
-    const int64_t warps = (int64_t)num_sms() * resident_ctas((const void *)unsharp_fused_kernel, UF_NT, 0) * (UF_NT / 32);
-    const int64_t columns = (int64_t)strips * in->batch;
-    int64_t segments = std::max<int64_t>(1, warps / columns);
-    const int rows_per = std::max(2, (int)((p.h + segments - 1) / segments));
-    segments = cdiv(p.h, rows_per);
-    const int64_t ctas = (columns * segments + UF_NT / 32 - 1) / (UF_NT / 32);
-    HGB_REQUIRE(ctas < 0x7fffffff, "hgb_unsharp: image too large");
+    const UnsharpShape u = unsharp_shape(p.w, p.h, in->batch);
+    HGB_REQUIRE(u.ctas < 0x7fffffff, "hgb_unsharp: image too large");
     cudaEvent_t ev = before_launch(st);
-    unsharp_fused_kernel<<<(unsigned)ctas, UF_NT, 0, st>>>(p, strips, rows_per, (int)segments);
+    unsharp_kernel(u.np)<<<(unsigned)u.ctas, UF_NT, 0, st>>>(p, u.strips, u.rows, u.segments);
     return after_launch("unsharp_fused_kernel", st, ev);
   }
   const size_t px = (size_t)p.w * p.h * in->batch;
