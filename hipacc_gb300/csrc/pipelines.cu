@@ -405,13 +405,7 @@ __device__ __forceinline__ float uns_ratio(float g, float blur) {
   return __fdiv_rn(sharp, fmaxf(g, 0.01f));
 }
 
-__device__ __forceinline__ uchar4 uns_load(const UnsharpParams &p, const uchar4 *img, int vx, int vy, bool &cst) {
-  const int rx = remap(p.bmode, vx, 0, p.w), ry = remap(p.bmode, vy, 0, p.h);
-  cst = rx == (int)0x80000000 || ry == (int)0x80000000;
-  return cst ? make_uchar4(0, 0, 0, 0) : img[(int64_t)ry * p.in_p + rx];
-}
-
-// Fused form.  A warp walks down a strip of 120 columns, a lane four columns
+// Fused form.  A warp walks down a strip of 120 or 60 columns, a lane four or two
 // (the outer two lanes only supply the strip's halo), and keeps everything but
 // the power table in registers: the gray of a row is formed once, its products
 // with the mask's three weights once, and each output row adds the nine products
@@ -420,12 +414,11 @@ __device__ __forceinline__ uchar4 uns_load(const UnsharpParams &p, const uchar4 
 //
 // The power table is a copy per lane, entry v of lane l at word 32 v + l, so the
 // three lookups of a pixel hit 32 banks whatever the bytes; the products 0.7152 p
-// and 0.0722 p come from p as exact float pairs instead of four more tables (one
-// shared copy of five tables cost about 17 shared-memory cycles per pixel row of
-// a warp against 3).  The warps of one wave share the rows of the strips evenly.
+// and 0.0722 p come from p as exact float pairs instead of four more tables.
+// unsharp_shape() shares out the rows.
 //
 // Bound by instruction issue (72 % of the slots busy).  One pixel per thread over
-// 32 x 16 tiles took 120 us for 4032 x 3024; this takes 55 us (HBM floor 14.4 us).
+// 32 x 16 tiles took 120 us for 4032 x 3024; this takes 54 us (HBM floor 14.4 us).
 constexpr int UF_NT = 256;
 constexpr int uf_cols(int np) { return 30 * 2 * np; }  // columns of a strip with np pairs per lane
 

@@ -67,8 +67,8 @@ using PyCfg1 = PyCfg<64, 16, 128>;
 using PyCfg2 = PyCfg<32, 32, 128>;
 using PyCfg3 = PyCfg<64, 32, 256>;
 constexpr int kPyCfgs = 4;
-constexpr int PY_TW = 64, PY_TH = 32;  // config 0, the collapse's tiles
-constexpr int kPyClaim = 4;            // tiles per claim of a persistent CTA
+constexpr int PY_TW = 64;    // config 0, the collapse's tiles (64 x 32)
+constexpr int kPyClaim = 4;  // tiles per claim of a persistent CTA
 
 struct LevelMeta {
   float *g;    // Gaussian level
