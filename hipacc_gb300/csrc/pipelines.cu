@@ -99,10 +99,10 @@ __device__ __forceinline__ uint8_t hc_response(const HarrisParams &p, int gx, in
 // sign).  The two-pixel frame takes four lanes per pixel and the
 // boundary rule at every read, in the grid's first CTAs.
 //
-// Bound by instructions at 20 warps per SM (83 registers): issue slots 58 % busy, the
-// FMA pipe, which a packed operation holds for two cycles, 50 %.  One pixel per thread
-// with 27 shared 4-byte reads and int products took 90 us for 4032 x 3024; this takes
-// 51 us (HBM floor 3.6 us).
+// Bound by instructions at 20 warps per SM (89 registers): issue slots 57 % busy, the
+// FMA pipe, which a packed operation holds for two cycles, 55 %.  One pixel per thread
+// with 27 shared 4-byte reads and int products took 89 us for 4032 x 3024; this takes
+// 43 us (HBM floor 3.6 us).
 constexpr int HT_W = 128, HT_NT = 128, HT_SW = HT_W + 8;  // tile and staged bytes per row
 
 __device__ __forceinline__ f2 f2_both(float v) { return f2_pack(v, v); }
@@ -794,7 +794,7 @@ extern "C" int hgb_harris_corner(const hgb_view *in, const hgb_view *out, float 
     // SM four CTAs, else 16-row ones, or 8-row ones where five quarters of the SMs have
     // one (the time of a small image is the chain of rows that a warp walks: 640 x 480
     // 5.95 us with 16 rows, 5.4 with 8; 800 x 600 5.97 and 6.4); 128-row tiles are slower
-    // (one wave of uneven CTAs, 60 us against 51 us for 4032 x 3024 at the time)
+    // (one wave of uneven CTAs, 60 us against 51 us for 4032 x 3024, with the frame before)
     const int64_t per_row = (int64_t)tiles_x * in->batch;
     const int rows = per_row * cdiv(p.h, 64) >= 4 * num_sms() ? 64 : 4 * per_row * cdiv(p.h, 16) > 5 * num_sms() ? 16 : 8;
     const int64_t ntiles = (int64_t)tiles_x * cdiv(p.h, rows);
