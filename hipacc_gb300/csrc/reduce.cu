@@ -15,25 +15,19 @@ namespace {
 struct HostSlot {
   unsigned long long *p = nullptr;
   ~HostSlot() {
-    if (p) with_relaxed_capture([&] { return cudaFreeHost(p); });
+    if (!p) return;
+    const RelaxedCapture relaxed;
+    if (cudaFreeHost(p) != cudaSuccess) cudaGetLastError();
   }
   unsigned long long *get() {
-    if (!p)
-      with_relaxed_capture([&] {
-        return cudaHostAlloc((void **)&p, sizeof(*p), cudaHostAllocMapped | cudaHostAllocPortable);
-      });
-    return p;  // unified addressing: the same address on every device
-  }
-  // allocation is no part of another thread's stream capture
-  template <typename F>
-  void with_relaxed_capture(F &&f) {
-    cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
-    if (cudaThreadExchangeStreamCaptureMode(&m) != cudaSuccess) return;
-    if (f() != cudaSuccess) {
-      p = nullptr;
-      cudaGetLastError();
+    if (!p) {
+      const RelaxedCapture relaxed;
+      if (cudaHostAlloc((void **)&p, sizeof(*p), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        p = nullptr;
+        cudaGetLastError();
+      }
     }
-    cudaThreadExchangeStreamCaptureMode(&m);
+    return p;  // unified addressing: the same address on every device
   }
 };
 thread_local HostSlot t_slot;
